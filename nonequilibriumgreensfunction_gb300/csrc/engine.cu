@@ -289,10 +289,10 @@ int Engine::alloc() {
   NEGF_TRY(dalloc(&dSrE_, (size_t)S_, bytes_, dry_, pool_, own_st_));
   NEGF_TRY(dalloc(&dSrHend_, (size_t)S_, bytes_, dry_, pool_, own_st_));
   NEGF_TRY(dalloc(&dSrStatus_, (size_t)S_, bytes_, dry_, pool_, own_st_));
-  {   // inv_work_alloc: R buffer, pivots, INFO
+  {   // inv_work_alloc: R buffer, pivots, INFO, interchange lists
     const long long cap = std::max(B_, S_);
     if (!dry_) NEGF_TRY(inv_work_alloc(inv_, M_, (int)cap, pool_, own_st_));
-    bytes_ += 16LL * cap * panel_width(M_) * M_ + 4LL * cap * M_ + 4LL * cap;
+    bytes_ += 16LL * cap * panel_width(M_) * M_ + 4LL * cap * M_ + 4LL * cap + 4LL * cap * kGjMoves;
   }
   if (mixed_) {
     const int cap = std::max(B_, S_);

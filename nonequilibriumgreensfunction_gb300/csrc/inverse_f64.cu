@@ -22,6 +22,7 @@ namespace {
 
 constexpr int PANEL_THREADS = 512;
 constexpr size_t kPanelSmemMax = 200 * 1024;
+constexpr int GJ_MOVES = kGjMoves;   // ints of one matrix's interchange list: count, 64 pairs
 
 // V is the real type of the matrix: the FP32 inverse compares floats, so its pivot search
 // stays off the FP64 pipe (comparing the floats orders them as their doubles would)
@@ -161,24 +162,162 @@ __global__ void __launch_bounds__(PANEL_THREADS) gj_panel_kernel(T* A, long long
   for (int e = t; e < n * kb; e += PANEL_THREADS) dst[e] = Ps[e];
 }
 
+// The FP32 panel with its rows in registers: thread t holds row t of the panel (32 float2), so
+// a column step reads shared memory only for the pivot row, which every thread of a warp reads
+// at one address.  The panel in shared memory (panel_factor) spends its time on the 32 x n
+// elements that each column step loads and stores there and on four barriers per step; here a
+// step has two.  The arrays are indexed statically: every step works on register column 0 and
+// writes the updated columns one place to the left, so after 32 steps the columns are back in
+// order (a panel of kb < 32 columns ends with 32 - kb plain rotations).  Interchanges move no
+// data: each thread carries the position of its row, and the rows are stored to their
+// positions at the end.  The candidate of the next step's pivot is formed from the first column
+// updated, so its warp reduction overlaps the other 31 columns' arithmetic.
+// Bound: issue slots, 128 FMA per row and step, and the latency of the pivot chain (two
+// barriers, one reciprocal).  Pivots, their ties (lowest position) and every element's
+// operations are those of panel_factor, so the panel is bitwise the same.
+// Measured on GB300 (panel alone, 32 matrices): MEASURE_PANEL
+constexpr int RP_MAX_N = 640;   // 640 threads of up to 102 registers
+constexpr int RP_C = 32;
+template <int MAXT>   // threads at most: 512 (128 registers each) or RP_MAX_N (96)
+__global__ void __launch_bounds__(MAXT, 1) gj_panel_reg_kernel(float2* A, long long sA, int n, int k0, int kb,
+                                                                   int* ipiv, int* info, int* moves) {
+  __shared__ __align__(16) float2 raw[RP_C], piv[RP_C];   // pivot row, unscaled and scaled
+  __shared__ unsigned w_key[RP_MAX_N / 32];
+  __shared__ int w_pos[RP_MAX_N / 32];
+  __shared__ int s_extra;
+  const int b = blockIdx.x;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5, nwarps = blockDim.x >> 5;
+  float2* Ab = A + (long long)b * sA;
+  int* ip = ipiv + (long long)b * n;
+  float2 row[RP_C];
+  const bool live = t < n;
+#pragma unroll
+  for (int j = 0; j < RP_C; ++j)
+    row[j] = (live && j < kb) ? Ab[(long long)(k0 + j) * n + t] : make_float2(0.f, 0.f);
+  int pos = live ? t : 0x7fffffff;
+  if (t == 0) s_extra = kb;
+  // key of a pivot candidate: larger |re|+|im| first (non-negative floats order as their bits),
+  // 0 = no candidate (a row above the step, a NaN)
+  auto key_of = [&](float2 v, int r) -> unsigned {
+    const float a = cabs1(v);
+    return (live && pos >= r && a == a) ? __float_as_uint(a) + 1u : 0u;
+  };
+  unsigned key = key_of(row[0], k0);
+  unsigned wmax = __reduce_max_sync(0xffffffffu, key);
+#pragma unroll 1
+  for (int c = 0; c < kb; ++c) {
+    const int r = k0 + c;
+    const int wpos = __reduce_min_sync(0xffffffffu, key == wmax ? pos : 0x7fffffff);
+    if (lane == 0) { w_key[warp] = wmax; w_pos[warp] = wpos; }
+    __syncthreads();
+    const unsigned ck = lane < nwarps ? w_key[lane] : 0u;
+    const unsigned best = __reduce_max_sync(0xffffffffu, ck);
+    int p = __reduce_min_sync(0xffffffffu, (lane < nwarps && ck == best) ? w_pos[lane] : 0x7fffffff);
+    if (best == 0u) p = r;
+    const bool own = pos == p;
+    if (__any_sync(0xffffffffu, own)) {
+      // the owner's warp scales the pivot row, one element per lane
+      if (own) {
+#pragma unroll
+        for (int j = 0; j < RP_C; j += 2)
+          *reinterpret_cast<float4*>(&raw[j]) = make_float4(row[j].x, row[j].y, row[j + 1].x, row[j + 1].y);
+        ip[r] = p;
+        if (row[0].x == 0.f && row[0].y == 0.f && info[b] == 0) info[b] = r + 1;
+      }
+      __syncwarp();
+      const float2 pv = raw[0];
+      const float2 d = (pv.x == 0.f && pv.y == 0.f) ? make_float2(0.f, 0.f) : crcp(pv);
+      piv[lane] = lane == 0 ? d : cmul(raw[lane], d);
+    }
+    __syncthreads();
+    if (own) pos = r;
+    else if (pos == r) pos = p;
+    const float4 p01 = *reinterpret_cast<const float4*>(&piv[0]);
+    const float2 d = make_float2(p01.x, p01.y);
+    if (d.x == 0.f && d.y == 0.f) {   // no pivot: the interchange only
+      const float2 first = row[0];
+#pragma unroll
+      for (int j = 0; j < RP_C - 1; ++j) row[j] = row[j + 1];
+      row[RP_C - 1] = first;
+      key = key_of(row[0], r + 1);
+      wmax = __reduce_max_sync(0xffffffffu, key);
+      continue;
+    }
+    const float2 f = row[0];
+    auto step = [&](float2 v, float2 rv) -> float2 {
+      v.x = fmaf(-f.x, rv.x, v.x);
+      v.x = fmaf(f.y, rv.y, v.x);
+      v.y = fmaf(-f.x, rv.y, v.y);
+      v.y = fmaf(-f.y, rv.x, v.y);
+      return v;
+    };
+    row[0] = own ? make_float2(p01.z, p01.w) : step(row[1], make_float2(p01.z, p01.w));
+    key = key_of(row[0], r + 1);
+    wmax = __reduce_max_sync(0xffffffffu, key);
+    if (own) {   // the pivot row itself: one warp of the CTA takes both branches
+#pragma unroll
+      for (int j = 2; j < RP_C; ++j) row[j - 1] = piv[j];
+      row[RP_C - 1] = d;
+    } else {
+#pragma unroll
+      for (int j = 2; j < RP_C; j += 2) {
+        const float4 q = *reinterpret_cast<const float4*>(&piv[j]);
+        row[j - 1] = step(row[j], make_float2(q.x, q.y));
+        row[j] = step(row[j + 1], make_float2(q.z, q.w));
+      }
+      row[RP_C - 1] = cmul(make_float2(-f.x, -f.y), d);
+    }
+  }
+#pragma unroll 1
+  for (int c = kb; c < RP_C; ++c) {
+    const float2 first = row[0];
+#pragma unroll
+    for (int j = 0; j < RP_C - 1; ++j) row[j] = row[j + 1];
+    row[RP_C - 1] = first;
+  }
+  // the panel's interchanges as (destination, origin) rows for gj_swap, the rows K first: at
+  // most kb of the others moved
+  int* mv = moves + (long long)b * GJ_MOVES;
+  if (live) {
+#pragma unroll
+    for (int j = 0; j < RP_C; ++j)
+      if (j < kb) Ab[(long long)(k0 + j) * n + pos] = row[j];
+    const int q = (pos >= k0 && pos < k0 + kb) ? pos - k0 : (pos != t ? atomicAdd(&s_extra, 1) : -1);
+    if (q >= 0) {
+      mv[1 + 2 * q] = pos;
+      mv[2 + 2 * q] = t;
+    }
+  }
+  __syncthreads();
+  if (t == 0) mv[0] = s_extra;
+}
+
 // Row interchanges of one panel for the columns outside it, and the copy of rows K into R.
-// The kb interchanges (r, ip[r]) of the panel touch at most 2 kb rows.  Thread 0 of each
-// CTA composes them once into a gather list over the touched rows (row trow[t] receives the
-// value of row torig[t]); then one warp per column loads its touched values (all loads
+// The kb interchanges (r, ip[r]) of the panel touch at most 2 kb rows.  The register panel
+// leaves them composed as a gather list over the touched rows (row trow[t] receives the value
+// of row torig[t]); after the shared-memory panel thread 0 of each CTA composes it.  Then one warp per column loads its touched values (all loads
 // before any store, so the gather is a simultaneous permutation), writes rows K to R
 // (kb x n, column-major) with zeros in A, and the other touched rows back in place.
 // Panel columns get R = 0.
 constexpr int SWAP_WARPS = 8;
 template <typename T>
 __global__ void __launch_bounds__(SWAP_WARPS * 32) gj_swap_kernel(T* A, long long sA, int n, int k0, int kb,
-                                                                  const int* ipiv, T* R, long long sR) {
+                                                                  const int* ipiv, const int* moves, T* R,
+                                                                  long long sR) {
   __shared__ int trow[64], torig[64];
   __shared__ int s_nt;
   const int b = blockIdx.y;
   T* Ab = A + (long long)b * sA;
   const int* ip = ipiv + (long long)b * n;
   T* Rb = R + (long long)b * sR;
-  if (threadIdx.x == 0) {
+  if (moves) {   // the panel kernel composed the list
+    const int* mv = moves + (long long)b * GJ_MOVES;
+    if (threadIdx.x < 64 && (int)threadIdx.x < mv[0]) {
+      trow[threadIdx.x] = mv[1 + 2 * threadIdx.x];
+      torig[threadIdx.x] = mv[2 + 2 * threadIdx.x];
+    }
+    if (threadIdx.x == 0) s_nt = mv[0];
+  } else if (threadIdx.x == 0) {
     int nt = kb;
     for (int c = 0; c < kb; ++c) { trow[c] = k0 + c; torig[c] = k0 + c; }
     for (int c = 0; c < kb; ++c) {
@@ -580,13 +719,14 @@ int inv_work_alloc(InvWork& w, int n, int batch, cudaMemPool_t pool, cudaStream_
   if (!get((void**)&w.rbuf, sizeof(double2) * (size_t)batch * w.nb * n)) return NEGF_ENOMEM;
   if (!get((void**)&w.ipiv, sizeof(int) * (size_t)batch * n)) return NEGF_ENOMEM;
   if (!get((void**)&w.info, sizeof(int) * (size_t)batch)) return NEGF_ENOMEM;
+  if (!get((void**)&w.moves, sizeof(int) * (size_t)batch * kGjMoves)) return NEGF_ENOMEM;
   w.n_cap = n;
   w.batch_cap = batch;
   return NEGF_OK;
 }
 
 void inv_work_free(InvWork& w, cudaStream_t st) {
-  for (void* p : {(void*)w.rbuf, (void*)w.ipiv, (void*)w.info})
+  for (void* p : {(void*)w.rbuf, (void*)w.ipiv, (void*)w.info, (void*)w.moves})
     if (p) {
       if (w.pooled) cudaFreeAsync(p, st);
       else cudaFree(p);
@@ -646,11 +786,19 @@ int gj_invert(T* A, long long sA, int n, int batch, InvWork& w, cudaStream_t st)
     const int kb = (n - k0 < nb) ? (n - k0) : nb;
     cudaEvent_t ev;
     timed_begin(st, TK_PANEL, 8.0 * n * (double)kb * kb * batch, &ev);
-    gj_panel_kernel<T><<<batch, PANEL_THREADS, smem, st>>>(A, sA, n, k0, kb, w.ipiv, w.info);
+    const int* moves = nullptr;
+    if (sizeof(T) == 8 && n <= RP_MAX_N) {
+      const int threads = (n + 31) / 32 * 32;
+      auto panel = threads <= 512 ? gj_panel_reg_kernel<512> : gj_panel_reg_kernel<RP_MAX_N>;
+      panel<<<batch, threads, 0, st>>>(reinterpret_cast<float2*>(A), sA, n, k0, kb, w.ipiv, w.info, w.moves);
+      moves = w.moves;
+    } else {
+      gj_panel_kernel<T><<<batch, PANEL_THREADS, smem, st>>>(A, sA, n, k0, kb, w.ipiv, w.info);
+    }
     NEGF_CUDA_TRY(cudaGetLastError());
     timed_end(st, TK_PANEL, ev);
     dim3 g2((n + SWAP_WARPS - 1) / SWAP_WARPS, batch);
-    gj_swap_kernel<T><<<g2, SWAP_WARPS * 32, 0, st>>>(A, sA, n, k0, kb, w.ipiv, rbuf, sR);
+    gj_swap_kernel<T><<<g2, SWAP_WARPS * 32, 0, st>>>(A, sA, n, k0, kb, w.ipiv, moves, rbuf, sR);
     NEGF_CUDA_TRY(cudaGetLastError());
     count_launch(2);
     // A(:, j) += P R(:, j) for the columns outside the panel

@@ -147,10 +147,12 @@ int cgemm_f32(const GemmBatchT<float2>& g, cudaStream_t st);   // FP32 twin (inv
 // ----------------------------------------------------------------------------------
 // Batched in-place inverse (blocked Gauss-Jordan with partial row pivoting)
 // ----------------------------------------------------------------------------------
+constexpr int kGjMoves = 1 + 2 * 64;
 struct InvWork {
   double2* rbuf = nullptr;   // batch * nb * n (FP64; reused as float2 storage by the FP32 form)
   int* ipiv = nullptr;       // batch * n
   int* info = nullptr;       // batch
+  int* moves = nullptr;      // batch * kGjMoves: the interchanges of the panel at hand (FP32 form)
   int n_cap = 0, batch_cap = 0, nb = 0;
   bool pooled = false;       // allocated stream-ordered from a memory pool
 };

@@ -1,0 +1,39 @@
+"""Edges of the device kernels' size ranges, against the oracle."""
+import numpy as np
+import pytest
+
+from nonequilibriumgreensfunction_gb300 import Solver, hamiltonian
+from oracle import negf_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def _one_energy(npx, npy, npz, precision, energy=0.11, eta=1e-3):
+    htotd, hopx = hamiltonian.ti_wire(npx, npy, npz, W=0.1, seed=3, flux=0.4, zeeman=0.01)
+    with Solver(npx, npy, npz, eta=eta, sr_tol=1e-10, precision=precision) as s:
+        s.set_hamiltonian(htotd, hopx)
+        rho = s.new_site_array(1)
+        got = s.solve_batch([energy], 0.7, 0.2, 1e-3, rho_n=rho)
+    opt = O.SolveOptions(eta=eta, sr_tol=1e-10)
+    cse = O.contact_self_energy(htotd, hopx, energy, opt)
+    m = htotd.shape[1]
+    inv = np.stack([(energy + 1j * eta) * np.eye(m) - h for h in htotd])
+    inv[0] -= cse["SigmaL"]
+    inv[-1] -= cse["SigmaR"]
+    g = O.get_retarded_greens(inv, hopx)
+    y = g["GRRgt"][0] @ cse["GammaR"] @ g["GRRgt"][0].conj().T
+    t12 = np.real(np.trace(cse["GammaL"] @ y))
+    gnp = O.calculate_gnp(g["GRLef"], g["GRRgt"], cse["GammaL"], cse["GammaR"], 0.7, 0.2, with_offdiag=False)
+    want = O.site_density(gnp["Gnd"], npy, npz) * 1e-3 / (2 * np.pi)
+    assert got["status"][0] == 0
+    return got["T12"][0], t12, rho[..., 0], want
+
+
+# The FP32 panel holds a row per thread: a partial last warp and a last panel of fewer than 32
+# columns (M = 4, 36, 140), the switch from 512 to 640 threads (512, 520), its last size (640)
+# and the shared-memory panel beyond it (644).  Tolerance: the mixed form's 1e-6.
+@pytest.mark.parametrize("npy,npz", [(1, 1), (3, 3), (5, 7), (8, 16), (10, 13), (10, 16), (7, 23)])
+def test_mixed_form_at_the_panel_kernels_sizes(need_gpu, npy, npz):
+    t, want, rho, rho_want = _one_energy(3, npy, npz, "mixed")
+    assert abs(t - want) <= 1e-6 * max(abs(want), 1e-3)
+    assert np.abs(rho - rho_want).max() <= 1e-6 * np.abs(rho_want).max()
