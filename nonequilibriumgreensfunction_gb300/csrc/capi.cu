@@ -278,9 +278,11 @@ int negf_get_retarded_greens(negf_handle* h) {
   items[0] = negf::Item{e.cur_energy_, 0.0, 0.0, 0.0, 0, h->sr_l, h->sr_r, 0};
   e.rgf_valid_ = e.dens_valid_ = false;
   NEGF_TRY(e.solve_rgf(items, e.keep_columns_));
-  int st = 0;
+  int st = 0, tc_err = 0;
   NEGF_CUDA_TRY(cudaMemcpyAsync(&st, e.dStatus_, sizeof(int), cudaMemcpyDeviceToHost, e.st_));
+  NEGF_TRY(e.read_tc_error(&tc_err));
   NEGF_CUDA_TRY(cudaStreamSynchronize(e.st_));
+  if (tc_err) return NEGF_ETIMEDOUT;
   e.cur_rgf_status_ = st;
   e.rgf_valid_ = true;
   return st;

@@ -154,13 +154,18 @@ Engine::~Engine() {
   dfree(dSrCmax_, s); dfree(dSrDos_, s); dfree(dSrActive_, s); dfree(dSrE_, s); dfree(dSrHend_, s);
   dfree(dSrStatus_, s);
   inv_work_free(inv_, s);
+  free_tc();
+  cudaStreamSynchronize(own_st_);   // the frees have run: the blocks are back in the pool
+  pinned_give(hPin_, hPinBytes_);
+  cudaStreamDestroy(own_st_);
+}
+
+void Engine::free_tc() {
+  cudaStream_t s = own_st_;
   dfree(dWinv_, s); dfree(dW32_, s); dfree(dT_, s); dfree(sa_.data, s); dfree(sb_.data, s); dfree(sa_.exps, s);
   dfree(sb_.exps, s); dfree(sw_.data, s); dfree(sw_.exps, s); dfree(sgl_.data, s); dfree(sgl_.exps, s);
   dfree(sgr_.data, s); dfree(sgr_.exps, s);
   dfree(dRnorm_, s); dfree(dNsIdx_, s); dfree(dNsX_, s); dfree(dNsW_, s); dfree(dTcErr_, s);
-  cudaStreamSynchronize(own_st_);   // the frees have run: the blocks are back in the pool
-  pinned_give(hPin_, hPinBytes_);
-  cudaStreamDestroy(own_st_);
 }
 
 int pool_trim(int device) {
@@ -209,11 +214,34 @@ int Engine::configure(const negf_params& p) {
     if (p.residual_slices < 5 || p.residual_slices > 8) return NEGF_EINVAL;
     s_res_ = p.residual_slices;
   }
+  ns_step_[1].res = s_res_;
+  tc_cap_ = std::max(B_, S_);
+  tc_ = mixed_;
+  if (!mixed_ && !lean_ && M_ >= 32 && 2 * padded_k(M_) <= 1600) {
+    // The FP64 form on GB300's tensor cores: its FP64 pipe does two multiply-adds per clock and
+    // SM, the nine-slice product of 45 BF16 slice pairs about 25 times that (400^3: 0.4 ms
+    // against 10 ms for 64 products).  Below M = 32 the launches of the sliced path cost more
+    // than the arithmetic (M = 2: 46 against 28 ms an energy; M = 36: 11 against 34 ms).  Each step's residual is as fine as the step's result has to be: FP32
+    // Gauss-Jordan leaves ~1e-3, and the steps ~1e-7, ~1e-12 and the rounding of a double.
+    tc_ = true;
+    s_rgf_ = s_sr_ = s_res_ = 9;
+    ns_step_[0] = {5, 3};
+    ns_step_[1] = {7, 4};
+    ns_step_[2] = {9, 4};
+    s_upd_ = 4;
+    ns_steps_ = 3;
+    ns_max_steps_ = 6;
+    ns_tol_ = 1e-9;   // squared by the last update: below a double's rounding
+    // about 300 M^2 bytes a matrix: at most some 3 GB of workspace, and at least 32 matrices
+    const long long fit = 10000000 / std::max<long long>(MM_, 1);
+    tc_cap_ = (int)std::min<long long>(tc_cap_, std::max<long long>(fit, 32));
+  }
   return NEGF_OK;
 }
 
-long long Engine::estimate_bytes(const negf_params& p) {
+long long Engine::estimate_bytes(const negf_params& p, bool lean) {
   Engine e;
+  e.lean_ = lean;
   if (e.configure(p) != NEGF_OK) return -1;
   e.dry_ = true;
   if (e.alloc() != NEGF_OK) return -1;
@@ -294,34 +322,18 @@ int Engine::alloc() {
     if (!dry_) NEGF_TRY(inv_work_alloc(inv_, M_, (int)cap, pool_, own_st_));
     bytes_ += 16LL * cap * panel_width(M_) * M_ + 4LL * cap * M_ + 4LL * cap + 4LL * cap * kGjMoves;
   }
-  if (mixed_) {
-    const int cap = std::max(B_, S_);
-    const int smax = 8;   // every slice count a phase may use (RGF, Sancho-Rubio, residual: <= 8)
-    NEGF_TRY(dalloc(&dWinv_, (size_t)(cap * MM_), bytes_, dry_, pool_, own_st_));
-    NEGF_TRY(dalloc(&dW32_, (size_t)(cap * MM_), bytes_, dry_, pool_, own_st_));
-    NEGF_TRY(dalloc(&dT_, (size_t)(cap * MM_), bytes_, dry_, pool_, own_st_));
-    const int kp = padded_k(M_);
-    NEGF_TRY(dalloc(reinterpret_cast<char**>(&sa_.data), sliced_bytes_a(M_, kp, smax, cap), bytes_, dry_, pool_, own_st_));
-    NEGF_TRY(dalloc(reinterpret_cast<char**>(&sb_.data), sliced_bytes_b(M_, kp, smax, cap), bytes_, dry_, pool_, own_st_));
-    NEGF_TRY(dalloc(reinterpret_cast<char**>(&sw_.data), sliced_bytes_a(M_, kp, smax, cap), bytes_, dry_, pool_, own_st_));
-    NEGF_TRY(dalloc(&sw_.exps, (size_t)cap * M_, bytes_, dry_, pool_, own_st_));
-    NEGF_TRY(dalloc(&sa_.exps, (size_t)cap * M_, bytes_, dry_, pool_, own_st_));
-    NEGF_TRY(dalloc(&sb_.exps, (size_t)cap * M_, bytes_, dry_, pool_, own_st_));
-    NEGF_TRY(dalloc(reinterpret_cast<char**>(&sgl_.data), sliced_bytes_b(M_, kp, s_rgf_, B_), bytes_, dry_, pool_, own_st_));
-    NEGF_TRY(dalloc(reinterpret_cast<char**>(&sgr_.data), sliced_bytes_b(M_, kp, s_rgf_, B_), bytes_, dry_, pool_, own_st_));
-    NEGF_TRY(dalloc(&sgl_.exps, (size_t)B_ * M_, bytes_, dry_, pool_, own_st_));
-    NEGF_TRY(dalloc(&sgr_.exps, (size_t)B_ * M_, bytes_, dry_, pool_, own_st_));
-    sgl_.data_bytes = sgr_.data_bytes = sliced_bytes_b(M_, kp, s_rgf_, B_);
-    sgl_.exps_count = sgr_.exps_count = (size_t)B_ * M_;
-    sa_.data_bytes = sw_.data_bytes = sliced_bytes_a(M_, kp, smax, cap);
-    sb_.data_bytes = sliced_bytes_b(M_, kp, smax, cap);
-    sa_.exps_count = sb_.exps_count = sw_.exps_count = (size_t)cap * M_;
-    NEGF_TRY(dalloc(&dRnorm_, (size_t)cap, bytes_, dry_, pool_, own_st_));
-    NEGF_TRY(dalloc(&dNsIdx_, (size_t)cap, bytes_, dry_, pool_, own_st_));
-    NEGF_TRY(dalloc(&dNsX_, (size_t)cap * MM_, bytes_, dry_, pool_, own_st_));
-    NEGF_TRY(dalloc(&dNsW_, (size_t)cap * MM_, bytes_, dry_, pool_, own_st_));
-    NEGF_TRY(dalloc(&dTcErr_, (size_t)1, bytes_, dry_, pool_, own_st_));
-    if (!dry_) NEGF_CUDA_TRY(cudaMemsetAsync(dTcErr_, 0, sizeof(int), own_st_));
+  if (tc_) {
+    const long long before = bytes_;
+    int rc = alloc_tc();
+    if (rc == NEGF_ENOMEM && !mixed_) {   // the FP64 form runs without it
+      free_tc();
+      NEGF_CUDA_TRY(cudaStreamSynchronize(own_st_));
+      cudaGetLastError();   // (the failed allocation)
+      bytes_ = before;
+      tc_ = false;
+      rc = NEGF_OK;
+    }
+    NEGF_TRY(rc);
   }
   if (dry_) return NEGF_OK;   // estimate_bytes: device bytes only
   hPinBytes_ = sizeof(double) * (size_t)std::max<long long>(
@@ -366,6 +378,37 @@ int Engine::alloc() {
     at(2, 0, 0) = one; at(2, 1, 1) = m1;
   }
   NEGF_CUDA_TRY(cudaMemcpy(dSpin_, spin.data(), sizeof(double2) * spin.size(), cudaMemcpyHostToDevice));
+  return NEGF_OK;
+}
+
+int Engine::alloc_tc() {
+  const int cap = tc_cap_, gcap = std::min(B_, cap);
+  const int smax = mixed_ ? 8 : 9;   // every slice count a phase may use (RGF, Sancho-Rubio, residual)
+  NEGF_TRY(dalloc(&dWinv_, (size_t)(cap * MM_), bytes_, dry_, pool_, own_st_));
+  NEGF_TRY(dalloc(&dW32_, (size_t)(cap * MM_), bytes_, dry_, pool_, own_st_));
+  NEGF_TRY(dalloc(&dT_, (size_t)(cap * MM_), bytes_, dry_, pool_, own_st_));
+  const int kp = padded_k(M_);
+  NEGF_TRY(dalloc(reinterpret_cast<char**>(&sa_.data), sliced_bytes_a(M_, kp, smax, cap), bytes_, dry_, pool_, own_st_));
+  NEGF_TRY(dalloc(reinterpret_cast<char**>(&sb_.data), sliced_bytes_b(M_, kp, smax, cap), bytes_, dry_, pool_, own_st_));
+  NEGF_TRY(dalloc(reinterpret_cast<char**>(&sw_.data), sliced_bytes_a(M_, kp, smax, cap), bytes_, dry_, pool_, own_st_));
+  NEGF_TRY(dalloc(&sw_.exps, (size_t)cap * M_, bytes_, dry_, pool_, own_st_));
+  NEGF_TRY(dalloc(&sa_.exps, (size_t)cap * M_, bytes_, dry_, pool_, own_st_));
+  NEGF_TRY(dalloc(&sb_.exps, (size_t)cap * M_, bytes_, dry_, pool_, own_st_));
+  NEGF_TRY(dalloc(reinterpret_cast<char**>(&sgl_.data), sliced_bytes_b(M_, kp, s_rgf_, gcap), bytes_, dry_, pool_, own_st_));
+  NEGF_TRY(dalloc(reinterpret_cast<char**>(&sgr_.data), sliced_bytes_b(M_, kp, s_rgf_, gcap), bytes_, dry_, pool_, own_st_));
+  NEGF_TRY(dalloc(&sgl_.exps, (size_t)gcap * M_, bytes_, dry_, pool_, own_st_));
+  NEGF_TRY(dalloc(&sgr_.exps, (size_t)gcap * M_, bytes_, dry_, pool_, own_st_));
+  sgl_.data_bytes = sgr_.data_bytes = sliced_bytes_b(M_, kp, s_rgf_, gcap);
+  sgl_.exps_count = sgr_.exps_count = (size_t)gcap * M_;
+  sa_.data_bytes = sw_.data_bytes = sliced_bytes_a(M_, kp, smax, cap);
+  sb_.data_bytes = sliced_bytes_b(M_, kp, smax, cap);
+  sa_.exps_count = sb_.exps_count = sw_.exps_count = (size_t)cap * M_;
+  NEGF_TRY(dalloc(&dRnorm_, (size_t)cap, bytes_, dry_, pool_, own_st_));
+  NEGF_TRY(dalloc(&dNsIdx_, (size_t)cap, bytes_, dry_, pool_, own_st_));
+  NEGF_TRY(dalloc(&dNsX_, (size_t)cap * MM_, bytes_, dry_, pool_, own_st_));
+  NEGF_TRY(dalloc(&dNsW_, (size_t)cap * MM_, bytes_, dry_, pool_, own_st_));
+  NEGF_TRY(dalloc(&dTcErr_, (size_t)1, bytes_, dry_, pool_, own_st_));
+  if (!dry_) NEGF_CUDA_TRY(cudaMemsetAsync(dTcErr_, 0, sizeof(int), own_st_));
   return NEGF_OK;
 }
 
@@ -460,26 +503,51 @@ void Engine::recompute_lead_classes() {
   }
 }
 
-int Engine::gemm_tc_nn(int batch, const double2* A, long long sA, const double2* B, long long sB, double2* C,
-                       long long sC, double2 alpha, double2 beta, int slices) {
-  NEGF_TRY(slice_a(A, M_, sA, M_, M_, batch, slices, sa_, st_));
-  NEGF_TRY(slice_b(B, M_, sB, M_, M_, batch, slices, sb_, st_));
-  return zgemm_tc(sa_, sb_, alpha, beta, C, M_, sC, dTcErr_, st_);
+SlicedOperand Engine::view(const SlicedOperand& o, int first, int count) {
+  SlicedOperand v = o;
+  const size_t plane = (size_t)o.slices * o.rows * 2 * (size_t)o.k;
+  const size_t nexp = o.batch > 0 ? o.exps_used / (size_t)o.batch : 0;
+  v.data = o.data + plane * (size_t)first;
+  v.exps = o.exps + nexp * (size_t)first;
+  v.exps_used = nexp * (size_t)count;
+  v.batch = count;
+  if (v.src) v.src += o.sSrc * first;
+  return v;
 }
 
-// C = A G with G's B-operand slicing made once per sweep (Gamma_L, Gamma_R); FP64 form:
-// a plain product with G itself
+// The error flag of the tensor-core products so far (a bounded wait that ran out), read and
+// cleared in stream order: *err is valid after the caller's next synchronisation
+int Engine::read_tc_error(int* err) {
+  if (!tc_) return NEGF_OK;
+  NEGF_CUDA_TRY(cudaMemcpyAsync(err, dTcErr_, sizeof(int), cudaMemcpyDeviceToHost, st_));
+  NEGF_CUDA_TRY(cudaMemsetAsync(dTcErr_, 0, sizeof(int), st_));
+  return NEGF_OK;
+}
+
+int Engine::gemm_tc_nn(int batch, const double2* A, long long sA, const double2* B, long long sB, double2* C,
+                       long long sC, double2 alpha, double2 beta, int slices) {
+  for (int o = 0; o < batch; o += tc_cap_) {
+    const int nb = std::min(tc_cap_, batch - o);
+    NEGF_TRY(slice_a(A + o * sA, M_, sA, M_, M_, nb, slices, sa_, st_));
+    NEGF_TRY(slice_b(B + o * sB, M_, sB, M_, M_, nb, slices, sb_, st_));
+    NEGF_TRY(zgemm_tc(sa_, sb_, alpha, beta, C + o * sC, M_, sC, dTcErr_, st_));
+  }
+  return NEGF_OK;
+}
+
+// C = A G with G's B-operand slicing made once per sweep (Gamma_L, Gamma_R); without the
+// tensor cores, or for a batch in pieces, a plain product with G itself
 int Engine::gemm_gamma(int batch, const double2* A, long long sA, const double2* G, const SlicedOperand& sg,
                        double2* C, long long sC) {
   const double2 one = make_double2(1, 0), zero = make_double2(0, 0);
-  if (!mixed_) return gemm(batch, OP_N, A, sA, OP_N, G, MM_, C, sC, one, zero);
+  if (!tc_ || batch > tc_cap_) return gemm(batch, OP_N, A, sA, OP_N, G, MM_, C, sC, one, zero);
   NEGF_TRY(slice_a(A, M_, sA, M_, M_, batch, s_rgf_, sa_, st_));
   return zgemm_tc(sa_, sg, one, zero, C, M_, sC, dTcErr_, st_);
 }
 
 int Engine::gemm(int batch, Op opA, const double2* A, long long sA, Op opB, const double2* B, long long sB, double2* C,
                  long long sC, double2 alpha, double2 beta) {
-  if (mixed_ && opA == OP_N && opB == OP_N && sA != 0 && sB != 0)
+  if (tc_ && opA == OP_N && opB == OP_N && sA != 0 && sB != 0)
     return gemm_tc_nn(batch, A, sA, B, sB, C, sC, alpha, beta, cur_slices_);
   GemmBatch g{};
   g.m = M_; g.n = M_; g.k = M_;
@@ -503,10 +571,11 @@ int Engine::hop_mul(int left, Op op, const double2* X, long long sX, double2* Y,
 int Engine::merge_info(int batch) { return merge_info_kernel_launch(batch, inv_.info, dStatus_, st_); }
 
 // In-place inverse of `batch` matrices at stride sA; INFO of singular ones merged into
-// status_dev.  FP64 form: blocked Gauss-Jordan.  Mixed form: FP32 Gauss-Jordan, then
-// ns_steps_ Newton-Schulz steps X <- X + X (I - W X) with W X formed at s_res_ slices
-// (FP64-class) and X R at s_upd_ slices, and up to ns_max_steps_ in all for a matrix whose
-// residual norm before its last update is above ns_tol_.  A matrix is inverted again in
+// status_dev.  Without the tensor cores: blocked FP64 Gauss-Jordan.  With them: FP32
+// Gauss-Jordan, then ns_steps_ Newton-Schulz steps X <- X + X (I - W X) with W X and X R
+// formed at each step's slices (ns_step_; the last residual is FP64-class), and up to
+// ns_max_steps_ in all for a matrix whose residual norm before its last update is above
+// ns_tol_.  A matrix is inverted again in
 // FP64 when its first residual norm is above ns_accept_, its FP32 factorisation met a zero
 // pivot, or it is still above ns_tol_ after ns_max_steps_ steps.
 int Engine::invert(double2* A, long long sA, int batch, int* status_dev) {
@@ -518,10 +587,16 @@ int Engine::invert(double2* A, long long sA, int batch, int* status_dev) {
 }
 
 int Engine::invert_impl(double2* A, long long sA, int batch, int* status_dev) {
-  if (!mixed_) {
+  if (!tc_) {
     NEGF_TRY(zinv_f64(A, sA, M_, batch, inv_, st_));
     return merge_info_kernel_launch(batch, inv_.info, status_dev, st_);
   }
+  for (int o = 0; o < batch; o += tc_cap_)
+    NEGF_TRY(invert_refined(A + o * sA, sA, std::min(tc_cap_, batch - o), status_dev + o));
+  return NEGF_OK;
+}
+
+int Engine::invert_refined(double2* A, long long sA, int batch, int* status_dev) {
   const double2 one = make_double2(1, 0), zero = make_double2(0, 0);
   NEGF_TRY(split_copy(M_, batch, A, sA, dWinv_, MM_, dW32_, MM_, st_));
   NEGF_TRY(invert_f32(batch));
@@ -534,9 +609,9 @@ int Engine::invert_impl(double2* A, long long sA, int batch, int* status_dev) {
   // ns_steps_ steps for the whole batch
   for (int step = 0; step < ns_steps_; ++step) {
     if (step > 0) NEGF_CUDA_TRY(cudaMemsetAsync(dRnorm_, 0, sizeof(unsigned long long) * batch, st_));
-    // the first residual only has to be good to the square root of the target (the next
-    // step squares the error), so it takes s_res0_ slices: the leading planes of W's slicing
-    const int sr = (step == 0 && ns_steps_ > 1) ? s_res0_ : s_res_;
+    // an early residual only has to be good to the square root of the next step's target
+    // (that step squares the error): it takes the leading planes of W's slicing
+    const int sr = ns_step_[step].res, su = ns_step_[step].upd;
     NEGF_TRY(slice_b(A, M_, sA, M_, M_, batch, sr, sb_, st_));
     NEGF_TRY(zgemm_tc(sw_, sb_, one, zero, dT_, M_, MM_, dTcErr_, st_, sr));    // T = W X
     NEGF_TRY(ns_residual(M_, batch, dT_, MM_, dRnorm_, st_));                     // R = I - T
@@ -544,8 +619,8 @@ int Engine::invert_impl(double2* A, long long sA, int batch, int* status_dev) {
       NEGF_CUDA_TRY(cudaMemcpyAsync(r0.data(), dRnorm_, sizeof(unsigned long long) * batch, cudaMemcpyDeviceToHost, st_));
     if (step == ns_steps_ - 1)
       NEGF_CUDA_TRY(cudaMemcpyAsync(rk.data(), dRnorm_, sizeof(unsigned long long) * batch, cudaMemcpyDeviceToHost, st_));
-    NEGF_TRY(slice_a(A, M_, sA, M_, M_, batch, s_upd_, sa_, st_));
-    NEGF_TRY(slice_b(dT_, M_, MM_, M_, M_, batch, s_upd_, sb_, st_));
+    NEGF_TRY(slice_a(A, M_, sA, M_, M_, batch, su, sa_, st_));
+    NEGF_TRY(slice_b(dT_, M_, MM_, M_, M_, batch, su, sb_, st_));
     // X += X R; dT_ (R, already sliced) lends itself as the autotuner's scratch output
     NEGF_TRY(zgemm_tc(sa_, sb_, one, one, A, M_, sA, dTcErr_, st_, 0, dT_));
   }
@@ -721,6 +796,31 @@ int Engine::solve_sr_impl(const std::vector<SrJob>& jobs, std::vector<int>& stat
   auto at = [&](int r, int lead) { return buf(r) + (long long)lo[lead] * sM; };
   auto nlead = [&](int lead) { return hi[lead] > lo[lead] ? hi[lead] - lo[lead] : 0; };
 
+  // The iteration's products have t or t~ (then the new ones) as their right factor: on the
+  // tensor cores each is sliced as a B operand twice an iteration instead of five times, t in
+  // sb_ and t~ in the first half of sw_'s planes (an A operand has twice the rows of a B
+  // operand), which only the inverse uses otherwise; a left factor used twice in a row is
+  // sliced once.
+  const bool shared = tc_ && S <= tc_cap_;
+  SlicedOperand stt = sw_;
+  int sliced_a = -1, sliced_first = 0, sliced_n = 0;   // what sa_ holds
+  auto slice_tt = [&](int rt, int rtt) -> int {
+    sliced_a = -1;   // an inverse or an overwritten buffer may lie between
+    if (!shared) return NEGF_OK;
+    NEGF_TRY(slice_b(buf(rt), M_, sM, M_, M_, S, s_sr_, sb_, st_));
+    return slice_b(buf(rtt), M_, sM, M_, M_, S, s_sr_, stt, st_);
+  };
+  // C = alpha A B + beta C over problems [first, first + n); B is t, t~ or their successors
+  auto mul = [&](int ra, int first, int n, int rb, int rc, double2 al, double2 be) -> int {
+    const long long off = (long long)first * sM;
+    if (!shared) return gemm(n, OP_N, buf(ra) + off, sM, OP_N, buf(rb) + off, sM, buf(rc) + off, sM, al, be);
+    if (sliced_a != ra || sliced_first != first || sliced_n != n)
+      NEGF_TRY(slice_a(buf(ra) + off, M_, sM, M_, M_, n, s_sr_, sa_, st_));
+    sliced_a = ra; sliced_first = first; sliced_n = n;
+    const SlicedOperand& sb = (rb == SR_T || rb == SR_TN) ? sb_ : stt;
+    return zgemm_tc(sa_, n == S ? sb : view(sb, first, n), al, be, buf(rc) + off, M_, sM, dTcErr_, st_);
+  };
+
   // alpha = (E + i eta) I - H_end (:71-74 / :83-86)
   NEGF_TRY(form_alpha(M_, S, dSrE_, dSrHend_, p_.eta, 0.0, buf(SR_ALPHA), sM, st_));
   // g0 = inv(alpha + i eta I) (:141)
@@ -740,6 +840,7 @@ int Engine::solve_sr_impl(const std::vector<SrJob>& jobs, std::vector<int>& stat
   iters.assign(2 * S, 0);
   status.assign(S, 0);
   NEGF_CUDA_TRY(cudaMemcpyAsync(dSrActive_, act.data(), sizeof(int) * 2 * S, cudaMemcpyHostToDevice, st_));
+  NEGF_TRY(slice_tt(SR_T, SR_TT));
   int it = 0;
   auto any_active = [&]() { return std::any_of(act.begin(), act.end(), [](int a) { return a != 0; }); };
   while (any_active() && it < p_.sr_max_iter) {
@@ -747,30 +848,33 @@ int Engine::solve_sr_impl(const std::vector<SrJob>& jobs, std::vector<int>& stat
     // Told_L <- Told_L t~ ; Told_R <- Told_R t  (:157-158, with t <-> t~ for the right lead),
     // each over its lead's problems; W1 then takes the old Told's role, and the problems
     // outside the range keep their (unread) values in the swapped buffers
-    if (nlead(0))
-      NEGF_TRY(gemm(nlead(0), OP_N, at(SR_TOLDL, 0), sM, OP_N, at(SR_TT, 0), sM, at(SR_W1, 0), sM, one, zero));
-    std::swap(role[SR_TOLDL], role[SR_W1]);
-    if (nlead(1))
-      NEGF_TRY(gemm(nlead(1), OP_N, at(SR_TOLDR, 1), sM, OP_N, at(SR_T, 1), sM, at(SR_W1, 1), sM, one, zero));
+    // (the right lead's Told is what the last iteration sliced last)
+    if (nlead(1)) NEGF_TRY(mul(SR_TOLDR, lo[1], nlead(1), SR_T, SR_W1, one, zero));
     std::swap(role[SR_TOLDR], role[SR_W1]);
+    sliced_a = -1;
+    if (nlead(0)) NEGF_TRY(mul(SR_TOLDL, lo[0], nlead(0), SR_TT, SR_W1, one, zero));
+    std::swap(role[SR_TOLDL], role[SR_W1]);
+    sliced_a = -1;
     // tmp = inv(I - t t~ - t~ t) (:160-163)
     NEGF_TRY(set_identity(M_, S, buf(SR_TMP), sM, st_));
-    NEGF_TRY(gemm(S, OP_N, buf(SR_T), sM, OP_N, buf(SR_TT), sM, buf(SR_TMP), sM, mone, one));
-    NEGF_TRY(gemm(S, OP_N, buf(SR_TT), sM, OP_N, buf(SR_T), sM, buf(SR_TMP), sM, mone, one));
+    NEGF_TRY(mul(SR_T, 0, S, SR_TT, SR_TMP, mone, one));
+    NEGF_TRY(mul(SR_TT, 0, S, SR_T, SR_TMP, mone, one));
     NEGF_TRY(inv_merge(buf(SR_TMP)));
+    NEGF_TRY(slice_tt(SR_T, SR_TT));   // (the inverse used their buffers)
     // t <- tmp t t ; t~ <- tmp t~ t~ (:170-176)
-    NEGF_TRY(gemm(S, OP_N, buf(SR_TMP), sM, OP_N, buf(SR_T), sM, buf(SR_W1), sM, one, zero));
-    NEGF_TRY(gemm(S, OP_N, buf(SR_W1), sM, OP_N, buf(SR_T), sM, buf(SR_TN), sM, one, zero));
-    NEGF_TRY(gemm(S, OP_N, buf(SR_TMP), sM, OP_N, buf(SR_TT), sM, buf(SR_W1), sM, one, zero));
-    NEGF_TRY(gemm(S, OP_N, buf(SR_W1), sM, OP_N, buf(SR_TT), sM, buf(SR_TTN), sM, one, zero));
+    NEGF_TRY(mul(SR_TMP, 0, S, SR_T, SR_W1, one, zero));
+    NEGF_TRY(mul(SR_TMP, 0, S, SR_TT, SR_W2, one, zero));
+    NEGF_TRY(mul(SR_W1, 0, S, SR_T, SR_TN, one, zero));
+    NEGF_TRY(mul(SR_W2, 0, S, SR_TT, SR_TTN, one, zero));
+    NEGF_TRY(slice_tt(SR_TN, SR_TTN));
     // change = Told t ; T += change (:178-180), each over its lead's problems
     if (nlead(0)) {
-      NEGF_TRY(gemm(nlead(0), OP_N, at(SR_TOLDL, 0), sM, OP_N, at(SR_TN, 0), sM, at(SR_CHG, 0), sM, one, zero));
+      NEGF_TRY(mul(SR_TOLDL, lo[0], nlead(0), SR_TN, SR_CHG, one, zero));
       NEGF_TRY(sr_accumulate(M_, nlead(0), dSrActive_ + lo[0], at(SR_CHG, 0), sM, at(SR_TL, 0), sM,
                              dSrCmax_ + lo[0], st_));
     }
     if (nlead(1)) {
-      NEGF_TRY(gemm(nlead(1), OP_N, at(SR_TOLDR, 1), sM, OP_N, at(SR_TTN, 1), sM, at(SR_CHG, 1), sM, one, zero));
+      NEGF_TRY(mul(SR_TOLDR, lo[1], nlead(1), SR_TTN, SR_CHG, one, zero));
       NEGF_TRY(sr_accumulate(M_, nlead(1), dSrActive_ + S + lo[1], at(SR_CHG, 1), sM, at(SR_TR, 1), sM,
                              dSrCmax_ + S + lo[1], st_));
     }
@@ -822,8 +926,11 @@ int Engine::solve_sr_impl(const std::vector<SrJob>& jobs, std::vector<int>& stat
     }
   }
   std::vector<int> st(S);
+  int tc_err = 0;
   NEGF_CUDA_TRY(cudaMemcpyAsync(st.data(), dSrStatus_, sizeof(int) * S, cudaMemcpyDeviceToHost, st_));
+  NEGF_TRY(read_tc_error(&tc_err));
   NEGF_CUDA_TRY(cudaStreamSynchronize(st_));
+  if (tc_err) return NEGF_ETIMEDOUT;
   for (int s = 0; s < S; ++s)
     if (status[s] == 0 && st[s] != 0) status[s] = st[s];
   return NEGF_OK;
@@ -914,7 +1021,7 @@ int Engine::solve_rgf_impl(const std::vector<Item>& items, bool keep_columns) {
   NEGF_TRY(gather_blocks(M_, B, dSrSigR_, idx_r, istride, dSigR_, sM, st_));
   NEGF_TRY(gather_blocks(M_, B, dSrGamL_, idx_l, istride, dGamL_, sM, st_));
   NEGF_TRY(gather_blocks(M_, B, dSrGamR_, idx_r, istride, dGamR_, sM, st_));
-  if (mixed_) {   // Gamma is the right factor of every G(:,c) Gamma_c product of the sweep
+  if (tc_ && B <= tc_cap_) {   // Gamma is the right factor of every G(:,c) Gamma_c product of the sweep
     NEGF_TRY(slice_b(dGamL_, M_, sM, M_, M_, B, s_rgf_, sgl_, st_));
     NEGF_TRY(slice_b(dGamR_, M_, sM, M_, M_, B, s_rgf_, sgr_, st_));
   }
@@ -1194,7 +1301,10 @@ int Engine::batch_solve(const negf_request* req, int n, negf_result* res, double
     NEGF_CUDA_TRY(cudaMemcpyAsync(tr.data(), dTr_, sizeof(double) * 4 * nb, cudaMemcpyDeviceToHost, st_));
     if (sc_()) NEGF_CUDA_TRY(cudaMemcpyAsync(trj.data(), dTrJ_, sizeof(double) * nb, cudaMemcpyDeviceToHost, st_));
     NEGF_CUDA_TRY(cudaMemcpyAsync(rst.data(), dStatus_, sizeof(int) * nb, cudaMemcpyDeviceToHost, st_));
+    int tc_err = 0;
+    NEGF_TRY(read_tc_error(&tc_err));
     NEGF_CUDA_TRY(cudaStreamSynchronize(st_));
+    if (tc_err) return NEGF_ETIMEDOUT;
     for (int i = 0; i < nb; ++i) {
       negf_result& o = res[c0 + i];
       const Item& it = items[i];

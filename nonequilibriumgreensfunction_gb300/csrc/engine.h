@@ -34,7 +34,10 @@ class Engine {
   int init(const negf_params& p);
   // device bytes an engine with these parameters allocates at init (< 0: invalid
   // parameters); the serving layer admits engines by it
-  static long long estimate_bytes(const negf_params& p);
+  static long long estimate_bytes(const negf_params& p, bool lean = false);
+  // before init: an FP64 engine without the tensor-core workspace (DFMA products and FP64
+  // inverses), for a budget that does not hold the other
+  void set_lean() { lean_ = true; }
   int set_hamiltonian(int slot, const double* Htotd, const double* HopX);
   // Htotd of `slot` generated on the device from a wire model (Build_Hamiltonian)
   int build_hamiltonian(int slot, const negf_wire_model& m);
@@ -140,16 +143,23 @@ class Engine {
 
   InvWork inv_;
 
-  // mixed form (NEGF_PREC_MIXED): tensor-core GEMMs on S integer BF16 slices, inverses as
-  // FP32 Gauss-Jordan + Newton-Schulz steps with the residual at s_res_ slices
+  // Products on the tensor cores on S integer BF16 slices and inverses as FP32 Gauss-Jordan +
+  // Newton-Schulz steps with the residual at s_res_ slices: the mixed form always; the FP64
+  // form with nine slices (63 bits below each row's or column's maximum, more than a double
+  // holds) and three steps, for M <= 800 when its workspace fits the device.
   bool mixed_ = false;
+  bool tc_ = false;
+  bool lean_ = false;        // FP64 form: no workspace for it
+  int tc_cap_ = 0;           // matrices of one sliced product or inverse; larger batches go in pieces
   int s_rgf_ = 5;      // RGF block products
   int s_sr_ = 8;       // Sancho-Rubio products: 2^-56, the decimation is ill-conditioned near band edges
   int s_res_ = 7;      // Newton-Schulz residual W X (2^-49, FP64-class)
-  int s_res0_ = 5;     // the first residual (2^-35: the second step squares its error)
   int s_upd_ = 3;      // Newton-Schulz update X R: its error, ~sqrt(M) 2^-7S of |X||R|, must stay
                        // well below |R| for quadratic convergence; 2 slices (~1e-3 at M = 400)
                        // broke the mixed-form tolerance, 3 slices (~1e-5) keep it
+  struct NsStep { int res, upd; };   // slices of a step's residual and update
+  static constexpr int kNsFixedMax = 3;
+  NsStep ns_step_[kNsFixedMax] = {{5, 3}, {7, 3}, {0, 0}};   // the steps always taken
   int ns_steps_ = 2;        // Newton-Schulz steps always taken
   int ns_max_steps_ = 4;    // more while the latest residual norm is above ns_tol_
   double ns_tol_ = 1e-5;     // residual norm before the last update; that update squares it
@@ -177,6 +187,7 @@ class Engine {
   std::map<int, int> gj_form_;
   int invert_f32(int batch);
   int invert_impl(double2* A, long long sA, int batch, int* status_dev);
+  int invert_refined(double2* A, long long sA, int batch, int* status_dev);
   int solve_sr_impl(const std::vector<SrJob>& jobs, std::vector<int>& status, std::vector<int>& iters);
   int solve_rgf_impl(const std::vector<Item>& items, bool keep_columns);
   int densities_impl(const std::vector<Item>& items, std::vector<double>& edens, std::vector<double>& hdens);
@@ -204,6 +215,13 @@ class Engine {
   bool dry_ = false;                      // alloc() counts bytes without allocating
   cudaMemPool_t pool_ = nullptr;          // the library's stream-ordered pool on p_.device
   int alloc();
+  int alloc_tc();         // the tensor-core workspace
+ public:
+  int read_tc_error(int* err);
+ private:
+  void free_tc();
+  // items [first, first + count) of a sliced operand
+  static SlicedOperand view(const SlicedOperand& o, int first, int count);
   // Y = op(H) X (left) or X op(H) (right) for every block of a strided batch
   int hop_mul(int left, Op op, const double2* X, long long sX, double2* Y, long long sY, int batch);
   int gemm(int batch, Op opA, const double2* A, long long sA, Op opB, const double2* B, long long sB, double2* C,

@@ -166,7 +166,12 @@ struct negf_server {
       if (wi != workers.end()) {
         w = wi->second.get();
       } else {
-        const long long need = estimate(r->key);
+        long long need = estimate(r->key);
+        bool lean = false;
+        if (need > budget) {   // an FP64 engine also runs without its tensor-core workspace
+          const long long least = negf::Engine::estimate_bytes(engine_params(r->key), true);
+          if (least >= 0 && least <= budget) { need = least; lean = true; }
+        }
         if (need < 0 || need > budget) {
           // a geometry no engine accepts (e.g. M > 800 in the mixed form), or one whose
           // engine alone exceeds the whole budget: it would never be admitted
@@ -190,12 +195,14 @@ struct negf_server {
           auto nw = std::make_unique<Worker>();
           nw->key = r->key;
           nw->eng = std::make_unique<negf::Engine>();
+          if (lean) nw->eng->set_lean();
           const double t0 = now();
           int irc = nw->eng->init(engine_params(r->key));
           if (irc == NEGF_ENOMEM) {
             // the library's pool keeps released engines' blocks for reuse; when they do not
             // fit this engine's buffers, give them back to the device and try once more
             nw->eng = std::make_unique<negf::Engine>();
+            if (lean) nw->eng->set_lean();
             negf::pool_trim(p.device);
             irc = nw->eng->init(engine_params(r->key));
           }

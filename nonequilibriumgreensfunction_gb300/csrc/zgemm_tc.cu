@@ -247,13 +247,25 @@ __device__ __forceinline__ void slice_value(double x, int e, __nv_bfloat16 (&out
   if (ex != 0 && ex != 0x7FF) {                      // zero and subnormals slice to 0
     const unsigned long long m = (bits & ((1ULL << 52) - 1)) | (1ULL << 52);   // x = m 2^(ex - 1075)
     const int r = e - (ex - 1075) - (6 + 7 * (S - 1));                          // F = m 2^-r, r >= 46 - 7(S-1)
-    if (r <= 0) F = (long long)(m << (-r));                                      // S = 8: exact, |F| < 2^55
+    if (r <= 0) F = (long long)(m << (-r));                                      // S >= 8: exact
     else if (r < 64) F = (long long)((m + (1ULL << (r - 1))) >> r);
     if (bits >> 63) F = -F;
   }
   // Balanced digits from the bottom, d_p = F_p - 128 floor((F_p + 64) / 128), in 32-bit
   // arithmetic: the low 28 bits give up to four digits and a carry into F >> 28 (|F| < 2^55,
   // so that part fits an int).  The digits are unique, so this equals the 64-bit recurrence.
+  if constexpr (S == 9) {   // |F| <= 2^62: four digits, four more, and what is left
+    int w = (int)(F & ((1LL << 28) - 1));
+#pragma unroll
+    for (int p = 8; p >= 1; --p) {
+      if (p == 4) w += (int)((F >> 28) & ((1LL << 28) - 1));
+      const int nx = (w + 64) >> 7;
+      out[p] = __float2bfloat16_rn((float)(w - nx * 128));
+      w = nx;
+    }
+    out[0] = __float2bfloat16_rn((float)(w + (int)(F >> 56)));
+    return;
+  }
   int hi = (int)(F >> 28);
   int lo = (int)(F & ((1LL << 28) - 1));
   constexpr int NL = S - 1 < 4 ? S - 1 : 4;   // digits taken from the low word
@@ -299,8 +311,22 @@ __device__ __forceinline__ int scale_exponent(unsigned long long a) {
   return E - 1022;
 }
 
+// Nine-slice operands stand in for FP64 products: a row or column that the integers do not
+// hold as FP64 does -- an infinity or a NaN in it, or a maximum near the underflow threshold --
+// has this exponent instead, and the epilogue forms its products with FP64 multiply-adds.
+constexpr int EXP_DIRECT = 1 << 20;
+__device__ __forceinline__ unsigned long long abs_bits_all(double x) {   // NaN above infinity
+  return (unsigned long long)__double_as_longlong(x) & 0x7FFFFFFFFFFFFFFFULL;
+}
+__device__ __forceinline__ int scale_exponent_strict(unsigned long long a) {
+  const int E = (int)(a >> 52);
+  if (a == 0) return 0;
+  return (E == 0x7FF || E < 200) ? EXP_DIRECT : E - 1022;
+}
+
 // row exponents of A (M x K complex, column-major): a CTA covers 32 rows, its 8 thread
 // rows stride over the columns (coalesced 512-byte row segments), reduced in shared memory
+template <bool STRICT>
 __global__ void row_exp_kernel(const double2* A, int lda, long long sA, int m, int k, int* ea) {
   __shared__ unsigned long long part[8][32];
   const int b = blockIdx.y;
@@ -311,13 +337,14 @@ __global__ void row_exp_kernel(const double2* A, int lda, long long sA, int m, i
   if (i < m)
     for (int kk = ty; kk < k; kk += 8) {
       const double2 v = Ab[(long long)kk * lda + i];
-      mx = max(mx, max(abs_bits(v.x), abs_bits(v.y)));
+      if (STRICT) mx = max(mx, max(abs_bits_all(v.x), abs_bits_all(v.y)));
+      else mx = max(mx, max(abs_bits(v.x), abs_bits(v.y)));
     }
   part[ty][tx] = mx;
   __syncthreads();
   if (ty == 0 && i < m) {
     for (int q = 1; q < 8; ++q) mx = max(mx, part[q][tx]);
-    ea[(long long)b * m + i] = scale_exponent(mx);
+    ea[(long long)b * m + i] = STRICT ? scale_exponent_strict(mx) : scale_exponent(mx);
   }
 }
 
@@ -382,10 +409,14 @@ __global__ void __launch_bounds__(256) slice_b_kernel(const double2* B, int ldb,
   if (j >= n) return;   // whole warps leave together; no block-wide barrier below
   const double2* col = B + (long long)b * sB + (long long)j * ldb;
   unsigned long long mx = 0;
-  for (int kk = lane; kk < k; kk += 32) mx = max(mx, max(abs_bits(col[kk].x), abs_bits(col[kk].y)));
+  constexpr bool STRICT = S == 9;
+  for (int kk = lane; kk < k; kk += 32) {
+    if (STRICT) mx = max(mx, max(abs_bits_all(col[kk].x), abs_bits_all(col[kk].y)));
+    else mx = max(mx, max(abs_bits(col[kk].x), abs_bits(col[kk].y)));
+  }
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, off));
-  const int e = scale_exponent(mx);
+  const int e = STRICT ? scale_exponent_strict(mx) : scale_exponent(mx);
   if (lane == 0) fb[(long long)b * n + j] = e;
   double2* ch = chunk[warp];
   for (int c0 = 0; c0 < half; c0 += 256) {
@@ -490,7 +521,28 @@ struct TcArgs {
   int alpha_one;           // alpha == 1
   int beta_kind;           // 0: beta == 0, 1: beta == 1, 2: general
   int* err;
+  // what was sliced, for the rows and columns of exponent EXP_DIRECT (nine slices only)
+  const double2* A0; int lda0; long long sA0;
+  const double2* B0; int ldb0; long long sB0;
+  int k0;
 };
+
+__device__ __forceinline__ bool not_finite(double x) {
+  return ((unsigned)((unsigned long long)__double_as_longlong(x) >> 52) & 0x7FFu) == 0x7FFu;
+}
+
+// the real (part 0) or imaginary part of sum_k A(row, k) B(k, col) as zgemm_f64 forms it
+__device__ __noinline__ double direct_dot(const TcArgs& a, int b, int row, int col, int part) {
+  const double2* A = a.A0 + (long long)b * a.sA0 + row;
+  const double2* B = a.B0 + (long long)b * a.sB0 + (long long)col * a.ldb0;
+  double s = 0.0;
+  for (int k = 0; k < a.k0; ++k) {
+    const double2 x = A[(long long)k * a.lda0], y = B[k];
+    s = part ? fma(x.x, y.y, s) : fma(x.x, y.x, s);
+    s = part ? fma(x.y, y.x, s) : fma(-x.y, y.y, s);
+  }
+  return s;
+}
 
 // Stores one chunk of CW tile columns.  Each lane holds, for its real output row, the exact
 // integer sums of the real part (even row, part 0) or the imaginary part (odd row, part 1)
@@ -501,10 +553,16 @@ struct TcArgs {
 template <int S, int DH, int CW>
 __device__ __forceinline__ void store_chunk(const long long (&hi)[CW], const long long (&lo)[CW], const int* cexp,
                                             int e_row, int part, int row, int col0, bool valid, const TcArgs& a,
-                                            double2* Cb) {
+                                            double2* Cb, int b) {
   double v[CW];
 #pragma unroll
   for (int c = 0; c < CW; ++c) v[c] = recombine<S, DH>(hi[c], lo[c], e_row + cexp[c] - 12 - 7 * (S - 1));
+  if constexpr (S == 9) {
+#pragma unroll
+    for (int c = 0; c < CW; ++c)
+      if ((e_row == EXP_DIRECT || cexp[c] == EXP_DIRECT) && valid && col0 + c < a.n)
+        v[c] = direct_dot(a, b, row, col0 + c, part);
+  }
   double recv[CW / 2];   // the partner's half of the columns this lane stores
 #pragma unroll
   for (int h = 0; h < CW / 2; ++h) recv[h] = __shfl_xor_sync(0xffffffffu, part ? v[2 * h] : v[2 * h + 1], 1);
@@ -524,7 +582,10 @@ __device__ __forceinline__ void store_chunk(const long long (&hi)[CW], const lon
     const double mine = part ? v[2 * h + 1] : v[2 * h];
     double2 out = part ? make_double2(recv[h], mine) : make_double2(mine, recv[h]);
     if (!a.alpha_one) out = cmul(a.alpha, out);
-    if (a.beta_kind == 1) out = cadd(out, cin[h]);
+    else if (S == 9 && (not_finite(out.x) || not_finite(out.y))) out = cmul(a.alpha, out);   // as zgemm_f64
+    if (S == 9 && a.beta_kind == 1 && (not_finite(cin[h].x) || not_finite(cin[h].y)))
+      out = cadd(out, cmul(a.beta, cin[h]));
+    else if (a.beta_kind == 1) out = cadd(out, cin[h]);
     else if (a.beta_kind == 2) out = cadd(out, cmul(a.beta, cin[h]));
     Cb[(long long)col * a.ldc + row] = out;
   }
@@ -679,7 +740,7 @@ __global__ void __launch_bounds__(TC_THREADS, MINB)
           }
         }
       }
-      store_chunk<S, DH, CW>(hi, lo, col_exp + c0, e_row, part, row, tn * NT + c0, row < a.m && !aborted, a, Cb);
+      store_chunk<S, DH, CW>(hi, lo, col_exp + c0, e_row, part, row, tn * NT + c0, row < a.m && !aborted, a, Cb, b);
     }
   }
   tc_fence_before();
@@ -901,7 +962,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
             else lo[i] += q * (1LL << (7 * (S - 1 - d)));
           }
         }
-        store_chunk<S, DH, CW>(hi, lo, cexp + c0, e_row, part, row, tn * NT + c0, row < a.m, a, Cb);
+        store_chunk<S, DH, CW>(hi, lo, cexp + c0, e_row, part, row, tn * NT + c0, row < a.m, a, Cb, b);
       }
       tc_fence_before();
       mbar_arrive(&tempty[buf]);
@@ -1008,7 +1069,7 @@ int slice_a_t(const double2* A, int lda, long long sA, int m, int k, int batch, 
   cudaEvent_t ev;
   timed_begin(st, TK_SLICE, 0.0, &ev);
   dim3 g1((m + 31) / 32, batch);
-  row_exp_kernel<<<g1, dim3(32, 8), 0, st>>>(A, lda, sA, m, k, out.exps);
+  row_exp_kernel<S == 9><<<g1, dim3(32, 8), 0, st>>>(A, lda, sA, m, k, out.exps);
   NEGF_CUDA_TRY(cudaGetLastError());
   dim3 g2((m + 31) / 32, (out.k + 63) / 64, batch);
   slice_a_kernel<S><<<g2, 256, 0, st>>>(A, lda, sA, m, k, out.exps, out.data, out.k);
@@ -1047,6 +1108,8 @@ int slice_a(const double2* A, int lda, long long sA, int m, int k, int batch, in
   if (sliced_bytes_a(m, padded_k(k), slices, batch) > out.data_bytes || (size_t)m * batch > out.exps_count)
     return NEGF_EINVAL;
   out.rows = 2 * m; out.k = padded_k(k); out.slices = slices; out.batch = batch;
+  out.exps_used = (size_t)m * batch;
+  out.src = A; out.ld = lda; out.sSrc = sA; out.k_src = k;
   switch (slices) {
     case 2: return slice_a_t<2>(A, lda, sA, m, k, batch, out, st);
     case 3: return slice_a_t<3>(A, lda, sA, m, k, batch, out, st);
@@ -1054,6 +1117,7 @@ int slice_a(const double2* A, int lda, long long sA, int m, int k, int batch, in
     case 5: return slice_a_t<5>(A, lda, sA, m, k, batch, out, st);
     case 6: return slice_a_t<6>(A, lda, sA, m, k, batch, out, st);
     case 7: return slice_a_t<7>(A, lda, sA, m, k, batch, out, st);
+    case 9: return slice_a_t<9>(A, lda, sA, m, k, batch, out, st);
     case 8: return slice_a_t<8>(A, lda, sA, m, k, batch, out, st);
   }
   return NEGF_EINVAL;
@@ -1064,6 +1128,8 @@ int slice_b(const double2* B, int ldb, long long sB, int k, int n, int batch, in
   if (sliced_bytes_b(n, padded_k(k), slices, batch) > out.data_bytes || (size_t)n * batch > out.exps_count)
     return NEGF_EINVAL;
   out.rows = n; out.k = padded_k(k); out.slices = slices; out.batch = batch;
+  out.exps_used = (size_t)n * batch;
+  out.src = B; out.ld = ldb; out.sSrc = sB; out.k_src = k;
   switch (slices) {
     case 2: return slice_b_t<2>(B, ldb, sB, k, n, batch, out, st);
     case 3: return slice_b_t<3>(B, ldb, sB, k, n, batch, out, st);
@@ -1071,6 +1137,7 @@ int slice_b(const double2* B, int ldb, long long sB, int k, int n, int batch, in
     case 5: return slice_b_t<5>(B, ldb, sB, k, n, batch, out, st);
     case 6: return slice_b_t<6>(B, ldb, sB, k, n, batch, out, st);
     case 7: return slice_b_t<7>(B, ldb, sB, k, n, batch, out, st);
+    case 9: return slice_b_t<9>(B, ldb, sB, k, n, batch, out, st);
     case 8: return slice_b_t<8>(B, ldb, sB, k, n, batch, out, st);
   }
   return NEGF_EINVAL;
@@ -1175,6 +1242,9 @@ int zgemm_tc(const SlicedOperand& A, const SlicedOperand& B, double2 alpha, doub
   args.planesA = A.slices; args.planesB = B.slices;
   args.ea = A.exps; args.fb = B.exps;
   args.C = C; args.ldc = ldc; args.sC = sC;
+  args.A0 = A.src; args.lda0 = A.ld; args.sA0 = A.sSrc;
+  args.B0 = B.src; args.ldb0 = B.ld; args.sB0 = B.sSrc;
+  args.k0 = A.k_src;
   args.alpha = alpha; args.beta = beta; args.err = err;
   args.alpha_one = (alpha.x == 1.0 && alpha.y == 0.0) ? 1 : 0;
   args.beta_kind = (beta.x == 0.0 && beta.y == 0.0) ? 0 : (beta.x == 1.0 && beta.y == 0.0) ? 1 : 2;
@@ -1201,6 +1271,7 @@ int launch_variant(int v, int S, const SlicedOperand& A, const SlicedOperand& B,
       case 6: return launch_mma<6, 32, 1, 2>(A, B, args, st);
       case 7: return launch_mma<7, 32, 1, 2>(A, B, args, st);
       case 8: return launch_mma<8, 32, 1, 2>(A, B, args, st);
+      case 9: return launch_mma<9, 16, 1, 2>(A, B, args, st);
     }
     return NEGF_EINVAL;
   }
@@ -1213,6 +1284,7 @@ int launch_variant(int v, int S, const SlicedOperand& A, const SlicedOperand& B,
       case 6: return launch_persistent<6, 32>(A, B, args, st);
       case 7: return launch_persistent<7, 32>(A, B, args, st);
       case 8: return launch_persistent<8, 32>(A, B, args, st);
+      case 9: return launch_persistent<9, 16>(A, B, args, st);
     }
     return NEGF_EINVAL;
   }
@@ -1224,6 +1296,7 @@ int launch_variant(int v, int S, const SlicedOperand& A, const SlicedOperand& B,
     case 6: return v ? launch_mma<6, 80, 1>(A, B, args, st) : launch_mma<6, 64, 1>(A, B, args, st);
     case 7: return v ? launch_mma<7, 48, 1>(A, B, args, st) : launch_mma<7, 64, 1>(A, B, args, st);
     case 8: return v ? launch_mma<8, 48, 1>(A, B, args, st) : launch_mma<8, 64, 1>(A, B, args, st);
+    case 9: return v ? launch_mma<9, 32, 1>(A, B, args, st) : launch_mma<9, 48, 1>(A, B, args, st);
   }
   return NEGF_EINVAL;
 }

@@ -18,8 +18,15 @@ struct SlicedOperand {
   int rows = 0, k = 0, slices = 0, batch = 0;
   size_t data_bytes = 0;     // capacity of data; slice_a/slice_b refuse anything larger
   size_t exps_count = 0;     // capacity of exps (ints)
+  size_t exps_used = 0;      // exponents written: batch * M or batch * N
+  // what was sliced (column-major, leading dimension ld, batch stride sSrc, inner dimension
+  // k_src): nine-slice products take the rows and columns that integers cannot hold from it
+  const double2* src = nullptr;
+  int ld = 0, k_src = 0;
+  long long sSrc = 0;
 };
 
+// slice counts a caller may ask for (3..8); the engine's FP64 form also uses nine
 bool tc_supported_slices(int s);
 // K padded to a multiple of 4 (TMA rows must be a multiple of 16 bytes)
 int padded_k(int k);

@@ -37,3 +37,36 @@ def test_mixed_form_at_the_panel_kernels_sizes(need_gpu, npy, npz):
     t, want, rho, rho_want = _one_energy(3, npy, npz, "mixed")
     assert abs(t - want) <= 1e-6 * max(abs(want), 1e-3)
     assert np.abs(rho - rho_want).max() <= 1e-6 * np.abs(rho_want).max()
+
+
+# The FP64 form takes its products and inverses on the tensor cores from M = 32 (28 and 32)
+# with one set of accumulators up to K = 400 and two up to 800, and on the FP64 pipe beyond.
+# Tolerance: the FP64 form's 1e-9.
+@pytest.mark.parametrize("npy,npz", [(1, 7), (2, 4), (3, 3), (1, 33), (10, 10), (1, 101), (10, 20), (3, 67)])
+def test_fp64_form_at_its_path_switches(need_gpu, npy, npz):
+    t, want, rho, rho_want = _one_energy(3, npy, npz, "fp64")
+    assert abs(t - want) <= 1e-9 * max(abs(want), 1e-3)
+    assert np.abs(rho - rho_want).max() <= 1e-9 * np.abs(rho_want).max()
+
+
+# What a double holds and the slices' common scale of a row does not: a wall of 1e8 eV on a
+# site (the FP64 form's 1e-9), and a NaN or an infinity in one sample, which stays in that
+# sample and leaves its neighbour's bits alone.
+@pytest.mark.parametrize("value", [1e8, np.nan, np.inf])
+def test_fp64_form_with_extreme_entries(need_gpu, value):
+    npx, npy, npz = 4, 3, 3
+    htotd, hopx = hamiltonian.ti_wire(npx, npy, npz, W=0.1, seed=3, flux=0.4, zeeman=0.01)
+    bad = htotd.copy()
+    bad[1, 5, 5] = value
+    with Solver(npx, npy, npz, eta=1e-3, sr_tol=1e-10, n_hamiltonians=2, max_batch=2) as s:
+        s.set_hamiltonian(htotd, hopx, slot=0)
+        s.set_hamiltonian(bad, hopx, slot=1)
+        alone = s.solve_batch([0.11], 0.7, 0.2, 1e-3)
+        both = s.solve_batch([0.11, 0.11], 0.7, 0.2, 1e-3, slots=[0, 1])
+    assert both["T12"][0] == alone["T12"][0] and both["Modec1"][0] == alone["Modec1"][0]
+    if np.isfinite(value):
+        opt = O.SolveOptions(eta=1e-3, sr_tol=1e-10, kT=0.025)
+        want = O.energy_sweep(bad, hopx, 0.11, (0.005, -0.005), 1e-3, npy, npz, opt)
+        assert abs(both["T12"][1] - want["T12"]) <= 1e-9 * abs(want["T12"])
+    else:
+        assert np.isnan(both["T12"][1])
