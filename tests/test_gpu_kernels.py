@@ -2,7 +2,7 @@
 import numpy as np
 import pytest
 
-from nonequilibriumgreensfunction_gb300 import Solver, hamiltonian
+from nonequilibriumgreensfunction_gb300 import Solver, hamiltonian, scf
 from oracle import negf_oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -70,3 +70,15 @@ def test_fp64_form_with_extreme_entries(need_gpu, value):
         assert abs(both["T12"][1] - want["T12"]) <= 1e-9 * abs(want["T12"])
     else:
         assert np.isnan(both["T12"][1])
+
+
+# Up to 40 Poisson grids take a cluster of CTAs each, more take one CTA: the same bits and the
+# same number of steps, below, at and above one element per thread (1024 sites).
+@pytest.mark.parametrize("shape", [(5, 1, 1), (9, 3, 4), (16, 8, 8), (41, 5, 5), (30, 9, 8)])
+def test_poisson_cluster_gives_the_same_bits(need_gpu, shape):
+    rho = 1e-3 * np.random.default_rng(1).standard_normal(shape + (41,))
+    one_cta, steps = scf.poisson_solve(rho, (0.02, -0.02, 0.1), 1.8)
+    cluster, few = scf.poisson_solve(rho[..., :40], (0.02, -0.02, 0.1), 1.8)
+    last, more = scf.poisson_solve(rho[..., 40:], (0.02, -0.02, 0.1), 1.8)
+    assert np.array_equal(one_cta[..., :40], cluster) and np.array_equal(one_cta[..., 40:], last)
+    assert max(few, more) == steps
