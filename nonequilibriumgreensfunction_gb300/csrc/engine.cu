@@ -217,12 +217,15 @@ int Engine::configure(const negf_params& p) {
   ns_step_[1].res = s_res_;
   tc_cap_ = std::max(B_, S_);
   tc_ = mixed_;
-  if (!mixed_ && !lean_ && M_ >= 32 && 2 * padded_k(M_) <= 1600) {
-    // The FP64 form on GB300's tensor cores: its FP64 pipe does two multiply-adds per clock and
-    // SM, the nine-slice product of 45 BF16 slice pairs about 25 times that (400^3: 0.4 ms
-    // against 10 ms for 64 products).  Below M = 32 the launches of the sliced path cost more
-    // than the arithmetic (M = 2: 46 against 28 ms an energy; M = 36: 11 against 34 ms).  Each step's residual is as fine as the step's result has to be: FP32
-    // Gauss-Jordan leaves ~1e-3, and the steps ~1e-7, ~1e-12 and the rounding of a double.
+  // The FP64 form.  Cross-sections up to SMALL_MAX_M take one kernel per phase (small_f64.cu)
+  // unless they ask for what that leaves out.  Beyond, and from M = 32 then, the tensor cores:
+  // GB300's FP64 pipe does two multiply-adds per clock and SM, the nine-slice product of 45
+  // BF16 slice pairs some twenty times that (a sweep of M = 400: 1155 -> 116 ms); at M = 2 the
+  // launches of the sliced path cost more than they save (46 against 28 ms an energy).
+  const bool one_kernel = M_ <= SMALL_MAX_M && !currents_ && !keep_columns_ && p.contact_type != NEGF_CONTACT_SC;
+  if (!mixed_ && !lean_ && !one_kernel && M_ >= 32 && 2 * padded_k(M_) <= 1600) {
+    // Each step's residual is as fine as the step's result has to be: FP32 Gauss-Jordan leaves
+    // ~1e-3, and the steps ~1e-7, ~1e-12 and the rounding of a double.
     tc_ = true;
     s_rgf_ = s_sr_ = s_res_ = 9;
     ns_step_[0] = {5, 3};
@@ -313,7 +316,7 @@ int Engine::alloc() {
   for (double2** b : srb) NEGF_TRY(dalloc(b, (size_t)(S_ * MM_), bytes_, dry_, pool_, own_st_));
   NEGF_TRY(dalloc(&dSrCmax_, (size_t)2 * S_, bytes_, dry_, pool_, own_st_));
   NEGF_TRY(dalloc(&dSrDos_, (size_t)2 * S_, bytes_, dry_, pool_, own_st_));
-  NEGF_TRY(dalloc(&dSrActive_, (size_t)2 * S_, bytes_, dry_, pool_, own_st_));
+  NEGF_TRY(dalloc(&dSrActive_, (size_t)8 * S_, bytes_, dry_, pool_, own_st_));
   NEGF_TRY(dalloc(&dSrE_, (size_t)S_, bytes_, dry_, pool_, own_st_));
   NEGF_TRY(dalloc(&dSrHend_, (size_t)S_, bytes_, dry_, pool_, own_st_));
   NEGF_TRY(dalloc(&dSrStatus_, (size_t)S_, bytes_, dry_, pool_, own_st_));
@@ -766,6 +769,7 @@ int Engine::solve_sr_impl(const std::vector<SrJob>& jobs, std::vector<int>& stat
   const int S = (int)jobs.size();
   if (S == 0) return NEGF_OK;
   if (S > S_) return NEGF_EINVAL;
+  if (small_() && hop_bd_) return solve_sr_small(jobs, status, iters);
   const long long N = p_.npx;
   const double2 one = make_double2(1, 0), zero = make_double2(0, 0), mone = make_double2(-1, 0);
   std::vector<double> e(S);
@@ -936,6 +940,45 @@ int Engine::solve_sr_impl(const std::vector<SrJob>& jobs, std::vector<int>& stat
   return NEGF_OK;
 }
 
+// The same problems in one kernel (small_f64.cu)
+int Engine::solve_sr_small(const std::vector<SrJob>& jobs, std::vector<int>& status, std::vector<int>& iters) {
+  const int S = (int)jobs.size();
+  std::vector<double> e(S);
+  std::vector<const double2*> hend(S);
+  // dSrActive_: want, active, iters (two per problem each), then status and done
+  std::vector<int> ints((size_t)8 * S, 0);
+  for (int s = 0; s < S; ++s) {
+    e[s] = jobs[s].energy;
+    const int slot = jobs[s].slot;
+    if (slot < 0 || !slot_set_[slot]) return NEGF_ENOHAM;
+    hend[s] = dH_ + ((long long)slot * p_.npx + (jobs[s].use_last ? p_.npx - 1 : 0)) * MM_;
+    ints[s] = ints[2 * S + s] = jobs[s].want_l;
+    ints[S + s] = ints[3 * S + s] = jobs[s].want_r;
+  }
+  NEGF_CUDA_TRY(cudaMemcpyAsync(dSrE_, e.data(), sizeof(double) * S, cudaMemcpyHostToDevice, st_));
+  NEGF_CUDA_TRY(cudaMemcpyAsync(dSrHend_, hend.data(), sizeof(void*) * S, cudaMemcpyHostToDevice, st_));
+  NEGF_CUDA_TRY(cudaMemcpyAsync(dSrActive_, ints.data(), sizeof(int) * ints.size(), cudaMemcpyHostToDevice, st_));
+  SmallSr a{};
+  a.n = M_; a.count = S; a.hop = hop();
+  a.energies = dSrE_; a.hend = dSrHend_;
+  a.eta = p_.eta; a.tol = p_.sr_tol; a.max_iter = p_.sr_max_iter;
+  a.want = dSrActive_; a.active = dSrActive_ + 2 * S; a.iters = dSrActive_ + 4 * S;
+  a.status = dSrActive_ + 6 * S; a.done = dSrActive_ + 7 * S;
+  a.state = dSr_;
+  a.sigL = dSrSigL_; a.sigR = dSrSigR_; a.gamL = dSrGamL_; a.gamR = dSrGamR_;
+  a.dos = dSrDos_;
+  do {
+    NEGF_TRY(small_sr(a, st_));
+    a.first_step += small_sr_steps();
+    NEGF_CUDA_TRY(cudaMemcpyAsync(ints.data() + 4 * S, dSrActive_ + 4 * S, sizeof(int) * 4 * S, cudaMemcpyDeviceToHost,
+                                  st_));
+    NEGF_CUDA_TRY(cudaStreamSynchronize(st_));
+  } while (std::any_of(ints.begin() + 7 * S, ints.end(), [](int d) { return d == 0; }));
+  iters.assign(ints.begin() + 4 * S, ints.begin() + 6 * S);
+  status.assign(ints.begin() + 6 * S, ints.begin() + 7 * S);
+  return NEGF_OK;
+}
+
 // Contacts with a closed-form self-energy (Source/Contact_Self_Energy.F90:19-67): the
 // per-energy scalars are formed here, the blocks on the device; Gamma and the contact DOS
 // follow from Sigma as for the decimated leads (:94-101).
@@ -1014,6 +1057,14 @@ int Engine::solve_rgf_impl(const std::vector<Item>& items, bool keep_columns) {
   const double2 one = make_double2(1, 0), zero = make_double2(0, 0);
   NEGF_CUDA_TRY(cudaMemcpyAsync(dItems_, items.data(), sizeof(Item) * B, cudaMemcpyHostToDevice, st_));
   NEGF_CUDA_TRY(cudaMemsetAsync(dStatus_, 0, sizeof(int) * B, st_));
+  if (small_() && hop_bd_ && !currents_ && !sc_() && !keep_columns) {
+    SmallRgf a{};
+    a.n = M_; a.npx = N; a.eta = p_.eta; a.hop = hop();
+    a.items = dItems_; a.Hall = dH_;
+    a.sigL = dSrSigL_; a.sigR = dSrSigR_; a.gamL = dSrGamL_; a.gamR = dSrGamR_;
+    a.G = dG_; a.P1 = dP1_; a.P2 = dP2_; a.traces = dTr_; a.status = dStatus_;
+    return small_rgf(a, B, st_);
+  }
   const int istride = (int)(sizeof(Item) / sizeof(int));
   const int* idx_l = reinterpret_cast<const int*>(reinterpret_cast<const char*>(dItems_) + offsetof(Item, sr_l));
   const int* idx_r = reinterpret_cast<const int*>(reinterpret_cast<const char*>(dItems_) + offsetof(Item, sr_r));

@@ -189,6 +189,9 @@ class Engine {
   int invert_impl(double2* A, long long sA, int batch, int* status_dev);
   int invert_refined(double2* A, long long sA, int batch, int* status_dev);
   int solve_sr_impl(const std::vector<SrJob>& jobs, std::vector<int>& status, std::vector<int>& iters);
+  // FP64 solves of small cross-sections take one kernel per phase (small_f64.cu)
+  bool small_() const { return !mixed_ && !tc_ && M_ <= SMALL_MAX_M; }
+  int solve_sr_small(const std::vector<SrJob>& jobs, std::vector<int>& status, std::vector<int>& iters);
   int solve_rgf_impl(const std::vector<Item>& items, bool keep_columns);
   int densities_impl(const std::vector<Item>& items, std::vector<double>& edens, std::vector<double>& hdens);
   HopBD hop() const {

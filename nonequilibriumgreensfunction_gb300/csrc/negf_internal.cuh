@@ -275,6 +275,42 @@ int sr_form_final(const HopBD& h, int n, int nprob, int lead, const double2* alp
 int sr_sigma(const HopBD& h, int n, int nprob, int lead, const double2* g, long long sg, double2* sig,
              long long sSig, double2* gam, long long sGam, double* dos, cudaStream_t st);
 
+// ----------------------------------------------------------------------------------
+// whole phases of small cross-sections in one kernel (small_f64.cu)
+// ----------------------------------------------------------------------------------
+constexpr int SMALL_MAX_M = 38;   // nine blocks of the decimation in 227 KB of shared memory
+struct SmallSr {                  // `count` decimation problems; arrays [2 count]: left leads, then right
+  int n, count;
+  HopBD hop;
+  const double* energies;
+  const double2* const* hend;
+  double eta, tol;
+  int first_step, max_iter;       // steps taken by earlier launches; the cap of all
+  const int* want;                // leads whose self-energy is asked for
+  int* active;                    // leads not yet converged (in and out)
+  int* iters;
+  int* status;                    // [count]
+  int* done;                      // [count] self-energies written
+  double2* state;                 // [count][6][n n] between launches
+  double2 *sigL, *sigR, *gamL, *gamR;
+  double* dos;
+};
+int small_sr(const SmallSr& a, cudaStream_t st);
+int small_sr_steps();   // decimation steps of one launch at most
+struct SmallRgf {
+  int n, npx;
+  double eta;
+  HopBD hop;
+  const Item* items;
+  const double2* Hall;
+  const double2 *sigL, *sigR, *gamL, *gamR;   // by decimation problem
+  double2* G;                                 // [item][npx][n n] block store
+  double2 *P1, *P2;                           // [item][npx][n][norb]
+  double* traces;                             // [item][4]
+  int* status;                                // [item]
+};
+int small_rgf(const SmallRgf& a, int count, cudaStream_t st);
+
 // density / spin from the site blocks of both leads.  P1, P2: [item][x][n][norb].
 // site_out: [item][nf][npx*npy*npz], fields 0..4 = (RhoN, RhoP, SigX, SigY, SigZ) already
 // weighted by dE/(2 pi) (fields 5..7 = Jx, Jy, Jz when nf = 8, bond_currents);

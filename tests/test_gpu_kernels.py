@@ -82,3 +82,38 @@ def test_poisson_cluster_gives_the_same_bits(need_gpu, shape):
     last, more = scf.poisson_solve(rho[..., 40:], (0.02, -0.02, 0.1), 1.8)
     assert np.array_equal(one_cta[..., :40], cluster) and np.array_equal(one_cta[..., 40:], last)
     assert max(few, more) == steps
+
+
+# FP64 solves up to M = 38 run in one kernel per phase, with a cluster of 8, 4, 2 or 1 CTAs per
+# problem by their number (1, 12, 40, 80 energies): one channel of each orbital count, sizes at
+# the ends and at the cluster threshold (1, 2, 15, 16, 36, 38) and the first beyond (39).  The
+# same bits in every batch, and the oracle's values to the FP64 form's 1e-9.
+@pytest.mark.parametrize("channel,npy,npz", [(2, 1, 1), (4, 1, 1), (2, 5, 3), (0, 2, 2), (0, 3, 3), (3, 19, 1), (2, 13, 3)])
+def test_small_cross_sections_in_every_cluster(need_gpu, channel, npy, npz):
+    npx, norb, eta = 5, hamiltonian.CHANNEL_NORB[channel], 1e-3
+    model = hamiltonian.channel_model(channel, W=0.2, seed=4)
+    htotd, hopx = hamiltonian.build_from_model(npx, npy, npz, model)
+    energies = np.linspace(0.31, 0.73, 80) + (2.0 if channel == 2 else 0.0)
+    runs = []
+    for n in (80, 40, 12, 1):
+        with Solver(npx, npy, npz, norb=norb, eta=eta, sr_tol=1e-10, max_batch=n) as s:
+            s.build_hamiltonian(model)
+            rho = s.new_site_array(1)
+            runs.append((s.solve_batch(energies[:n], 0.7, 0.2, 1e-3, rho_n=rho), rho))
+    for n, (r, _) in zip((40, 12, 1), runs[1:]):
+        for k in r:
+            assert np.array_equal(r[k], runs[0][0][k][:n]), k
+    r, rho = runs[3]
+    opt = O.SolveOptions(eta=eta, sr_tol=1e-10, norb=norb)
+    cse = O.contact_self_energy(htotd, hopx, energies[0], opt)
+    inv = np.stack([(energies[0] + 1j * eta) * np.eye(h.shape[0]) - h for h in htotd])
+    inv[0] -= cse["SigmaL"]
+    inv[-1] -= cse["SigmaR"]
+    g = O.get_retarded_greens(inv, hopx)
+    gnp = O.calculate_gnp(g["GRLef"], g["GRRgt"], cse["GammaL"], cse["GammaR"], 0.7, 0.2, with_offdiag=False)
+    want = O.site_density(gnp["Gnd"], npy, npz, norb) * 1e-3 / (2 * np.pi)
+    t12 = np.real(np.trace(cse["GammaL"] @ g["GRRgt"][0] @ cse["GammaR"] @ g["GRRgt"][0].conj().T))
+    assert r["status"][0] == 0 and r["sr_iters"][0] == cse["sr_iters"].max()
+    assert abs(r["T12"][0] - t12) <= 1e-9 * max(abs(t12), 1e-3)
+    assert abs(r["DOSc1"][0] - cse["dosc"][0]) <= 1e-9 * abs(cse["dosc"][0])
+    assert np.abs(rho[..., 0] - want).max() <= 1e-9 * np.abs(want).max()
