@@ -257,11 +257,9 @@ int negf_contact_self_energy(negf_handle* h, double energy, double* SigmaL, doub
       {GammaL, e.dSrGamL_ + (long long)h->sr_l * e.MM_}, {GammaR, e.dSrGamR_ + (long long)h->sr_r * e.MM_}};
   for (const Out& o : outs)
     if (o.dst) NEGF_CUDA_TRY(cudaMemcpyAsync(o.dst, o.src, bytes, cudaMemcpyDeviceToHost, e.st_));
-  double dos[2];
-  NEGF_CUDA_TRY(cudaMemcpyAsync(&dos[0], e.dSrDos_ + h->sr_l, sizeof(double), cudaMemcpyDeviceToHost, e.st_));
-  NEGF_CUDA_TRY(cudaMemcpyAsync(&dos[1], e.dSrDos_ + S + h->sr_r, sizeof(double), cudaMemcpyDeviceToHost, e.st_));
+  NEGF_CUDA_TRY(cudaMemcpyAsync(e.hDos_, e.dSrDos_, sizeof(double) * 2 * S, cudaMemcpyDeviceToHost, e.st_));
   NEGF_CUDA_TRY(cudaStreamSynchronize(e.st_));
-  if (dosc) { dosc[0] = dos[0]; dosc[1] = dos[1]; }
+  if (dosc) { dosc[0] = e.hDos_[h->sr_l]; dosc[1] = e.hDos_[S + h->sr_r]; }
   h->sr_status = status[h->sr_l] ? status[h->sr_l] : status[h->sr_r];
   h->sr_iters = std::max(iters[h->sr_l], iters[S + h->sr_r]);
   e.cur_energy_ = energy;
@@ -278,11 +276,11 @@ int negf_get_retarded_greens(negf_handle* h) {
   items[0] = negf::Item{e.cur_energy_, 0.0, 0.0, 0.0, 0, h->sr_l, h->sr_r, 0};
   e.rgf_valid_ = e.dens_valid_ = false;
   NEGF_TRY(e.solve_rgf(items, e.keep_columns_));
-  int st = 0, tc_err = 0;
-  NEGF_CUDA_TRY(cudaMemcpyAsync(&st, e.dStatus_, sizeof(int), cudaMemcpyDeviceToHost, e.st_));
-  NEGF_TRY(e.read_tc_error(&tc_err));
+  NEGF_CUDA_TRY(cudaMemcpyAsync(e.hRst_, e.dStatus_, sizeof(int), cudaMemcpyDeviceToHost, e.st_));
+  NEGF_TRY(e.read_tc_error());
   NEGF_CUDA_TRY(cudaStreamSynchronize(e.st_));
-  if (tc_err) return NEGF_ETIMEDOUT;
+  const int st = e.hRst_[0];
+  if (*e.hErr_) return NEGF_ETIMEDOUT;
   e.cur_rgf_status_ = st;
   e.rgf_valid_ = true;
   return st;
@@ -319,10 +317,9 @@ int negf_calculate_gnp(negf_handle* h, double f1, double f2, double dE, double* 
   std::vector<double> ed, hd;
   NEGF_TRY(e.densities(items, ed, hd));
   const long long total = e.nsite_total();
-  e.last_site_.resize((size_t)e.nf_ * total);
-  NEGF_CUDA_TRY(cudaMemcpyAsync(e.last_site_.data(), e.dSite_, sizeof(double) * e.nf_ * total,
-                                cudaMemcpyDeviceToHost, e.st_));
+  NEGF_CUDA_TRY(cudaMemcpyAsync(e.hPin_, e.dSite_, sizeof(double) * e.nf_ * total, cudaMemcpyDeviceToHost, e.st_));
   NEGF_CUDA_TRY(cudaStreamSynchronize(e.st_));
+  e.last_site_.assign(e.hPin_, e.hPin_ + (size_t)e.nf_ * total);
   for (long long i = 0; i < total; ++i) {
     if (RhoN) RhoN[i] += e.last_site_[i];
     if (RhoP) RhoP[i] += e.last_site_[total + i];
@@ -340,11 +337,11 @@ int negf_calculate_observables(negf_handle* h, double dE, double f1, double f2, 
   Engine& e = h->eng;
   if (!e.dens_valid_) return NEGF_ESTATE;
   NEGF_CUDA_TRY(cudaSetDevice(e.p_.device));
-  double tr[4], trj = 0.0;
-  NEGF_CUDA_TRY(cudaMemcpyAsync(tr, e.dTr_, sizeof(tr), cudaMemcpyDeviceToHost, e.st_));
-  if (e.sc_()) NEGF_CUDA_TRY(cudaMemcpyAsync(&trj, e.dTrJ_, sizeof(double), cudaMemcpyDeviceToHost, e.st_));
+  const double* tr = e.hTr_;
+  NEGF_CUDA_TRY(cudaMemcpyAsync(e.hTr_, e.dTr_, sizeof(double) * 4, cudaMemcpyDeviceToHost, e.st_));
+  if (e.sc_()) NEGF_CUDA_TRY(cudaMemcpyAsync(e.hTrJ_, e.dTrJ_, sizeof(double), cudaMemcpyDeviceToHost, e.st_));
   NEGF_CUDA_TRY(cudaStreamSynchronize(e.st_));
-  const double t12 = e.sc_() ? trj : tr[1];
+  const double t12 = e.sc_() ? e.hTrJ_[0] : tr[1];
   if (T12) *T12 = t12;
   if (EDensity) *EDensity = e.last_edens_;
   if (HDensity) *HDensity = e.last_hdens_;

@@ -157,6 +157,7 @@ Engine::~Engine() {
   free_tc();
   cudaStreamSynchronize(own_st_);   // the frees have run: the blocks are back in the pool
   pinned_give(hPin_, hPinBytes_);
+  pinned_give(static_cast<double*>(hSmall_), hSmallBytes_);
   cudaStreamDestroy(own_st_);
 }
 
@@ -343,6 +344,23 @@ int Engine::alloc() {
                    {(long long)B_ * sums_blocks_ * 2, (long long)B_ * 4, 4LL * S_,
                     (long long)p_.n_hamiltonians * nf_ * total, (long long)nf_ * total, 64});
   NEGF_TRY(pinned_take(hPinBytes_, &hPin_, &hPinBytes_));
+  {
+    const size_t cap = (size_t)std::max(B_, S_);
+    double* p = nullptr;
+    NEGF_TRY(pinned_take(sizeof(double) * (2 * (size_t)S_ + 5 * (size_t)B_ + 2 * cap) +
+                             sizeof(int) * (cap + 4 * (size_t)S_ + (size_t)B_ + 2), &p, &hSmallBytes_));
+    hSmall_ = p;
+    hDos_ = p;
+    hTr_ = hDos_ + 2 * (size_t)S_;
+    hTrJ_ = hTr_ + 4 * (size_t)B_;
+    hR0_ = reinterpret_cast<unsigned long long*>(hTrJ_ + B_);
+    hRk_ = hR0_ + cap;
+    hInfo_ = reinterpret_cast<int*>(hRk_ + cap);
+    hSr_ = hInfo_ + cap;
+    hRst_ = hSr_ + 4 * (size_t)S_;
+    hErr_ = hRst_ + B_;
+    *hErr_ = 0;
+  }
   // the allocations are ordered on the engine's stream; after this they are usable from
   // any stream (the caller's, through negf_set_stream) and by the synchronous copies below
   NEGF_CUDA_TRY(cudaStreamSynchronize(own_st_));
@@ -519,10 +537,10 @@ SlicedOperand Engine::view(const SlicedOperand& o, int first, int count) {
 }
 
 // The error flag of the tensor-core products so far (a bounded wait that ran out), read and
-// cleared in stream order: *err is valid after the caller's next synchronisation
-int Engine::read_tc_error(int* err) {
+// cleared in stream order: *hErr_ is valid after the caller's next synchronisation
+int Engine::read_tc_error() {
   if (!tc_) return NEGF_OK;
-  NEGF_CUDA_TRY(cudaMemcpyAsync(err, dTcErr_, sizeof(int), cudaMemcpyDeviceToHost, st_));
+  NEGF_CUDA_TRY(cudaMemcpyAsync(hErr_, dTcErr_, sizeof(int), cudaMemcpyDeviceToHost, st_));
   NEGF_CUDA_TRY(cudaMemsetAsync(dTcErr_, 0, sizeof(int), st_));
   return NEGF_OK;
 }
@@ -604,11 +622,11 @@ int Engine::invert_refined(double2* A, long long sA, int batch, int* status_dev)
   NEGF_TRY(split_copy(M_, batch, A, sA, dWinv_, MM_, dW32_, MM_, st_));
   NEGF_TRY(invert_f32(batch));
   NEGF_TRY(to_f64(M_, batch, dW32_, MM_, A, sA, st_));
-  std::vector<int> info32(batch);
-  NEGF_CUDA_TRY(cudaMemcpyAsync(info32.data(), inv_.info, sizeof(int) * batch, cudaMemcpyDeviceToHost, st_));
+  const int* info32 = hInfo_;
+  NEGF_CUDA_TRY(cudaMemcpyAsync(hInfo_, inv_.info, sizeof(int) * batch, cudaMemcpyDeviceToHost, st_));
   NEGF_CUDA_TRY(cudaMemsetAsync(dRnorm_, 0, sizeof(unsigned long long) * batch, st_));
   NEGF_TRY(slice_a(dWinv_, M_, MM_, M_, M_, batch, s_res_, sw_, st_));
-  std::vector<unsigned long long> r0(batch), rk(batch);
+  const unsigned long long *r0 = hR0_, *rk = hRk_;
   // ns_steps_ steps for the whole batch
   for (int step = 0; step < ns_steps_; ++step) {
     if (step > 0) NEGF_CUDA_TRY(cudaMemsetAsync(dRnorm_, 0, sizeof(unsigned long long) * batch, st_));
@@ -619,9 +637,9 @@ int Engine::invert_refined(double2* A, long long sA, int batch, int* status_dev)
     NEGF_TRY(zgemm_tc(sw_, sb_, one, zero, dT_, M_, MM_, dTcErr_, st_, sr));    // T = W X
     NEGF_TRY(ns_residual(M_, batch, dT_, MM_, dRnorm_, st_));                     // R = I - T
     if (step == 0)
-      NEGF_CUDA_TRY(cudaMemcpyAsync(r0.data(), dRnorm_, sizeof(unsigned long long) * batch, cudaMemcpyDeviceToHost, st_));
+      NEGF_CUDA_TRY(cudaMemcpyAsync(hR0_, dRnorm_, sizeof(unsigned long long) * batch, cudaMemcpyDeviceToHost, st_));
     if (step == ns_steps_ - 1)
-      NEGF_CUDA_TRY(cudaMemcpyAsync(rk.data(), dRnorm_, sizeof(unsigned long long) * batch, cudaMemcpyDeviceToHost, st_));
+      NEGF_CUDA_TRY(cudaMemcpyAsync(hRk_, dRnorm_, sizeof(unsigned long long) * batch, cudaMemcpyDeviceToHost, st_));
     NEGF_TRY(slice_a(A, M_, sA, M_, M_, batch, su, sa_, st_));
     NEGF_TRY(slice_b(dT_, M_, MM_, M_, M_, batch, su, sb_, st_));
     // X += X R; dT_ (R, already sliced) lends itself as the autotuner's scratch output
@@ -652,7 +670,7 @@ int Engine::invert_refined(double2* A, long long sA, int batch, int* status_dev)
     NEGF_TRY(slice_b(dNsX_, M_, MM_, M_, M_, na, s_res_, sb_, st_));
     NEGF_TRY(zgemm_tc(sa_, sb_, one, zero, dT_, M_, MM_, dTcErr_, st_));            // T = W X
     NEGF_TRY(ns_residual(M_, na, dT_, MM_, dRnorm_, st_));                           // R = I - T
-    NEGF_CUDA_TRY(cudaMemcpyAsync(rk.data(), dRnorm_, sizeof(unsigned long long) * na, cudaMemcpyDeviceToHost, st_));
+    NEGF_CUDA_TRY(cudaMemcpyAsync(hRk_, dRnorm_, sizeof(unsigned long long) * na, cudaMemcpyDeviceToHost, st_));
     NEGF_TRY(slice_a(dNsX_, M_, MM_, M_, M_, na, s_upd_, sa_, st_));
     NEGF_TRY(slice_b(dT_, M_, MM_, M_, M_, na, s_upd_, sb_, st_));
     NEGF_TRY(zgemm_tc(sa_, sb_, one, one, dNsX_, M_, MM_, dTcErr_, st_, 0, dT_));  // X += X R
@@ -929,12 +947,11 @@ int Engine::solve_sr_impl(const std::vector<SrJob>& jobs, std::vector<int>& stat
       NEGF_TRY(sr_sigma(HopBD{}, M_, n, -1, nullptr, 0, sig, sM, gam, sM, dSrDos_ + lead * S + a, st_));
     }
   }
-  std::vector<int> st(S);
-  int tc_err = 0;
-  NEGF_CUDA_TRY(cudaMemcpyAsync(st.data(), dSrStatus_, sizeof(int) * S, cudaMemcpyDeviceToHost, st_));
-  NEGF_TRY(read_tc_error(&tc_err));
+  const int* st = hSr_;
+  NEGF_CUDA_TRY(cudaMemcpyAsync(hSr_, dSrStatus_, sizeof(int) * S, cudaMemcpyDeviceToHost, st_));
+  NEGF_TRY(read_tc_error());
   NEGF_CUDA_TRY(cudaStreamSynchronize(st_));
-  if (tc_err) return NEGF_ETIMEDOUT;
+  if (*hErr_) return NEGF_ETIMEDOUT;
   for (int s = 0; s < S; ++s)
     if (status[s] == 0 && st[s] != 0) status[s] = st[s];
   return NEGF_OK;
@@ -970,12 +987,11 @@ int Engine::solve_sr_small(const std::vector<SrJob>& jobs, std::vector<int>& sta
   do {
     NEGF_TRY(small_sr(a, st_));
     a.first_step += small_sr_steps();
-    NEGF_CUDA_TRY(cudaMemcpyAsync(ints.data() + 4 * S, dSrActive_ + 4 * S, sizeof(int) * 4 * S, cudaMemcpyDeviceToHost,
-                                  st_));
+    NEGF_CUDA_TRY(cudaMemcpyAsync(hSr_, dSrActive_ + 4 * S, sizeof(int) * 4 * S, cudaMemcpyDeviceToHost, st_));
     NEGF_CUDA_TRY(cudaStreamSynchronize(st_));
-  } while (std::any_of(ints.begin() + 7 * S, ints.end(), [](int d) { return d == 0; }));
-  iters.assign(ints.begin() + 4 * S, ints.begin() + 6 * S);
-  status.assign(ints.begin() + 6 * S, ints.begin() + 7 * S);
+  } while (std::any_of(hSr_ + 3 * S, hSr_ + 4 * S, [](int d) { return d == 0; }));
+  iters.assign(hSr_, hSr_ + 2 * S);
+  status.assign(hSr_ + 2 * S, hSr_ + 3 * S);
   return NEGF_OK;
 }
 
@@ -1333,9 +1349,8 @@ int Engine::batch_solve(const negf_request* req, int n, negf_result* res, double
     std::vector<int> sr_status, sr_iters;
     NEGF_TRY(solve_sr(jobs, sr_status, sr_iters));
     const int S = (int)jobs.size();
-    std::vector<double> dos(2 * S);
-    NEGF_CUDA_TRY(cudaMemcpyAsync(dos.data(), dSrDos_, sizeof(double) * S, cudaMemcpyDeviceToHost, st_));
-    NEGF_CUDA_TRY(cudaMemcpyAsync(dos.data() + S, dSrDos_ + S, sizeof(double) * S, cudaMemcpyDeviceToHost, st_));
+    const double* dos = hDos_;
+    NEGF_CUDA_TRY(cudaMemcpyAsync(hDos_, dSrDos_, sizeof(double) * 2 * S, cudaMemcpyDeviceToHost, st_));
     NEGF_TRY(solve_rgf(items, false));
     std::vector<double> ed, hd;
     NEGF_TRY(densities(items, ed, hd));
@@ -1347,15 +1362,14 @@ int Engine::batch_solve(const negf_request* req, int n, negf_result* res, double
     if (site_items)
       NEGF_CUDA_TRY(cudaMemcpyAsync(site_items + (size_t)c0 * nf_ * total, dSite_,
                                     sizeof(double) * nf_ * total * nb, cudaMemcpyDeviceToHost, st_));
-    std::vector<double> tr(4 * (size_t)nb), trj(sc_() ? nb : 0);
-    std::vector<int> rst(nb);
-    NEGF_CUDA_TRY(cudaMemcpyAsync(tr.data(), dTr_, sizeof(double) * 4 * nb, cudaMemcpyDeviceToHost, st_));
-    if (sc_()) NEGF_CUDA_TRY(cudaMemcpyAsync(trj.data(), dTrJ_, sizeof(double) * nb, cudaMemcpyDeviceToHost, st_));
-    NEGF_CUDA_TRY(cudaMemcpyAsync(rst.data(), dStatus_, sizeof(int) * nb, cudaMemcpyDeviceToHost, st_));
-    int tc_err = 0;
-    NEGF_TRY(read_tc_error(&tc_err));
+    const double *tr = hTr_, *trj = hTrJ_;
+    const int* rst = hRst_;
+    NEGF_CUDA_TRY(cudaMemcpyAsync(hTr_, dTr_, sizeof(double) * 4 * nb, cudaMemcpyDeviceToHost, st_));
+    if (sc_()) NEGF_CUDA_TRY(cudaMemcpyAsync(hTrJ_, dTrJ_, sizeof(double) * nb, cudaMemcpyDeviceToHost, st_));
+    NEGF_CUDA_TRY(cudaMemcpyAsync(hRst_, dStatus_, sizeof(int) * nb, cudaMemcpyDeviceToHost, st_));
+    NEGF_TRY(read_tc_error());
     NEGF_CUDA_TRY(cudaStreamSynchronize(st_));
-    if (tc_err) return NEGF_ETIMEDOUT;
+    if (*hErr_) return NEGF_ETIMEDOUT;
     for (int i = 0; i < nb; ++i) {
       negf_result& o = res[c0 + i];
       const Item& it = items[i];

@@ -140,6 +140,13 @@ class Engine {
   // pinned host staging
   double* hPin_ = nullptr;
   size_t hPinBytes_ = 0;
+  // pinned destinations of the small results read inside and after the phases: a copy into
+  // pageable memory would hold the host back until the device got there
+  void* hSmall_ = nullptr;
+  size_t hSmallBytes_ = 0;
+  double *hDos_ = nullptr, *hTr_ = nullptr, *hTrJ_ = nullptr;     // [2 S_], [4 B_], [B_]
+  unsigned long long *hR0_ = nullptr, *hRk_ = nullptr;            // [cap] residual norms of an inverse
+  int *hInfo_ = nullptr, *hSr_ = nullptr, *hRst_ = nullptr, *hErr_ = nullptr;   // [cap], [4 S_], [B_], [1]
 
   InvWork inv_;
 
@@ -220,7 +227,7 @@ class Engine {
   int alloc();
   int alloc_tc();         // the tensor-core workspace
  public:
-  int read_tc_error(int* err);
+  int read_tc_error();
  private:
   void free_tc();
   // items [first, first + count) of a sliced operand
