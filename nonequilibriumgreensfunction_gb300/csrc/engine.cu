@@ -321,10 +321,10 @@ int Engine::alloc() {
   NEGF_TRY(dalloc(&dSrE_, (size_t)S_, bytes_, dry_, pool_, own_st_));
   NEGF_TRY(dalloc(&dSrHend_, (size_t)S_, bytes_, dry_, pool_, own_st_));
   NEGF_TRY(dalloc(&dSrStatus_, (size_t)S_, bytes_, dry_, pool_, own_st_));
-  {   // inv_work_alloc: R buffer, pivots, INFO, interchange lists
+  {   // inv_work_alloc: R buffer, pivots, row origins, INFO, interchange lists
     const long long cap = std::max(B_, S_);
     if (!dry_) NEGF_TRY(inv_work_alloc(inv_, M_, (int)cap, pool_, own_st_));
-    bytes_ += 16LL * cap * panel_width(M_) * M_ + 4LL * cap * M_ + 4LL * cap + 4LL * cap * kGjMoves;
+    bytes_ += 16LL * cap * panel_width(M_) * M_ + 8LL * cap * M_ + 4LL * cap + 4LL * cap * kGjMoves;
   }
   if (tc_) {
     const long long before = bytes_;
@@ -596,13 +596,14 @@ int Engine::merge_info(int batch) { return merge_info_kernel_launch(batch, inv_.
 // Gauss-Jordan, then ns_steps_ Newton-Schulz steps X <- X + X (I - W X) with W X and X R
 // formed at each step's slices (ns_step_; the last residual is FP64-class), and up to
 // ns_max_steps_ in all for a matrix whose residual norm before its last update is above
-// ns_tol_.  A matrix is inverted again in
+// ns_tol_.  staged: the matrices are in dWinv_ and, in FP32, dW32_ (at most tc_cap_ of them), and
+// A only receives the inverses.  A matrix is inverted again in
 // FP64 when its first residual norm is above ns_accept_, its FP32 factorisation met a zero
 // pivot, or it is still above ns_tol_ after ns_max_steps_ steps.
-int Engine::invert(double2* A, long long sA, int batch, int* status_dev) {
+int Engine::invert(double2* A, long long sA, int batch, int* status_dev, bool staged) {
   cudaEvent_t ph;
   timed_begin(st_, TK_PH_INV, 0.0, &ph);
-  const int rc = invert_impl(A, sA, batch, status_dev);
+  const int rc = staged ? invert_refined(A, sA, batch, status_dev, true) : invert_impl(A, sA, batch, status_dev);
   timed_end(st_, TK_PH_INV, ph);
   return rc;
 }
@@ -613,15 +614,16 @@ int Engine::invert_impl(double2* A, long long sA, int batch, int* status_dev) {
     return merge_info_kernel_launch(batch, inv_.info, status_dev, st_);
   }
   for (int o = 0; o < batch; o += tc_cap_)
-    NEGF_TRY(invert_refined(A + o * sA, sA, std::min(tc_cap_, batch - o), status_dev + o));
+    NEGF_TRY(invert_refined(A + o * sA, sA, std::min(tc_cap_, batch - o), status_dev + o, false));
   return NEGF_OK;
 }
 
-int Engine::invert_refined(double2* A, long long sA, int batch, int* status_dev) {
+int Engine::invert_refined(double2* A, long long sA, int batch, int* status_dev, bool staged) {
   const double2 one = make_double2(1, 0), zero = make_double2(0, 0);
-  NEGF_TRY(split_copy(M_, batch, A, sA, dWinv_, MM_, dW32_, MM_, st_));
+  if (!staged) NEGF_TRY(split_copy(M_, batch, A, sA, dWinv_, MM_, dW32_, MM_, st_));
   NEGF_TRY(invert_f32(batch));
-  NEGF_TRY(to_f64(M_, batch, dW32_, MM_, A, sA, st_));
+  if (inv_.columns_pending) NEGF_TRY(to_f64_columns(M_, batch, dW32_, MM_, inv_.orig, A, sA, st_));
+  else NEGF_TRY(to_f64(M_, batch, dW32_, MM_, A, sA, st_));
   const int* info32 = hInfo_;
   NEGF_CUDA_TRY(cudaMemcpyAsync(hInfo_, inv_.info, sizeof(int) * batch, cudaMemcpyDeviceToHost, st_));
   NEGF_CUDA_TRY(cudaMemsetAsync(dRnorm_, 0, sizeof(unsigned long long) * batch, st_));
@@ -1116,8 +1118,14 @@ int Engine::solve_rgf_impl(const std::vector<Item>& items, bool keep_columns) {
         fw.zsub = dQ_;
       }
     }
+    // on the tensor cores W goes straight to where the inverse keeps it, in FP64 and FP32
+    const bool staged = tc_ && B <= tc_cap_;
+    if (staged) {
+      fw.W = dWinv_; fw.sW = MM_;
+      fw.W32 = dW32_; fw.sW32 = MM_;
+    }
     NEGF_TRY(form_w(fw, st_));
-    return invert(dG_ + (long long)x * MM_, sG, B, dStatus_);
+    return invert(dG_ + (long long)x * MM_, sG, B, dStatus_, staged);
   };
   cur_slices_ = s_rgf_;
 

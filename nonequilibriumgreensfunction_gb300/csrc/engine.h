@@ -188,13 +188,13 @@ class Engine {
   double last_rnorm_max_ = 0.0;
   // Newton-Schulz policy of the mixed form (negf_set_refinement); <= 0 restores a default
   int set_refinement(int max_steps, double tol, double accept);
-  int invert(double2* A, long long sA, int batch, int* status_dev);
+  int invert(double2* A, long long sA, int batch, int* status_dev, bool staged = false);
   // FP32 Gauss-Jordan form per batch (rounded up to a power of two): 0 three launches per
   // panel, 1 fused; chosen by timing both on the first inverse of that batch size
   std::map<int, int> gj_form_;
   int invert_f32(int batch);
   int invert_impl(double2* A, long long sA, int batch, int* status_dev);
-  int invert_refined(double2* A, long long sA, int batch, int* status_dev);
+  int invert_refined(double2* A, long long sA, int batch, int* status_dev, bool staged);
   int solve_sr_impl(const std::vector<SrJob>& jobs, std::vector<int>& status, std::vector<int>& iters);
   // FP64 solves of small cross-sections take one kernel per phase (small_f64.cu)
   bool small_() const { return !mixed_ && !tc_ && M_ <= SMALL_MAX_M; }

@@ -180,7 +180,7 @@ constexpr int RP_MAX_N = 640;   // 640 threads of up to 102 registers
 constexpr int RP_C = 32;
 template <int MAXT>   // threads at most: 512 (128 registers each) or RP_MAX_N (96)
 __global__ void __launch_bounds__(MAXT, 1) gj_panel_reg_kernel(float2* A, long long sA, int n, int k0, int kb,
-                                                                   int* ipiv, int* info, int* moves) {
+                                                                   int* ipiv, int* info, int* moves, int* orig) {
   __shared__ __align__(16) float2 raw[RP_C], piv[RP_C];   // pivot row, unscaled and scaled
   __shared__ unsigned w_key[RP_MAX_N / 32];
   __shared__ int w_pos[RP_MAX_N / 32];
@@ -195,6 +195,7 @@ __global__ void __launch_bounds__(MAXT, 1) gj_panel_reg_kernel(float2* A, long l
   for (int j = 0; j < RP_C; ++j)
     row[j] = (live && j < kb) ? Ab[(long long)(k0 + j) * n + t] : make_float2(0.f, 0.f);
   int pos = live ? t : 0x7fffffff;
+  const int from = live && k0 > 0 ? orig[(long long)b * n + t] : t;   // the row of A that is here
   if (t == 0) s_extra = kb;
   // key of a pivot candidate: larger |re|+|im| first (non-negative floats order as their bits),
   // 0 = no candidate (a row above the step, a NaN)
@@ -282,6 +283,7 @@ __global__ void __launch_bounds__(MAXT, 1) gj_panel_reg_kernel(float2* A, long l
 #pragma unroll
     for (int j = 0; j < RP_C; ++j)
       if (j < kb) Ab[(long long)(k0 + j) * n + pos] = row[j];
+    orig[(long long)b * n + pos] = from;
     const int q = (pos >= k0 && pos < k0 + kb) ? pos - k0 : (pos != t ? atomicAdd(&s_extra, 1) : -1);
     if (q >= 0) {
       mv[1 + 2 * q] = pos;
@@ -719,6 +721,7 @@ int inv_work_alloc(InvWork& w, int n, int batch, cudaMemPool_t pool, cudaStream_
   if (!get((void**)&w.rbuf, sizeof(double2) * (size_t)batch * w.nb * n)) return NEGF_ENOMEM;
   if (!get((void**)&w.ipiv, sizeof(int) * (size_t)batch * n)) return NEGF_ENOMEM;
   if (!get((void**)&w.info, sizeof(int) * (size_t)batch)) return NEGF_ENOMEM;
+  if (!get((void**)&w.orig, sizeof(int) * (size_t)batch * n)) return NEGF_ENOMEM;
   if (!get((void**)&w.moves, sizeof(int) * (size_t)batch * kGjMoves)) return NEGF_ENOMEM;
   w.n_cap = n;
   w.batch_cap = batch;
@@ -726,7 +729,7 @@ int inv_work_alloc(InvWork& w, int n, int batch, cudaMemPool_t pool, cudaStream_
 }
 
 void inv_work_free(InvWork& w, cudaStream_t st) {
-  for (void* p : {(void*)w.rbuf, (void*)w.ipiv, (void*)w.info, (void*)w.moves})
+  for (void* p : {(void*)w.rbuf, (void*)w.ipiv, (void*)w.info, (void*)w.orig, (void*)w.moves})
     if (p) {
       if (w.pooled) cudaFreeAsync(p, st);
       else cudaFree(p);
@@ -750,6 +753,7 @@ int sm_count_cached() {
 // FP32 inverse as one fused launch per batch (plus the column interchanges)
 int gj_invert_fused_f32(float2* A, long long sA, int n, int batch, InvWork& w, cudaStream_t st) {
   const size_t smem = gj_fused_smem(n);
+  w.columns_pending = false;
   NEGF_CUDA_TRY(cudaFuncSetAttribute(gj_fused_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   NEGF_CUDA_TRY(cudaMemsetAsync(w.info, 0, sizeof(int) * batch, st));
   cudaEvent_t ev;
@@ -790,7 +794,7 @@ int gj_invert(T* A, long long sA, int n, int batch, InvWork& w, cudaStream_t st)
     if (sizeof(T) == 8 && n <= RP_MAX_N) {
       const int threads = (n + 31) / 32 * 32;
       auto panel = threads <= 512 ? gj_panel_reg_kernel<512> : gj_panel_reg_kernel<RP_MAX_N>;
-      panel<<<batch, threads, 0, st>>>(reinterpret_cast<float2*>(A), sA, n, k0, kb, w.ipiv, w.info, w.moves);
+      panel<<<batch, threads, 0, st>>>(reinterpret_cast<float2*>(A), sA, n, k0, kb, w.ipiv, w.info, w.moves, w.orig);
       moves = w.moves;
     } else {
       gj_panel_kernel<T><<<batch, PANEL_THREADS, smem, st>>>(A, sA, n, k0, kb, w.ipiv, w.info);
@@ -821,6 +825,8 @@ int gj_invert(T* A, long long sA, int n, int batch, InvWork& w, cudaStream_t st)
       count_launch();
     }
   }
+  w.columns_pending = sizeof(T) == 8 && n <= RP_MAX_N;   // the register panels tracked the rows
+  if (w.columns_pending) return NEGF_OK;
   dim3 g3((n + 127) / 128, batch);
   gj_colswap_kernel<T><<<g3, 128, 0, st>>>(A, sA, n, w.ipiv);
   NEGF_CUDA_TRY(cudaGetLastError());

@@ -152,6 +152,8 @@ struct InvWork {
   double2* rbuf = nullptr;   // batch * nb * n (FP64; reused as float2 storage by the FP32 form)
   int* ipiv = nullptr;       // batch * n
   int* info = nullptr;       // batch
+  int* orig = nullptr;       // batch * n: row that each place held at first (FP32 form, register panels)
+  bool columns_pending = false;   // the last FP32 inverse left its column interchanges to orig
   int* moves = nullptr;      // batch * kGjMoves: the interchanges of the panel at hand (FP32 form)
   int n_cap = 0, batch_cap = 0, nb = 0;
   bool pooled = false;       // allocated stream-ordered from a memory pool
@@ -165,7 +167,9 @@ int panel_width(int n, int elem_bytes = 16);
 int zinv_f64(double2* A, long long sA, int n, int batch, InvWork& w, cudaStream_t st);
 // FP32 twin (the first guess of the mixed-form inverse).  form 0: panel / interchange /
 // update launches per 32-column panel; form 1: one fused launch with a CTA per matrix (needs
-// cinv_f32_fused_ok).  Both give bitwise the same result.
+// cinv_f32_fused_ok).  Both give bitwise the same result, form 0 perhaps with its columns still
+// to be put in place: w.columns_pending, column k of A is column w.orig[b][k] of the inverse
+// (to_f64_columns).
 int cinv_f32(float2* A, long long sA, int n, int batch, InvWork& w, cudaStream_t st, int form = 0);
 bool cinv_f32_fused_ok(int n, int batch);
 
@@ -221,6 +225,7 @@ struct FormW {
   HopBD hop;
   const double2* zsub; long long sZ;
   double2* W; long long sW;
+  float2* W32 = nullptr; long long sW32 = 0;   // also in FP32 (for an inverse that starts from it)
   // every site shares one 4 x 4 hop block: the coupling term L G R from compact terms,
   // lrow = L by rows (left form), rrow = R by columns (right form)
   int use_rows = 0;
@@ -373,6 +378,9 @@ int reduce_sites(int batch, int nsite_total, int nf, int nslots, const Item* ite
 // rnorm[b] = atomic max of the row-sum norm of R as the bit pattern of a double
 int to_f32(int n, int batch, const double2* src, long long sS, float2* dst, long long sD, cudaStream_t st);
 int to_f64(int n, int batch, const float2* src, long long sS, double2* dst, long long sD, cudaStream_t st);
+// dst's column orig[b][k] = src's column k
+int to_f64_columns(int n, int batch, const float2* src, long long sS, const int* orig, double2* dst, long long sD,
+                   cudaStream_t st);
 int split_copy(int n, int batch, const double2* src, long long sS, double2* d64, long long s64, float2* d32,
                long long s32, cudaStream_t st);
 int ns_residual(int n, int batch, double2* T, long long sT, unsigned long long* rnorm, cudaStream_t st);

@@ -23,7 +23,32 @@ __device__ __forceinline__ double2 hbe(const HopBD& h, int s, int a, int c) {
   return h.hb[((long long)s * h.norb + a) * h.norb + c];
 }
 
+// FP64 <-> FP32 by integer operations where the value is in FP32's normal range (or zero): the
+// conversion instructions occupy the FP64 pipe for several multiply-adds each.  Rounded to
+// nearest even, as the conversions round.
+__device__ __forceinline__ float narrow(double x) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+  const unsigned e = (unsigned)(b >> 52) & 0x7FFu, sign = (unsigned)(b >> 32) & 0x80000000u;
+  if (e - 897u > 1150u - 897u) return (b << 1) == 0 ? __uint_as_float(sign) : (float)x;
+  const unsigned long long t = (b & 0x7FFFFFFFFFFFFFFFULL) - ((unsigned long long)896 << 52);
+  return __uint_as_float(sign | (unsigned)((t + 0x0FFFFFFFULL + ((t >> 29) & 1ULL)) >> 29));
+}
+__device__ __forceinline__ double widen(float x) {
+  const unsigned b = __float_as_uint(x), m = b & 0x7FFFFFFFu;
+  if (m - 0x00800000u >= 0x7F000000u) return m == 0 ? __longlong_as_double((long long)((unsigned long long)b << 32)) : (double)x;
+  const unsigned long long t = ((unsigned long long)m << 29) + ((unsigned long long)896 << 52);
+  return __longlong_as_double((long long)(t | ((unsigned long long)(b & 0x80000000u) << 32)));
+}
+__device__ __forceinline__ float2 narrow(double2 v) { return make_float2(narrow(v.x), narrow(v.y)); }
+__device__ __forceinline__ double2 widen(float2 v) { return make_double2(widen(v.x), widen(v.y)); }
+
 // ---- W assembly (Energy_Sweep.F90:31-38 + Recursive_Greens.F90:18-20 / :70-72) ----------
+// element e of item b's W, and its FP32 copy where the inverse starts from one
+__device__ __forceinline__ void store_w(const FormW& a, double2* W, int b, long long e, double2 v) {
+  W[e] = v;
+  if (a.W32) a.W32[(long long)b * a.sW32 + e] = narrow(v);
+}
+
 __global__ void form_w_kernel(FormW a) {
   const int b = blockIdx.y;
   const int n = a.n;
@@ -62,7 +87,7 @@ __global__ void form_w_kernel(FormW a) {
       }
       v = csub(v, acc);
     }
-    W[e] = v;
+    store_w(a, W, b, e, v);
   }
 }
 
@@ -83,35 +108,84 @@ __device__ __forceinline__ void term_fma(double2& acc, double2 x, double2 c, int
 
 // W with the coupling term from the compact terms of a hop block shared by every site:
 // W(i, j) -= sum_p L(a, p) sum_q G(4 si + p, 4 sj + q) R(q, c) over the nonzero terms only
-// (i = 4 si + a, j = 4 sj + c), the nesting of form_w_blocks_kernel.  Lanes of a warp share
-// j and take the same kinds of terms, so they branch together; the G elements come from L1.
-__global__ void form_w_rows_kernel(FormW a) {
-  const int b = blockIdx.y;
-  const int n = a.n;
+// (i = 4 si + a, j = 4 sj + c), the nesting of form_w_blocks_kernel.  A warp takes 32 rows of a
+// site's four columns at a time: each lane forms its row of T = G R once, and the rows of L T
+// read the T of their site from shared memory.  Ten FP64 operations per element with two-term
+// rows instead of the fourteen of an element that forms its own inner sums; the FP64 pipe (two
+// multiply-adds per clock and SM) bounds the kernel.  Per element the operations and their
+// order are those of the element-wise form.  n = 400, 32 items on GB300: 291 -> 187 us; n = 144:
+// 42 -> 34 us.
+constexpr int FW_WARPS = 8, FW_SITES = 1;   // site columns of a warp
+// PAIR: every row of both lists is one real and one imaginary term (the wire models); the
+// general loop over kinds costs the FP64 pipe the instructions of the kinds it does not take
+template <bool PAIR>
+__global__ void __launch_bounds__(FW_WARPS * 32) form_w_rows_kernel(FormW a) {
+  __shared__ double2 gs[FW_WARPS][4][32], ts[FW_WARPS][4][32];
+  const int b = blockIdx.z, n = a.n;
   const long long nn = (long long)n * n;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int i = blockIdx.x * 32 + lane, ra = i & 3, l0 = lane & ~3;   // n is a multiple of 4: whole sites
+  const bool live = i < n;
   const Item it = a.items[b];
   const double2* Hx = a.Hall + ((long long)it.slot * a.npx + a.x) * nn;
   const double2* gp = a.gprev + (long long)b * a.sG;
   const double2* sl = (a.x == 0 && a.sigL) ? a.sigL + (long long)b * a.sSig : nullptr;
   const double2* sr = (a.x == a.npx - 1 && a.sigR) ? a.sigR + (long long)b * a.sSig : nullptr;
   double2* W = a.W + (long long)b * a.sW;
-  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < nn; e += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(e % n), j = (int)(e / n);
-    double2 v = make_double2(-Hx[e].x, -Hx[e].y);
-    if (i == j) { v.x += it.energy; v.y += a.eta; }
-    if (sl) v = csub(v, sl[e]);
-    if (sr) v = csub(v, sr[e]);
-    const int ra = i & 3, ca = j & 3;
-    const double2* gb = gp + (long long)(j - ca) * n + (i - ra);   // G(4 si + p, 4 sj + q) = gb[q n + p]
-    double2 acc = make_double2(0.0, 0.0);
-    for (int tl = 0; tl < a.lrow.cnt[ra]; ++tl) {
-      const int p = a.lrow.p[ra][tl];
-      double2 t = make_double2(0.0, 0.0);
-      for (int tr = 0; tr < a.rrow.cnt[ca]; ++tr)
-        term_fma(t, gb[(long long)a.rrow.p[ca][tr] * n + p], a.rrow.c[ca][tr], a.rrow.kind[ca][tr], false);
-      term_fma(acc, t, a.lrow.c[ra][tl], a.lrow.kind[ra][tl], true);
+  double2 (*g)[32] = gs[warp], (*t)[32] = ts[warp];
+  // this lane's row of L (read once: the lanes of a warp read four different rows)
+  const int lcnt = a.lrow.cnt[ra];
+  int lp[4], lkind[4];
+  double2 lc[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    lp[q] = q < lcnt ? a.lrow.p[ra][q] : 0;
+    lkind[q] = q < lcnt ? a.lrow.kind[ra][q] : 0;
+    lc[q] = q < lcnt ? a.lrow.c[ra][q] : make_double2(0.0, 0.0);
+  }
+  for (int s = 0; s < FW_SITES; ++s) {
+    const int sj = (blockIdx.y * FW_SITES + s) * FW_WARPS + warp;
+    if (4 * sj >= n) break;
+    const long long e0 = (long long)(4 * sj) * n + i;
+    double2 h[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      g[c][lane] = live ? gp[e0 + (long long)c * n] : make_double2(0.0, 0.0);
+      h[c] = live ? Hx[e0 + (long long)c * n] : make_double2(0.0, 0.0);
     }
-    W[e] = csub(v, acc);
+    __syncwarp();
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      double2 v = make_double2(0.0, 0.0);
+      if constexpr (PAIR) {
+        term_fma(v, g[a.rrow.p[c][0]][lane], a.rrow.c[c][0], 0, false);
+        term_fma(v, g[a.rrow.p[c][1]][lane], a.rrow.c[c][1], 1, false);
+      } else
+      for (int tr = 0; tr < a.rrow.cnt[c]; ++tr)
+        term_fma(v, g[a.rrow.p[c][tr]][lane], a.rrow.c[c][tr], a.rrow.kind[c][tr], false);
+      t[c][lane] = v;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const long long e = e0 + (long long)c * n;
+      double2 v = make_double2(-h[c].x, -h[c].y);
+      if ((4 * sj) / 32 == (int)blockIdx.x) {   // (the warp's rows meet the diagonal)
+        if (i == 4 * sj + c) { v.x += it.energy; v.y += a.eta; }
+      }
+      if (live && sl) v = csub(v, sl[e]);
+      if (live && sr) v = csub(v, sr[e]);
+      double2 acc = make_double2(0.0, 0.0);
+      if constexpr (PAIR) {
+        term_fma(acc, t[c][l0 + lp[0]], lc[0], 0, true);
+        term_fma(acc, t[c][l0 + lp[1]], lc[1], 1, true);
+      } else
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (q < lcnt) term_fma(acc, t[c][l0 + lp[q]], lc[q], lkind[q], true);
+      if (live) store_w(a, W, b, e, csub(v, acc));
+    }
+    __syncwarp();
   }
 }
 
@@ -171,7 +245,7 @@ __global__ void form_w_blocks_kernel(FormW a) {
         if (si == sj && r == c) { v.x += it.energy; v.y += a.eta; }
         if (sl) v = csub(v, sl[e]);
         if (sr) v = csub(v, sr[e]);
-        W[e] = csub(v, acc);
+        store_w(a, W, b, e, csub(v, acc));
       }
     }
   }
@@ -805,7 +879,14 @@ __global__ void reduce_sites_kernel(int batch, int total, int nf, int nslots, co
 // =====================================================================================
 int form_w(const FormW& a, cudaStream_t st) {
   if (a.gprev && a.use_rows && a.hop.norb == 4 && !a.zsub && a.n % 4 == 0) {
-    form_w_rows_kernel<<<ew_grid((long long)a.n * a.n, a.batch), EW_THREADS, 0, st>>>(a);
+    const int sites = FW_WARPS * FW_SITES;
+    const dim3 grid((a.n + 31) / 32, (a.n / 4 + sites - 1) / sites, a.batch);
+    bool pair = true;
+    for (int r = 0; r < 4; ++r)
+      for (const HopRows* l : {&a.lrow, &a.rrow})
+        pair = pair && l->cnt[r] == 2 && l->kind[r][0] == 0 && l->kind[r][1] == 1;
+    auto kernel = pair ? form_w_rows_kernel<true> : form_w_rows_kernel<false>;
+    kernel<<<grid, FW_WARPS * 32, 0, st>>>(a);
     NEGF_CUDA_TRY(cudaGetLastError());
     count_launch();
     return NEGF_OK;
@@ -1015,7 +1096,7 @@ __global__ void to_f32_kernel(int n, const double2* src, long long sS, float2* d
   const double2* s = src + (long long)b * sS;
   float2* d = dst + (long long)b * sD;
   for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < nn; e += (long long)gridDim.x * blockDim.x)
-    d[e] = make_float2((float)s[e].x, (float)s[e].y);
+    d[e] = narrow(s[e]);
 }
 
 // one read of the matrix to invert: its FP64 copy (kept for the residual) and FP32 copy
@@ -1029,7 +1110,7 @@ __global__ void split_copy_kernel(int n, const double2* src, long long sS, doubl
   for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < nn; e += (long long)gridDim.x * blockDim.x) {
     const double2 v = s[e];
     a[e] = v;
-    c[e] = make_float2((float)v.x, (float)v.y);
+    c[e] = narrow(v);
   }
 }
 
@@ -1039,7 +1120,23 @@ __global__ void to_f64_kernel(int n, const float2* src, long long sS, double2* d
   const float2* s = src + (long long)b * sS;
   double2* d = dst + (long long)b * sD;
   for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < nn; e += (long long)gridDim.x * blockDim.x)
-    d[e] = make_double2((double)s[e].x, (double)s[e].y);
+    d[e] = widen(s[e]);
+}
+
+// The same of an FP32 Gauss-Jordan inverse whose column interchanges are still to be undone:
+// column k becomes column orig[k]
+__global__ void to_f64_columns_kernel(int n, const float2* src, long long sS, const int* orig, double2* dst,
+                                      long long sD) {
+  const int b = blockIdx.y;
+  const long long nn = (long long)n * n;
+  const float2* s = src + (long long)b * sS;
+  double2* d = dst + (long long)b * sD;
+  const int* o = orig + (long long)b * n;
+  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < nn; e += (long long)gridDim.x * blockDim.x) {
+    const int k = (int)(e / n), i = (int)(e - (long long)k * n);
+    const float2 v = s[e];
+    d[(long long)o[k] * n + i] = widen(v);
+  }
 }
 
 // R = I - T in place; rnorm[b] = max over rows of sum_j |R_ij| (the infinity norm, the
@@ -1107,6 +1204,14 @@ int split_copy(int n, int batch, const double2* src, long long sS, double2* d64,
 
 int to_f64(int n, int batch, const float2* src, long long sS, double2* dst, long long sD, cudaStream_t st) {
   to_f64_kernel<<<ew_grid((long long)n * n, batch), EW_THREADS, 0, st>>>(n, src, sS, dst, sD);
+  NEGF_CUDA_TRY(cudaGetLastError());
+  count_launch();
+  return NEGF_OK;
+}
+
+int to_f64_columns(int n, int batch, const float2* src, long long sS, const int* orig, double2* dst, long long sD,
+                   cudaStream_t st) {
+  to_f64_columns_kernel<<<ew_grid((long long)n * n, batch), EW_THREADS, 0, st>>>(n, src, sS, orig, dst, sD);
   NEGF_CUDA_TRY(cudaGetLastError());
   count_launch();
   return NEGF_OK;
