@@ -45,6 +45,7 @@ constexpr int kSrBlocks = 13;
 enum SrRole { SR_ALPHA = 0, SR_T, SR_TT, SR_TOLDL, SR_TOLDR, SR_TL, SR_TR, SR_TMP, SR_W1, SR_TN, SR_TTN, SR_CHG, SR_W2 };
 
 __global__ void merge_info_k(int batch, const int* info, int* status) {
+  pdl_wait();
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b < batch && status[b] == 0 && info[b] != 0) status[b] = info[b];
 }
@@ -129,7 +130,7 @@ double __longlong_as_double_host(unsigned long long v) {
 }  // namespace
 
 int merge_info_kernel_launch(int batch, const int* info, int* status, cudaStream_t st) {
-  merge_info_k<<<(batch + 127) / 128, 128, 0, st>>>(batch, info, status);
+  pdl_launch(merge_info_k, (batch + 127) / 128, 128, 0, st, batch, info, status);
   NEGF_CUDA_TRY(cudaGetLastError());
   count_launch();
   return NEGF_OK;

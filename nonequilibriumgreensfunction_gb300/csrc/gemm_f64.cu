@@ -39,6 +39,7 @@ __device__ __forceinline__ T load_b(const T* __restrict__ B, int ldb, int n, int
 
 template <int OPA, int OPB, typename T>
 __global__ void __launch_bounds__(NT) zgemm_kernel(GemmBatchT<T> g) {
+  pdl_wait();
   __shared__ T As[2][BK][BM];
   __shared__ T Bs[2][BK][BN];
   const int b = blockIdx.z;
@@ -133,7 +134,7 @@ __global__ void __launch_bounds__(NT) zgemm_kernel(GemmBatchT<T> g) {
 template <int OPA, int OPB, typename T>
 void launch(const GemmBatchT<T>& g, cudaStream_t st) {
   dim3 grid((g.m + BM - 1) / BM, (g.n + BN - 1) / BN, g.batch);
-  zgemm_kernel<OPA, OPB, T><<<grid, NT, 0, st>>>(g);
+  pdl_launch(zgemm_kernel<OPA, OPB, T>, grid, NT, 0, st, g);
 }
 
 }  // namespace

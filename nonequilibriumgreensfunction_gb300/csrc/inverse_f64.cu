@@ -144,6 +144,7 @@ __device__ __forceinline__ void panel_factor(T* Ps, int n, int k0, int kb, int* 
 template <typename T>
 __global__ void __launch_bounds__(PANEL_THREADS) gj_panel_kernel(T* A, long long sA, int n, int k0, int kb,
                                                                  int* ipiv, int* info) {
+  pdl_wait();
   extern __shared__ __align__(16) unsigned char panel_raw[];
   T* Ps = reinterpret_cast<T*>(panel_raw);
   using R = typename CplxTraits<T>::R;
@@ -181,6 +182,7 @@ constexpr int RP_C = 32;
 template <int MAXT>   // threads at most: 512 (128 registers each) or RP_MAX_N (96)
 __global__ void __launch_bounds__(MAXT, 1) gj_panel_reg_kernel(float2* A, long long sA, int n, int k0, int kb,
                                                                    int* ipiv, int* info, int* moves, int* orig) {
+  pdl_wait();
   __shared__ __align__(16) float2 raw[RP_C], piv[RP_C];   // pivot row, unscaled and scaled
   __shared__ unsigned w_key[RP_MAX_N / 32];
   __shared__ int w_pos[RP_MAX_N / 32];
@@ -306,6 +308,7 @@ template <typename T>
 __global__ void __launch_bounds__(SWAP_WARPS * 32) gj_swap_kernel(T* A, long long sA, int n, int k0, int kb,
                                                                   const int* ipiv, const int* moves, T* R,
                                                                   long long sR) {
+  pdl_wait();
   __shared__ int trow[64], torig[64];
   __shared__ int s_nt;
   const int b = blockIdx.y;
@@ -376,6 +379,7 @@ constexpr int UPD_T = 80, UPD_R = 5, UPD_RS = UPD_T + 1;
 template <typename T>
 __global__ void __launch_bounds__(256, sizeof(T) == 8 ? 2 : 1) gj_update_kernel(T* A, long long sA, int n, int k0, int kb, const T* R,
                                                         long long sR) {
+  pdl_wait();
   extern __shared__ __align__(16) unsigned char upd_raw[];
   T* Ps = reinterpret_cast<T*>(upd_raw);              // [kb][UPD_T]
   T* Rs = Ps + 32 * UPD_T;                              // [kb][UPD_RS]
@@ -466,6 +470,7 @@ constexpr int UPD_SLABS = 32 * UPD_T + 32 * UPD_RS;   // float2 of one buffer: P
 __global__ void __launch_bounds__(256, 2) gj_update_f32_pipelined(float2* A, long long sA, int n, int k0, int kb,
                                                                   const float2* R, long long sR, int ntm, int ntn,
                                                                   long long ntiles) {
+  pdl_wait();
   extern __shared__ __align__(16) unsigned char upp_raw[];
   float2* bufs = reinterpret_cast<float2*>(upp_raw);   // [2][UPD_SLABS]
   const int t = threadIdx.x;
@@ -551,6 +556,7 @@ __global__ void __launch_bounds__(256, 2) gj_update_f32_pipelined(float2* A, lon
 // One thread per row: column interchanges in reverse pivot order.
 template <typename T>
 __global__ void gj_colswap_kernel(T* A, long long sA, int n, const int* ipiv) {
+  pdl_wait();
   const int b = blockIdx.y;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -585,6 +591,7 @@ __global__ void gj_colswap_kernel(T* A, long long sA, int n, const int* ipiv) {
 constexpr int FUSED_THREADS = 256, FUSED_JC = 32, FUSED_RS = FUSED_JC + 1, FUSED_MAX_N = 400;
 __global__ void __launch_bounds__(FUSED_THREADS, 2) gj_fused_f32_kernel(float2* A, long long sA, int n, int* ipiv,
                                                                         int* info) {
+  pdl_wait();
   extern __shared__ __align__(16) unsigned char fused_raw[];
   float2* Ps = reinterpret_cast<float2*>(fused_raw);   // [32][n]: the panel, column-major
   float2* Rs = Ps + 32 * n;                             // [32][FUSED_RS]: rows K of a chunk
@@ -758,11 +765,11 @@ int gj_invert_fused_f32(float2* A, long long sA, int n, int batch, InvWork& w, c
   NEGF_CUDA_TRY(cudaMemsetAsync(w.info, 0, sizeof(int) * batch, st));
   cudaEvent_t ev;
   timed_begin(st, TK_F32, 8.0 * (double)n * n * n * batch, &ev);
-  gj_fused_f32_kernel<<<batch, FUSED_THREADS, smem, st>>>(A, sA, n, w.ipiv, w.info);
+  pdl_launch(gj_fused_f32_kernel, batch, FUSED_THREADS, smem, st, A, sA, n, w.ipiv, w.info);
   NEGF_CUDA_TRY(cudaGetLastError());
   timed_end(st, TK_F32, ev);
   dim3 g3((n + 127) / 128, batch);
-  gj_colswap_kernel<float2><<<g3, 128, 0, st>>>(A, sA, n, w.ipiv);
+  pdl_launch(gj_colswap_kernel<float2>, g3, 128, 0, st, A, sA, n, w.ipiv);
   NEGF_CUDA_TRY(cudaGetLastError());
   count_launch(2);
   return NEGF_OK;
@@ -794,15 +801,15 @@ int gj_invert(T* A, long long sA, int n, int batch, InvWork& w, cudaStream_t st)
     if (sizeof(T) == 8 && n <= RP_MAX_N) {
       const int threads = (n + 31) / 32 * 32;
       auto panel = threads <= 512 ? gj_panel_reg_kernel<512> : gj_panel_reg_kernel<RP_MAX_N>;
-      panel<<<batch, threads, 0, st>>>(reinterpret_cast<float2*>(A), sA, n, k0, kb, w.ipiv, w.info, w.moves, w.orig);
+      pdl_launch(panel, batch, threads, 0, st, reinterpret_cast<float2*>(A), sA, n, k0, kb, w.ipiv, w.info, w.moves, w.orig);
       moves = w.moves;
     } else {
-      gj_panel_kernel<T><<<batch, PANEL_THREADS, smem, st>>>(A, sA, n, k0, kb, w.ipiv, w.info);
+      pdl_launch(gj_panel_kernel<T>, batch, PANEL_THREADS, smem, st, A, sA, n, k0, kb, w.ipiv, w.info);
     }
     NEGF_CUDA_TRY(cudaGetLastError());
     timed_end(st, TK_PANEL, ev);
     dim3 g2((n + SWAP_WARPS - 1) / SWAP_WARPS, batch);
-    gj_swap_kernel<T><<<g2, SWAP_WARPS * 32, 0, st>>>(A, sA, n, k0, kb, w.ipiv, moves, rbuf, sR);
+    pdl_launch(gj_swap_kernel<T>, g2, SWAP_WARPS * 32, 0, st, A, sA, n, k0, kb, w.ipiv, moves, rbuf, sR);
     NEGF_CUDA_TRY(cudaGetLastError());
     count_launch(2);
     // A(:, j) += P R(:, j) for the columns outside the panel
@@ -813,12 +820,12 @@ int gj_invert(T* A, long long sA, int n, int batch, InvWork& w, cudaStream_t st)
       if constexpr (sizeof(T) == 8) {
         const long long ntiles = (long long)nt * nt * batch;
         const int grid = (int)std::min<long long>(ntiles, 2LL * sm_count_cached());
-        gj_update_f32_pipelined<<<grid, 256, upp_smem, st>>>(reinterpret_cast<float2*>(A), sA, n, k0, kb,
+        pdl_launch(gj_update_f32_pipelined, grid, 256, upp_smem, st, reinterpret_cast<float2*>(A), sA, n, k0, kb,
                                                              reinterpret_cast<const float2*>(rbuf), sR, nt, nt,
                                                              ntiles);
       } else {
         dim3 gu(nt, nt, batch);
-        gj_update_kernel<T><<<gu, 256, upd_smem, st>>>(A, sA, n, k0, kb, rbuf, sR);
+        pdl_launch(gj_update_kernel<T>, gu, 256, upd_smem, st, A, sA, n, k0, kb, rbuf, sR);
       }
       NEGF_CUDA_TRY(cudaGetLastError());
       timed_end(st, sizeof(T) == 8 ? TK_F32 : TK_GEMM, eu);
@@ -828,7 +835,7 @@ int gj_invert(T* A, long long sA, int n, int batch, InvWork& w, cudaStream_t st)
   w.columns_pending = sizeof(T) == 8 && n <= RP_MAX_N;   // the register panels tracked the rows
   if (w.columns_pending) return NEGF_OK;
   dim3 g3((n + 127) / 128, batch);
-  gj_colswap_kernel<T><<<g3, 128, 0, st>>>(A, sA, n, w.ipiv);
+  pdl_launch(gj_colswap_kernel<T>, g3, 128, 0, st, A, sA, n, w.ipiv);
   NEGF_CUDA_TRY(cudaGetLastError());
   count_launch();
   return NEGF_OK;

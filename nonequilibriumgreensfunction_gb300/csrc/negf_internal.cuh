@@ -10,6 +10,7 @@
 #include <cstdint>
 #include <cstdio>
 #include <mutex>
+#include <utility>
 #include <vector>
 
 #include "../../include/negf.h"
@@ -125,6 +126,32 @@ void add_tc_complex_flops(double f);
 void timed_begin(cudaStream_t st, int kind, double flops, cudaEvent_t* a);
 void timed_end(cudaStream_t st, int kind, cudaEvent_t a);
 void instrument_resolve();   // accumulate the elapsed times of finished event pairs
+
+// ----------------------------------------------------------------------------------
+// Dependent launches.  A solve is thousands of kernels of a few microseconds, each waiting for
+// the one before.  pdl_launch lets the device prepare a kernel's launch while its predecessor
+// ends, and pdl_wait, before the first access to memory that another kernel reads or writes (or
+// to tensor memory), waits until the predecessor is complete and its writes are visible.  The
+// kernels do not announce their end early (launch_dependents): CTAs that wait on an SM then take
+// the place and the shared memory of those that work.  Whole calls on GB300, plain launches /
+// these / these with an early announcement: fp64 M = 64 31.3 / 27.1 / 31.6 ms, M = 320 74.2 /
+// 68.2 / 78.5 ms, mixed M = 144 153 / 135 / 160 ms, mixed M = 400 832 / 796 / 876 ms.
+// ----------------------------------------------------------------------------------
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <typename... P, typename... A>
+inline cudaError_t pdl_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+}
 
 // ----------------------------------------------------------------------------------
 // GEMM: C = alpha * op(A) * op(B) + beta * C, strided batch (FP64 complex, SIMT DFMA)

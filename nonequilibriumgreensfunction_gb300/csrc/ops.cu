@@ -50,6 +50,7 @@ __device__ __forceinline__ void store_w(const FormW& a, double2* W, int b, long 
 }
 
 __global__ void form_w_kernel(FormW a) {
+  pdl_wait();
   const int b = blockIdx.y;
   const int n = a.n;
   const long long nn = (long long)n * n;
@@ -120,6 +121,7 @@ constexpr int FW_WARPS = 8, FW_SITES = 1;   // site columns of a warp
 // general loop over kinds costs the FP64 pipe the instructions of the kinds it does not take
 template <bool PAIR>
 __global__ void __launch_bounds__(FW_WARPS * 32) form_w_rows_kernel(FormW a) {
+  pdl_wait();
   __shared__ double2 gs[FW_WARPS][4][32], ts[FW_WARPS][4][32];
   const int b = blockIdx.z, n = a.n;
   const long long nn = (long long)n * n;
@@ -198,6 +200,7 @@ __global__ void __launch_bounds__(FW_WARPS * 32) form_w_rows_kernel(FormW a) {
 // reads and writes its block as four 64-byte column pieces; consecutive threads take
 // consecutive row blocks, so a warp's accesses to a column are contiguous.
 __global__ void form_w_blocks_kernel(FormW a) {
+  pdl_wait();
   const int b = blockIdx.y;
   const int n = a.n, ns = n / 4;
   const long long nblk = (long long)ns * ns;
@@ -254,6 +257,7 @@ __global__ void form_w_blocks_kernel(FormW a) {
 // ---- Y = op(H) X  or  X op(H), H block diagonal ------------------------------------
 __global__ void hop_apply_kernel(HopBD h, int n, int left, int op, const double2* X, long long sX, double2* Y,
                                  long long sY) {
+  pdl_wait();
   const int b = blockIdx.y;
   const long long nn = (long long)n * n;
   const double2* Xb = X + (long long)b * sX;
@@ -287,6 +291,7 @@ __global__ void hop_apply_kernel(HopBD h, int n, int left, int op, const double2
 // lists are kernel parameters sorted by kind, so every lane runs the same kinds of terms;
 // the skipped terms are exact zeros of hop_apply_kernel's sequence.
 __global__ void hop_rows_kernel(HopRows r, int n, int left, const double2* X, long long sX, double2* Y, long long sY) {
+  pdl_wait();
   const int b = blockIdx.y;
   const long long nn = (long long)n * n;
   const double2* Xb = X + (long long)b * sX;
@@ -327,6 +332,7 @@ template <int NOM>
 __global__ void __launch_bounds__(SB_ROWS* SB_KSPLIT) site_blocks_kernel(int n, int no, const double2* Y, long long sY,
                                                                          const double2* X, long long sX, double2* P,
                                                                          long long sP) {
+  pdl_wait();
   __shared__ double2 part[SB_KSPLIT][SB_ROWS][NOM];
   const int b = blockIdx.y;
   const int lr = threadIdx.x % SB_ROWS, kg = threadIdx.x / SB_ROWS;
@@ -367,6 +373,7 @@ __global__ void __launch_bounds__(SB_ROWS* SB_KSPLIT) site_pairs_kernel(int n, i
                                                                         const double2* Y, long long sY,
                                                                         const double2* X, long long sX, double2* P0,
                                                                         double2* P1, double2* P2, long long sP) {
+  pdl_wait();
   __shared__ double2 part[SB_KSPLIT][SB_ROWS][NOM];
   const int b = blockIdx.y;
   const int lr = threadIdx.x % SB_ROWS, kg = threadIdx.x / SB_ROWS;
@@ -412,6 +419,7 @@ __global__ void __launch_bounds__(SB_ROWS* SB_KSPLIT) site_pairs_kernel(int n, i
 // ---- Re sum Q .* conj(X) (one CTA per item, fixed reduction order) -------------------
 __global__ void trace_dot_kernel(int n, const double2* Q, long long sQ, const double2* X, long long sX, double* out,
                                  int out_stride) {
+  pdl_wait();
   __shared__ double red[EW_THREADS];
   const int b = blockIdx.x;
   const long long nn = (long long)n * n;
@@ -433,6 +441,7 @@ __global__ void trace_dot_kernel(int n, const double2* Q, long long sQ, const do
 }
 
 __global__ void gather_kernel(int n, const double2* src, const int* idx, int idx_stride, double2* dst, long long sDst) {
+  pdl_wait();
   const int b = blockIdx.y;
   const long long nn = (long long)n * n;
   const double2* s = src + (long long)idx[(long long)b * idx_stride] * nn;
@@ -442,6 +451,7 @@ __global__ void gather_kernel(int n, const double2* src, const int* idx, int idx
 }
 
 __global__ void copy_kernel(int n, const double2* src, long long sSrc, double2* dst, long long sDst) {
+  pdl_wait();
   const int b = blockIdx.y;
   const long long nn = (long long)n * n;
   const double2* s = src + (long long)b * sSrc;
@@ -451,6 +461,7 @@ __global__ void copy_kernel(int n, const double2* src, long long sSrc, double2* 
 }
 
 __global__ void identity_kernel(int n, double2* A, long long sA) {
+  pdl_wait();
   const int b = blockIdx.y;
   const long long nn = (long long)n * n;
   double2* d = A + (long long)b * sA;
@@ -461,6 +472,7 @@ __global__ void identity_kernel(int n, double2* A, long long sA) {
 // ---- Sancho-Rubio pieces (Contact_Self_Energy.F90:110-223) ---------------------------
 __global__ void form_alpha_kernel(int n, const double* energies, const double2* const* hend, double eta, double extra,
                                   double2* A, long long sA) {
+  pdl_wait();
   const int b = blockIdx.y;
   const long long nn = (long long)n * n;
   const double2* H = hend[b];
@@ -478,6 +490,7 @@ __global__ void form_alpha_kernel(int n, const double* energies, const double2* 
 // pattern exceeds every finite one).  cmax must be zeroed before the launch.
 __global__ void sr_accumulate_kernel(int n, const int* active, const double2* change, long long sC, double2* T,
                                      long long sT, unsigned long long* cmax) {
+  pdl_wait();
   __shared__ double red[EW_THREADS];
   const int b = blockIdx.y;
   const long long nn = (long long)n * n;
@@ -508,6 +521,7 @@ __global__ void sr_accumulate_kernel(int n, const int* active, const double2* ch
 // W = alpha - L T with L = H^H (lead 0) or H (lead 1), H block diagonal
 __global__ void sr_form_final_kernel(HopBD h, int n, int lead, const double2* alpha, long long sA, const double2* T,
                                      long long sT, double2* W, long long sW) {
+  pdl_wait();
   const int b = blockIdx.y;
   const long long nn = (long long)n * n;
   const double2* al = alpha + (long long)b * sA;
@@ -528,6 +542,7 @@ __global__ void sr_form_final_kernel(HopBD h, int n, int lead, const double2* al
 
 // Sigma = L g R; lead 0: H^H g H; lead 1: H g H^H.  Gamma = i (Sigma - Sigma^H).
 __global__ void sr_sigma_kernel(HopBD h, int n, int lead, const double2* g, long long sg, double2* sig, long long sS) {
+  pdl_wait();
   const int b = blockIdx.y;
   const long long nn = (long long)n * n;
   const double2* gb = g + (long long)b * sg;
@@ -552,6 +567,7 @@ __global__ void sr_sigma_kernel(HopBD h, int n, int lead, const double2* g, long
 }
 
 __global__ void gamma_dos_kernel(int n, const double2* sig, long long sS, double2* gam, long long sG, double* dos) {
+  pdl_wait();
   __shared__ double red[EW_THREADS];
   const int b = blockIdx.x;
   const long long nn = (long long)n * n;
@@ -579,6 +595,7 @@ __global__ void gamma_dos_kernel(int n, const double2* sig, long long sS, double
 //      Calculate_Observables.F90:10-43) -------------------------------------------------
 // One thread per (item, x, site).  Gn_site = f1 P1 + f2 P2, Gp_site = (1-f1) P1 + (1-f2) P2.
 __global__ void density_spin_kernel(DensityArgs a) {
+  pdl_wait();
   const int b = blockIdx.y;
   const int nsite = a.npy * a.npz;
   const int total = a.npx * nsite;
@@ -693,6 +710,7 @@ __device__ __forceinline__ void bond_pair(const CurrentArgs& a, const double2* H
 }
 
 __global__ void bond_currents_kernel(CurrentArgs a) {
+  pdl_wait();
   const int b = blockIdx.y;
   const int nsite = a.npy * a.npz;
   const int total = a.npx * nsite;
@@ -746,6 +764,7 @@ __global__ void bond_currents_kernel(CurrentArgs a) {
 // of the density.  or_acc[slot][q][site] += sum_b dE_b/(2 pi) value_b, q fastest across
 // threads so that a warp reads whole site blocks.
 __global__ void orbital_resolved_kernel(CurrentArgs a) {
+  pdl_wait();
   const int no = a.norb, nq = 3 * no * no + no;
   const int nsite = a.npy * a.npz;
   const int total = a.npx * nsite;
@@ -792,6 +811,7 @@ __global__ void orbital_resolved_kernel(CurrentArgs a) {
 // diagonal blocks, up * gds in the electron-hole block, lo * gds in the hole-electron one.
 __global__ void contact_fill_kernel(int n, int no, int nh, int type, int ndiag, const double2* coef, ContactGds g,
                                     double2* sigL, double2* sigR, long long sS) {
+  pdl_wait();
   const int job = blockIdx.y;
   const long long nn = (long long)n * n;
   for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < 2 * nn;
@@ -820,6 +840,7 @@ __global__ void contact_fill_kernel(int n, int no, int nh, int type, int ndiag, 
 
 // out[b][r][a] = X[b](r, site(r)*no + a): the diagonal site blocks of a column-major block
 __global__ void site_diag_kernel(int n, int no, const double2* X, long long sX, double2* out, long long sO) {
+  pdl_wait();
   const int b = blockIdx.y;
   const long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (e >= (long long)n * no) return;
@@ -834,6 +855,7 @@ __global__ void site_diag_kernel(int n, int no, const double2* X, long long sX, 
 __global__ void josephson_kernel(int n, int no, const Item* items, const double2* P1, const double2* P2, long long sP,
                                  const double2* G11, long long sG, const double2* sig, const double2* gam,
                                  long long sS, double* out) {
+  pdl_wait();
   __shared__ double red[EW_THREADS];
   const int b = blockIdx.x;
   const Item it = items[b];
@@ -863,6 +885,7 @@ __global__ void josephson_kernel(int n, int no, const Item* items, const double2
 
 __global__ void reduce_sites_kernel(int batch, int total, int nf, int nslots, const Item* items,
                                     const double* site_out, double* acc) {
+  pdl_wait();
   const long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   const long long per_slot = (long long)nf * total;
   if (i >= per_slot * nslots) return;
@@ -886,19 +909,19 @@ int form_w(const FormW& a, cudaStream_t st) {
       for (const HopRows* l : {&a.lrow, &a.rrow})
         pair = pair && l->cnt[r] == 2 && l->kind[r][0] == 0 && l->kind[r][1] == 1;
     auto kernel = pair ? form_w_rows_kernel<true> : form_w_rows_kernel<false>;
-    kernel<<<grid, FW_WARPS * 32, 0, st>>>(a);
+    pdl_launch(kernel, grid, FW_WARPS * 32, 0, st, a);
     NEGF_CUDA_TRY(cudaGetLastError());
     count_launch();
     return NEGF_OK;
   }
   if (a.gprev && a.hop.hb && a.hop.norb == 4 && !a.zsub && a.n % 4 == 0) {
     const long long nblk = (long long)(a.n / 4) * (a.n / 4);
-    form_w_blocks_kernel<<<ew_grid(nblk, a.batch), 128, 0, st>>>(a);
+    pdl_launch(form_w_blocks_kernel, ew_grid(nblk, a.batch), 128, 0, st, a);
     NEGF_CUDA_TRY(cudaGetLastError());
     count_launch();
     return NEGF_OK;
   }
-  form_w_kernel<<<ew_grid((long long)a.n * a.n, a.batch), EW_THREADS, 0, st>>>(a);
+  pdl_launch(form_w_kernel, ew_grid((long long)a.n * a.n, a.batch), EW_THREADS, 0, st, a);
   NEGF_CUDA_TRY(cudaGetLastError());
   count_launch();
   return NEGF_OK;
@@ -907,12 +930,12 @@ int form_w(const FormW& a, cudaStream_t st) {
 int hop_apply(const HopBD& h, const HopRows* rows, int n, int batch, int left, Op op, const double2* X, long long sX,
               double2* Y, long long sY, cudaStream_t st) {
   if (rows && h.norb == 4 && n % 4 == 0 && X != Y) {
-    hop_rows_kernel<<<ew_grid((long long)n * n, batch), EW_THREADS, 0, st>>>(*rows, n, left, X, sX, Y, sY);
+    pdl_launch(hop_rows_kernel, ew_grid((long long)n * n, batch), EW_THREADS, 0, st, *rows, n, left, X, sX, Y, sY);
     NEGF_CUDA_TRY(cudaGetLastError());
     count_launch();
     return NEGF_OK;
   }
-  hop_apply_kernel<<<ew_grid((long long)n * n, batch), EW_THREADS, 0, st>>>(h, n, left, (int)op, X, sX, Y, sY);
+  pdl_launch(hop_apply_kernel, ew_grid((long long)n * n, batch), EW_THREADS, 0, st, h, n, left, (int)op, X, sX, Y, sY);
   NEGF_CUDA_TRY(cudaGetLastError());
   count_launch();
   return NEGF_OK;
@@ -923,9 +946,9 @@ int site_blocks(int n, int norb, int batch, const double2* Y, long long sY, cons
   if (norb < 1 || norb > 8) return NEGF_EINVAL;
   dim3 grid((n + SB_ROWS - 1) / SB_ROWS, batch);
   if (norb <= 4)
-    site_blocks_kernel<4><<<grid, SB_ROWS * SB_KSPLIT, 0, st>>>(n, norb, Y, sY, X, sX, P, sP);
+    pdl_launch(site_blocks_kernel<4>, grid, SB_ROWS * SB_KSPLIT, 0, st, n, norb, Y, sY, X, sX, P, sP);
   else
-    site_blocks_kernel<8><<<grid, SB_ROWS * SB_KSPLIT, 0, st>>>(n, norb, Y, sY, X, sX, P, sP);
+    pdl_launch(site_blocks_kernel<8>, grid, SB_ROWS * SB_KSPLIT, 0, st, n, norb, Y, sY, X, sX, P, sP);
   NEGF_CUDA_TRY(cudaGetLastError());
   count_launch();
   return NEGF_OK;
@@ -936,9 +959,9 @@ int site_pairs(int n, int norb, int npy, int npz, int batch, const double2* Y, l
   if (norb < 1 || norb > 8 || n != norb * npy * npz) return NEGF_EINVAL;
   dim3 grid((n + SB_ROWS - 1) / SB_ROWS, batch);
   if (norb <= 4)
-    site_pairs_kernel<4><<<grid, SB_ROWS * SB_KSPLIT, 0, st>>>(n, norb, npy, npz, Y, sY, X, sX, P, Py, Pz, sP);
+    pdl_launch(site_pairs_kernel<4>, grid, SB_ROWS * SB_KSPLIT, 0, st, n, norb, npy, npz, Y, sY, X, sX, P, Py, Pz, sP);
   else
-    site_pairs_kernel<8><<<grid, SB_ROWS * SB_KSPLIT, 0, st>>>(n, norb, npy, npz, Y, sY, X, sX, P, Py, Pz, sP);
+    pdl_launch(site_pairs_kernel<8>, grid, SB_ROWS * SB_KSPLIT, 0, st, n, norb, npy, npz, Y, sY, X, sX, P, Py, Pz, sP);
   NEGF_CUDA_TRY(cudaGetLastError());
   count_launch();
   return NEGF_OK;
@@ -948,7 +971,7 @@ int bond_currents(const CurrentArgs& a, cudaStream_t st) {
   if (a.norb > 8 || a.nh < 1 || a.nh > a.norb || a.nf < 8) return NEGF_EINVAL;
   const int total = a.npx * a.npy * a.npz;
   dim3 grid((total + 127) / 128, a.batch);
-  bond_currents_kernel<<<grid, 128, 0, st>>>(a);
+  pdl_launch(bond_currents_kernel, grid, 128, 0, st, a);
   NEGF_CUDA_TRY(cudaGetLastError());
   count_launch();
   return NEGF_OK;
@@ -958,7 +981,7 @@ int orbital_resolved(const CurrentArgs& a, int nslots, cudaStream_t st) {
   if (a.norb > 8 || a.nh < 1 || a.nh > a.norb || !a.or_acc || nslots < 1) return NEGF_EINVAL;
   const long long work = (long long)a.npx * a.npy * a.npz * (3 * a.norb * a.norb + a.norb);
   dim3 grid((unsigned)((work + 255) / 256), nslots);
-  orbital_resolved_kernel<<<grid, 256, 0, st>>>(a);
+  pdl_launch(orbital_resolved_kernel, grid, 256, 0, st, a);
   NEGF_CUDA_TRY(cudaGetLastError());
   count_launch();
   return NEGF_OK;
@@ -967,7 +990,7 @@ int orbital_resolved(const CurrentArgs& a, int nslots, cudaStream_t st) {
 int contact_fill(int n, int no, int nh, int type, int ndiag, int njobs, const double2* coef, const ContactGds& g,
                  double2* sigL, double2* sigR, long long sS, cudaStream_t st) {
   if (njobs < 1) return NEGF_OK;
-  contact_fill_kernel<<<ew_grid(2LL * n * n, njobs), EW_THREADS, 0, st>>>(n, no, nh, type, ndiag, coef, g, sigL, sigR,
+  pdl_launch(contact_fill_kernel, ew_grid(2LL * n * n, njobs), EW_THREADS, 0, st, n, no, nh, type, ndiag, coef, g, sigL, sigR,
                                                                           sS);
   NEGF_CUDA_TRY(cudaGetLastError());
   count_launch();
@@ -976,7 +999,7 @@ int contact_fill(int n, int no, int nh, int type, int ndiag, int njobs, const do
 
 int site_diag(int n, int no, int batch, const double2* X, long long sX, double2* out, long long sO, cudaStream_t st) {
   const long long work = (long long)n * no;
-  site_diag_kernel<<<dim3((unsigned)((work + 255) / 256), batch), 256, 0, st>>>(n, no, X, sX, out, sO);
+  pdl_launch(site_diag_kernel, dim3((unsigned)((work + 255) / 256), batch), 256, 0, st, n, no, X, sX, out, sO);
   NEGF_CUDA_TRY(cudaGetLastError());
   count_launch();
   return NEGF_OK;
@@ -985,7 +1008,7 @@ int site_diag(int n, int no, int batch, const double2* X, long long sX, double2*
 int josephson(int n, int no, int batch, const Item* items, const double2* P1, const double2* P2, long long sP,
               const double2* G11, long long sG, const double2* sig, const double2* gam, long long sS, double* out,
               cudaStream_t st) {
-  josephson_kernel<<<batch, EW_THREADS, 0, st>>>(n, no, items, P1, P2, sP, G11, sG, sig, gam, sS, out);
+  pdl_launch(josephson_kernel, batch, EW_THREADS, 0, st, n, no, items, P1, P2, sP, G11, sG, sig, gam, sS, out);
   NEGF_CUDA_TRY(cudaGetLastError());
   count_launch();
   return NEGF_OK;
@@ -993,7 +1016,7 @@ int josephson(int n, int no, int batch, const Item* items, const double2* P1, co
 
 int trace_dot(int n, int batch, const double2* Q, long long sQ, const double2* X, long long sX, double* out,
               int out_stride, cudaStream_t st) {
-  trace_dot_kernel<<<batch, EW_THREADS, 0, st>>>(n, Q, sQ, X, sX, out, out_stride);
+  pdl_launch(trace_dot_kernel, batch, EW_THREADS, 0, st, n, Q, sQ, X, sX, out, out_stride);
   NEGF_CUDA_TRY(cudaGetLastError());
   count_launch();
   return NEGF_OK;
@@ -1001,21 +1024,21 @@ int trace_dot(int n, int batch, const double2* Q, long long sQ, const double2* X
 
 int gather_blocks(int n, int batch, const double2* src, const int* idx, int idx_stride, double2* dst, long long sDst,
                   cudaStream_t st) {
-  gather_kernel<<<ew_grid((long long)n * n, batch), EW_THREADS, 0, st>>>(n, src, idx, idx_stride, dst, sDst);
+  pdl_launch(gather_kernel, ew_grid((long long)n * n, batch), EW_THREADS, 0, st, n, src, idx, idx_stride, dst, sDst);
   NEGF_CUDA_TRY(cudaGetLastError());
   count_launch();
   return NEGF_OK;
 }
 
 int copy_blocks(int n, int batch, const double2* src, long long sSrc, double2* dst, long long sDst, cudaStream_t st) {
-  copy_kernel<<<ew_grid((long long)n * n, batch), EW_THREADS, 0, st>>>(n, src, sSrc, dst, sDst);
+  pdl_launch(copy_kernel, ew_grid((long long)n * n, batch), EW_THREADS, 0, st, n, src, sSrc, dst, sDst);
   NEGF_CUDA_TRY(cudaGetLastError());
   count_launch();
   return NEGF_OK;
 }
 
 int set_identity(int n, int batch, double2* A, long long sA, cudaStream_t st) {
-  identity_kernel<<<ew_grid((long long)n * n, batch), EW_THREADS, 0, st>>>(n, A, sA);
+  pdl_launch(identity_kernel, ew_grid((long long)n * n, batch), EW_THREADS, 0, st, n, A, sA);
   NEGF_CUDA_TRY(cudaGetLastError());
   count_launch();
   return NEGF_OK;
@@ -1023,7 +1046,7 @@ int set_identity(int n, int batch, double2* A, long long sA, cudaStream_t st) {
 
 int form_alpha(int n, int nprob, const double* energies, const double2* const* hend, double eta, double extra_eta,
                double2* A, long long sA, cudaStream_t st) {
-  form_alpha_kernel<<<ew_grid((long long)n * n, nprob), EW_THREADS, 0, st>>>(n, energies, hend, eta, extra_eta, A, sA);
+  pdl_launch(form_alpha_kernel, ew_grid((long long)n * n, nprob), EW_THREADS, 0, st, n, energies, hend, eta, extra_eta, A, sA);
   NEGF_CUDA_TRY(cudaGetLastError());
   count_launch();
   return NEGF_OK;
@@ -1035,7 +1058,7 @@ int sr_accumulate(int n, int nprob, const int* active, const double2* change, lo
   NEGF_CUDA_TRY(cudaMemsetAsync(bits, 0, sizeof(unsigned long long) * nprob, st));
   const long long nn = (long long)n * n;
   const int per = (int)std::min<long long>((nn + EW_THREADS * 16 - 1) / (EW_THREADS * 16), 64);
-  sr_accumulate_kernel<<<dim3(per, nprob), EW_THREADS, 0, st>>>(n, active, change, sC, T, sT, bits);
+  pdl_launch(sr_accumulate_kernel, dim3(per, nprob), EW_THREADS, 0, st, n, active, change, sC, T, sT, bits);
   NEGF_CUDA_TRY(cudaGetLastError());
   count_launch();
   return NEGF_OK;
@@ -1043,7 +1066,7 @@ int sr_accumulate(int n, int nprob, const int* active, const double2* change, lo
 
 int sr_form_final(const HopBD& h, int n, int nprob, int lead, const double2* alpha, long long sA, const double2* T,
                   long long sT, double2* W, long long sW, cudaStream_t st) {
-  sr_form_final_kernel<<<ew_grid((long long)n * n, nprob), EW_THREADS, 0, st>>>(h, n, lead, alpha, sA, T, sT, W, sW);
+  pdl_launch(sr_form_final_kernel, ew_grid((long long)n * n, nprob), EW_THREADS, 0, st, h, n, lead, alpha, sA, T, sT, W, sW);
   NEGF_CUDA_TRY(cudaGetLastError());
   count_launch();
   return NEGF_OK;
@@ -1052,11 +1075,11 @@ int sr_form_final(const HopBD& h, int n, int nprob, int lead, const double2* alp
 int sr_sigma(const HopBD& h, int n, int nprob, int lead, const double2* g, long long sg, double2* sig, long long sSig,
              double2* gam, long long sGam, double* dos, cudaStream_t st) {
   if (lead >= 0) {  // lead < 0: sig already formed (dense HopX), only Gamma and DOS
-    sr_sigma_kernel<<<ew_grid((long long)n * n, nprob), EW_THREADS, 0, st>>>(h, n, lead, g, sg, sig, sSig);
+    pdl_launch(sr_sigma_kernel, ew_grid((long long)n * n, nprob), EW_THREADS, 0, st, h, n, lead, g, sg, sig, sSig);
     NEGF_CUDA_TRY(cudaGetLastError());
     count_launch();
   }
-  gamma_dos_kernel<<<nprob, EW_THREADS, 0, st>>>(n, sig, sSig, gam, sGam, dos);
+  pdl_launch(gamma_dos_kernel, nprob, EW_THREADS, 0, st, n, sig, sSig, gam, sGam, dos);
   NEGF_CUDA_TRY(cudaGetLastError());
   count_launch();
   return NEGF_OK;
@@ -1065,7 +1088,7 @@ int sr_sigma(const HopBD& h, int n, int nprob, int lead, const double2* g, long 
 int density_spin(const DensityArgs& a, cudaStream_t st) {
   const int total = a.npx * a.npy * a.npz;
   dim3 grid((total + 255) / 256, a.batch);
-  density_spin_kernel<<<grid, 256, 0, st>>>(a);
+  pdl_launch(density_spin_kernel, grid, 256, 0, st, a);
   NEGF_CUDA_TRY(cudaGetLastError());
   count_launch();
   return NEGF_OK;
@@ -1074,7 +1097,7 @@ int density_spin(const DensityArgs& a, cudaStream_t st) {
 int reduce_sites(int batch, int nsite_total, int nf, int nslots, const Item* items, const double* site_out,
                  double* acc, cudaStream_t st) {
   const long long n = (long long)nf * nsite_total * nslots;
-  reduce_sites_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(batch, nsite_total, nf, nslots, items, site_out,
+  pdl_launch(reduce_sites_kernel, (unsigned)((n + 255) / 256), 256, 0, st, batch, nsite_total, nf, nslots, items, site_out,
                                                                    acc);
   NEGF_CUDA_TRY(cudaGetLastError());
   count_launch();
@@ -1091,6 +1114,7 @@ namespace negf {
 namespace {
 
 __global__ void to_f32_kernel(int n, const double2* src, long long sS, float2* dst, long long sD) {
+  pdl_wait();
   const int b = blockIdx.y;
   const long long nn = (long long)n * n;
   const double2* s = src + (long long)b * sS;
@@ -1102,6 +1126,7 @@ __global__ void to_f32_kernel(int n, const double2* src, long long sS, float2* d
 // one read of the matrix to invert: its FP64 copy (kept for the residual) and FP32 copy
 __global__ void split_copy_kernel(int n, const double2* src, long long sS, double2* d64, long long s64, float2* d32,
                                   long long s32) {
+  pdl_wait();
   const int b = blockIdx.y;
   const long long nn = (long long)n * n;
   const double2* s = src + (long long)b * sS;
@@ -1115,6 +1140,7 @@ __global__ void split_copy_kernel(int n, const double2* src, long long sS, doubl
 }
 
 __global__ void to_f64_kernel(int n, const float2* src, long long sS, double2* dst, long long sD) {
+  pdl_wait();
   const int b = blockIdx.y;
   const long long nn = (long long)n * n;
   const float2* s = src + (long long)b * sS;
@@ -1127,6 +1153,7 @@ __global__ void to_f64_kernel(int n, const float2* src, long long sS, double2* d
 // column k becomes column orig[k]
 __global__ void to_f64_columns_kernel(int n, const float2* src, long long sS, const int* orig, double2* dst,
                                       long long sD) {
+  pdl_wait();
   const int b = blockIdx.y;
   const long long nn = (long long)n * n;
   const float2* s = src + (long long)b * sS;
@@ -1157,6 +1184,7 @@ __device__ __forceinline__ float abs_to_float(double x) {
 }
 
 __global__ void ns_residual_kernel(int n, double2* T, long long sT, unsigned long long* rnorm) {
+  pdl_wait();
   __shared__ float part[8][32];
   const int b = blockIdx.y;
   const int tx = threadIdx.x, ty = threadIdx.y;
@@ -1188,7 +1216,7 @@ __global__ void ns_residual_kernel(int n, double2* T, long long sT, unsigned lon
 }  // namespace
 
 int to_f32(int n, int batch, const double2* src, long long sS, float2* dst, long long sD, cudaStream_t st) {
-  to_f32_kernel<<<ew_grid((long long)n * n, batch), EW_THREADS, 0, st>>>(n, src, sS, dst, sD);
+  pdl_launch(to_f32_kernel, ew_grid((long long)n * n, batch), EW_THREADS, 0, st, n, src, sS, dst, sD);
   NEGF_CUDA_TRY(cudaGetLastError());
   count_launch();
   return NEGF_OK;
@@ -1196,14 +1224,14 @@ int to_f32(int n, int batch, const double2* src, long long sS, float2* dst, long
 
 int split_copy(int n, int batch, const double2* src, long long sS, double2* d64, long long s64, float2* d32,
                long long s32, cudaStream_t st) {
-  split_copy_kernel<<<ew_grid((long long)n * n, batch), EW_THREADS, 0, st>>>(n, src, sS, d64, s64, d32, s32);
+  pdl_launch(split_copy_kernel, ew_grid((long long)n * n, batch), EW_THREADS, 0, st, n, src, sS, d64, s64, d32, s32);
   NEGF_CUDA_TRY(cudaGetLastError());
   count_launch();
   return NEGF_OK;
 }
 
 int to_f64(int n, int batch, const float2* src, long long sS, double2* dst, long long sD, cudaStream_t st) {
-  to_f64_kernel<<<ew_grid((long long)n * n, batch), EW_THREADS, 0, st>>>(n, src, sS, dst, sD);
+  pdl_launch(to_f64_kernel, ew_grid((long long)n * n, batch), EW_THREADS, 0, st, n, src, sS, dst, sD);
   NEGF_CUDA_TRY(cudaGetLastError());
   count_launch();
   return NEGF_OK;
@@ -1211,7 +1239,7 @@ int to_f64(int n, int batch, const float2* src, long long sS, double2* dst, long
 
 int to_f64_columns(int n, int batch, const float2* src, long long sS, const int* orig, double2* dst, long long sD,
                    cudaStream_t st) {
-  to_f64_columns_kernel<<<ew_grid((long long)n * n, batch), EW_THREADS, 0, st>>>(n, src, sS, orig, dst, sD);
+  pdl_launch(to_f64_columns_kernel, ew_grid((long long)n * n, batch), EW_THREADS, 0, st, n, src, sS, orig, dst, sD);
   NEGF_CUDA_TRY(cudaGetLastError());
   count_launch();
   return NEGF_OK;
@@ -1220,6 +1248,7 @@ int to_f64_columns(int n, int batch, const float2* src, long long sS, const int*
 namespace {
 __global__ void gather_strided_kernel(int n, const double2* src, long long sSrc, const int* idx, double2* dst,
                                       long long sDst, int scatter) {
+  pdl_wait();
   const int i = blockIdx.y;
   const long long nn = (long long)n * n;
   const double2* s_ = scatter ? src + (long long)i * sSrc : src + (long long)idx[i] * sSrc;
@@ -1232,7 +1261,7 @@ __global__ void gather_strided_kernel(int n, const double2* src, long long sSrc,
 int gather_strided(int n, int count, const double2* src, long long sSrc, const int* idx, double2* dst, long long sDst,
                    cudaStream_t st) {
   if (count <= 0) return NEGF_OK;
-  gather_strided_kernel<<<ew_grid((long long)n * n, count), EW_THREADS, 0, st>>>(n, src, sSrc, idx, dst, sDst, 0);
+  pdl_launch(gather_strided_kernel, ew_grid((long long)n * n, count), EW_THREADS, 0, st, n, src, sSrc, idx, dst, sDst, 0);
   NEGF_CUDA_TRY(cudaGetLastError());
   count_launch();
   return NEGF_OK;
@@ -1241,7 +1270,7 @@ int gather_strided(int n, int count, const double2* src, long long sSrc, const i
 int scatter_strided(int n, int count, const double2* src, long long sSrc, const int* idx, double2* dst,
                     long long sDst, cudaStream_t st) {
   if (count <= 0) return NEGF_OK;
-  gather_strided_kernel<<<ew_grid((long long)n * n, count), EW_THREADS, 0, st>>>(n, src, sSrc, idx, dst, sDst, 1);
+  pdl_launch(gather_strided_kernel, ew_grid((long long)n * n, count), EW_THREADS, 0, st, n, src, sSrc, idx, dst, sDst, 1);
   NEGF_CUDA_TRY(cudaGetLastError());
   count_launch();
   return NEGF_OK;
@@ -1250,7 +1279,7 @@ int scatter_strided(int n, int count, const double2* src, long long sSrc, const 
 
 int ns_residual(int n, int batch, double2* T, long long sT, unsigned long long* rnorm, cudaStream_t st) {
   dim3 grid((n + 31) / 32, batch);
-  ns_residual_kernel<<<grid, dim3(32, 8), 0, st>>>(n, T, sT, rnorm);
+  pdl_launch(ns_residual_kernel, grid, dim3(32, 8), 0, st, n, T, sT, rnorm);
   NEGF_CUDA_TRY(cudaGetLastError());
   count_launch();
   return NEGF_OK;

@@ -328,6 +328,7 @@ __device__ __forceinline__ int scale_exponent_strict(unsigned long long a) {
 // rows stride over the columns (coalesced 512-byte row segments), reduced in shared memory
 template <bool STRICT>
 __global__ void row_exp_kernel(const double2* A, int lda, long long sA, int m, int k, int* ea) {
+  pdl_wait();
   __shared__ unsigned long long part[8][32];
   const int b = blockIdx.y;
   const int tx = threadIdx.x, ty = threadIdx.y;
@@ -357,6 +358,7 @@ __global__ void row_exp_kernel(const double2* A, int lda, long long sA, int m, i
 template <int S>
 __global__ void __launch_bounds__(256) slice_a_kernel(const double2* A, int lda, long long sA, int m, int k,
                                                       const int* ea, __nv_bfloat16* out, int half) {
+  pdl_wait();
   __shared__ double2 tile[64][33];
   const int kp = 2 * half;
   const int b = blockIdx.z;
@@ -401,6 +403,7 @@ __global__ void __launch_bounds__(256) slice_a_kernel(const double2* A, int lda,
 template <int S>
 __global__ void __launch_bounds__(256) slice_b_kernel(const double2* B, int ldb, long long sB, int k, int n, int* fb,
                                                       __nv_bfloat16* out, int half) {
+  pdl_wait();
   __shared__ double2 chunk[8][256];
   const int kp = 2 * half;
   const int b = blockIdx.y;
@@ -617,6 +620,7 @@ __global__ void __launch_bounds__(TC_THREADS, MINB)
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  pdl_wait();
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
                  "r"((uint32_t)Cfg::TMEM_COLS));
@@ -829,6 +833,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  pdl_wait();
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
                  "r"(512u));
@@ -1025,7 +1030,7 @@ int launch_mma(const SlicedOperand& A, const SlicedOperand& B, const TcArgs& arg
   const double cflops = 8.0 * args.m * (double)args.n * (args.kp / 2) * args.batch;
   add_tc_complex_flops(cflops);
   timed_begin(st, TK_TC, cflops * (S * (S + 1) / 2), &ev);
-  zgemm_tc_kernel<S, NT, MINB, KS><<<grid, TC_THREADS, Cfg::SMEM, st>>>(ma, mb, args);
+  pdl_launch(zgemm_tc_kernel<S, NT, MINB, KS>, grid, TC_THREADS, Cfg::SMEM, st, ma, mb, args);
   NEGF_CUDA_TRY(cudaGetLastError());
   timed_end(st, TK_TC, ev);
   count_launch();
@@ -1057,7 +1062,7 @@ int launch_persistent(const SlicedOperand& A, const SlicedOperand& B, const TcAr
   const double cflops = 8.0 * args.m * (double)args.n * (args.kp / 2) * args.batch;
   add_tc_complex_flops(cflops);
   timed_begin(st, TK_TC, cflops * (S * (S + 1) / 2), &ev);
-  zgemm_tc_persistent<S, NT><<<grid, TC_THREADS, Cfg::SMEM, st>>>(ma, mb, args, tiles_m, tiles_n);
+  pdl_launch(zgemm_tc_persistent<S, NT>, grid, TC_THREADS, Cfg::SMEM, st, ma, mb, args, tiles_m, tiles_n);
   NEGF_CUDA_TRY(cudaGetLastError());
   timed_end(st, TK_TC, ev);
   count_launch();
@@ -1069,10 +1074,10 @@ int slice_a_t(const double2* A, int lda, long long sA, int m, int k, int batch, 
   cudaEvent_t ev;
   timed_begin(st, TK_SLICE, 0.0, &ev);
   dim3 g1((m + 31) / 32, batch);
-  row_exp_kernel<S == 9><<<g1, dim3(32, 8), 0, st>>>(A, lda, sA, m, k, out.exps);
+  pdl_launch(row_exp_kernel<S == 9>, g1, dim3(32, 8), 0, st, A, lda, sA, m, k, out.exps);
   NEGF_CUDA_TRY(cudaGetLastError());
   dim3 g2((m + 31) / 32, (out.k + 63) / 64, batch);
-  slice_a_kernel<S><<<g2, 256, 0, st>>>(A, lda, sA, m, k, out.exps, out.data, out.k);
+  pdl_launch(slice_a_kernel<S>, g2, 256, 0, st, A, lda, sA, m, k, out.exps, out.data, out.k);
   NEGF_CUDA_TRY(cudaGetLastError());
   timed_end(st, TK_SLICE, ev);
   count_launch(2);
@@ -1084,7 +1089,7 @@ int slice_b_t(const double2* B, int ldb, long long sB, int k, int n, int batch, 
   dim3 g((n + 7) / 8, batch);
   cudaEvent_t ev;
   timed_begin(st, TK_SLICE, 0.0, &ev);
-  slice_b_kernel<S><<<g, 256, 0, st>>>(B, ldb, sB, k, n, out.exps, out.data, out.k);
+  pdl_launch(slice_b_kernel<S>, g, 256, 0, st, B, ldb, sB, k, n, out.exps, out.data, out.k);
   NEGF_CUDA_TRY(cudaGetLastError());
   timed_end(st, TK_SLICE, ev);
   count_launch();
