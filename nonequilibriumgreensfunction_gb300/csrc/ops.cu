@@ -325,8 +325,11 @@ __global__ void hop_rows_kernel(HopRows r, int n, int left, const double2* X, lo
 
 // ---- site blocks of X Gamma X^H ------------------------------------------------------
 // P[r][a] = sum_k Y(r,k) conj(X(site(r)*no + a, k)); one thread per row r, the k loop is
-// split over KSPLIT groups of threads and reduced in shared memory (fixed order).
-constexpr int SB_ROWS = 64, SB_KSPLIT = 4;
+// split over KSPLIT groups of threads and reduced in shared memory (fixed order).  FP64 pipe
+// bound where the batch fills the device; 16 rows a CTA spread a small batch over more SMs than
+// 64 rows did: n = 400, 4 items 126 -> 39 us; n = 144, 32 items 45 -> 25 us; n = 400, 32 items
+// 210 -> 166 us.
+constexpr int SB_ROWS = 16, SB_KSPLIT = 16;
 // NOM bounds the orbitals per site (4, or 8 for the BdG form); no <= NOM
 template <int NOM>
 __global__ void __launch_bounds__(SB_ROWS* SB_KSPLIT) site_blocks_kernel(int n, int no, const double2* Y, long long sY,
@@ -417,23 +420,24 @@ __global__ void __launch_bounds__(SB_ROWS* SB_KSPLIT) site_pairs_kernel(int n, i
 }
 
 // ---- Re sum Q .* conj(X) (one CTA per item, fixed reduction order) -------------------
-__global__ void trace_dot_kernel(int n, const double2* Q, long long sQ, const double2* X, long long sX, double* out,
+constexpr int RED_THREADS = 1024;   // one CTA reduces an item's block: as many loads in flight as it can have
+__global__ void __launch_bounds__(RED_THREADS) trace_dot_kernel(int n, const double2* Q, long long sQ, const double2* X, long long sX, double* out,
                                  int out_stride) {
   pdl_wait();
-  __shared__ double red[EW_THREADS];
+  __shared__ double red[RED_THREADS];
   const int b = blockIdx.x;
   const long long nn = (long long)n * n;
   const double2* Qb = Q + (long long)b * sQ;
   const double2* Xb = X + (long long)b * sX;
   double s = 0.0;
-  for (long long e = threadIdx.x; e < nn; e += EW_THREADS) {
+  for (long long e = threadIdx.x; e < nn; e += RED_THREADS) {
     const double2 q = Qb[e], x = Xb[e];
     s = fma(q.x, x.x, s);
     s = fma(q.y, x.y, s);
   }
   red[threadIdx.x] = s;
   __syncthreads();
-  for (int w = EW_THREADS / 2; w > 0; w >>= 1) {
+  for (int w = RED_THREADS / 2; w > 0; w >>= 1) {
     if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
     __syncthreads();
   }
@@ -566,14 +570,14 @@ __global__ void sr_sigma_kernel(HopBD h, int n, int lead, const double2* g, long
   }
 }
 
-__global__ void gamma_dos_kernel(int n, const double2* sig, long long sS, double2* gam, long long sG, double* dos) {
+__global__ void __launch_bounds__(RED_THREADS) gamma_dos_kernel(int n, const double2* sig, long long sS, double2* gam, long long sG, double* dos) {
   pdl_wait();
-  __shared__ double red[EW_THREADS];
+  __shared__ double red[RED_THREADS];
   const int b = blockIdx.x;
   const long long nn = (long long)n * n;
   const double2* Sb = sig + (long long)b * sS;
   double2* Gb = gam + (long long)b * sG;
-  for (long long e = threadIdx.x; e < nn; e += EW_THREADS) {
+  for (long long e = threadIdx.x; e < nn; e += RED_THREADS) {
     const int i = (int)(e % n), j = (int)(e / n);
     const double2 s = Sb[e], st = Sb[(long long)i * n + j];
     // i (S - S^H): S^H(i,j) = conj(S(j,i))
@@ -581,10 +585,10 @@ __global__ void gamma_dos_kernel(int n, const double2* sig, long long sS, double
     Gb[e] = make_double2(-d.y, d.x);
   }
   double s = 0.0;
-  for (int i = threadIdx.x; i < n; i += EW_THREADS) s += Sb[(long long)i * n + i].y;
+  for (int i = threadIdx.x; i < n; i += RED_THREADS) s += Sb[(long long)i * n + i].y;
   red[threadIdx.x] = s;
   __syncthreads();
-  for (int w = EW_THREADS / 2; w > 0; w >>= 1) {
+  for (int w = RED_THREADS / 2; w > 0; w >>= 1) {
     if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
     __syncthreads();
   }
@@ -1016,7 +1020,7 @@ int josephson(int n, int no, int batch, const Item* items, const double2* P1, co
 
 int trace_dot(int n, int batch, const double2* Q, long long sQ, const double2* X, long long sX, double* out,
               int out_stride, cudaStream_t st) {
-  pdl_launch(trace_dot_kernel, batch, EW_THREADS, 0, st, n, Q, sQ, X, sX, out, out_stride);
+  pdl_launch(trace_dot_kernel, batch, RED_THREADS, 0, st, n, Q, sQ, X, sX, out, out_stride);
   NEGF_CUDA_TRY(cudaGetLastError());
   count_launch();
   return NEGF_OK;
@@ -1079,7 +1083,7 @@ int sr_sigma(const HopBD& h, int n, int nprob, int lead, const double2* g, long 
     NEGF_CUDA_TRY(cudaGetLastError());
     count_launch();
   }
-  pdl_launch(gamma_dos_kernel, nprob, EW_THREADS, 0, st, n, sig, sSig, gam, sGam, dos);
+  pdl_launch(gamma_dos_kernel, nprob, RED_THREADS, 0, st, n, sig, sSig, gam, sGam, dos);
   NEGF_CUDA_TRY(cudaGetLastError());
   count_launch();
   return NEGF_OK;
