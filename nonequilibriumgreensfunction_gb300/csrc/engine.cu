@@ -710,7 +710,7 @@ int Engine::invert_refined(double2* A, long long sA, int batch, int* status_dev,
     for (int i = 0; i < nb; ++i)
       NEGF_CUDA_TRY(cudaMemcpyAsync(dT_ + (long long)i * MM_, dWinv_ + (long long)bad[i] * MM_,
                                     sizeof(double2) * MM_, cudaMemcpyDeviceToDevice, st_));
-    NEGF_TRY(zinv_f64(dT_, MM_, M_, nb, inv_, st_));
+    NEGF_TRY(zinv_f64(dT_, MM_, M_, nb, inv_, st_, mixed_));
     for (int i = 0; i < nb; ++i) {
       NEGF_CUDA_TRY(cudaMemcpyAsync(A + (long long)bad[i] * sA, dT_ + (long long)i * MM_, sizeof(double2) * MM_,
                                     cudaMemcpyDeviceToDevice, st_));

@@ -6,7 +6,7 @@
 // factorisation is ONE rank-nb update of the whole matrix (a GEMM), with no triangular
 // solves, which keeps the FP64 pipe of all SMs busy across a batch of matrices.
 //
-// Per panel K = [k0, k0+nb):
+// Per panel K = [k0, k0+nb), nb = 8 in FP64 up to n = 1024 and 32 otherwise:
 //   1. gj_panel:   one CTA per matrix factorises the n x nb panel in shared memory
 //                  (pivot = first max of |re|+|im| over rows >= k, as LAPACK izamax).
 //   2. gj_swap:    applies the panel's row interchanges to the other columns, copies
@@ -176,7 +176,8 @@ __global__ void __launch_bounds__(PANEL_THREADS) gj_panel_kernel(T* A, long long
 // Bound: issue slots, 128 FMA per row and step, and the latency of the pivot chain (two
 // barriers, one reciprocal).  Pivots, their ties (lowest position) and every element's
 // operations are those of panel_factor, so the panel is bitwise the same.
-// Measured on GB300 (panel alone, 32 matrices): MEASURE_PANEL
+// Measured on GB300 (panel alone, 32 matrices), panel_factor against this: n = 144 51 / 23 us, 400
+// 72 / 33 us, 576 96 / 44 us.
 constexpr int RP_MAX_N = 640;   // 640 threads of up to 102 registers
 constexpr int RP_C = 32;
 template <int MAXT>   // threads at most: 512 (128 registers each) or RP_MAX_N (96)
@@ -294,6 +295,153 @@ __global__ void __launch_bounds__(MAXT, 1) gj_panel_reg_kernel(float2* A, long l
   }
   __syncthreads();
   if (t == 0) mv[0] = s_extra;
+}
+
+// The FP64 inverse (n <= 1024; not the mixed form's redone ones, see zinv_f64) with panels of
+// eight columns.  A panel is one SM's work, 4 n nb^2
+// multiply-adds on a pipe of two per clock: with 32 columns and a few matrices the panels were
+// most of the time while the other SMs waited, and with many they were the longest part of a
+// wave.  The rank-8 updates are split into enough tiles for every SM.  The panel has its rows in
+// registers as the FP32 one above: a thread a row, a step on register column 0, two barriers a
+// step, the interchanges as moves.
+// Whole INVERT calls with the copies on GB300, 32-column panels against these: n = 144, 1 matrix
+// 2.76 / 0.92 ms, 304 matrices 13.1 / 9.3 ms; n = 400, 1 10.9 / 3.7 ms, 200 114 / 103 ms;
+// n = 784, 1 21.1 / 12.4 ms; n = 1000, 16 149 / 129 ms.
+constexpr int NP_C = 8, NP_MAX_N = 1024;
+__global__ void __launch_bounds__(NP_MAX_N, 1) gj_panel_narrow_kernel(double2* A, long long sA, int n, int k0, int kb,
+                                                                      int* ipiv, int* info, int* moves) {
+  pdl_wait();
+  __shared__ double2 raw[NP_C], piv[NP_C];   // pivot row, unscaled and scaled
+  __shared__ unsigned long long w_key[NP_MAX_N / 32];
+  __shared__ int w_pos[NP_MAX_N / 32];
+  __shared__ int s_extra;
+  const int b = blockIdx.x;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5, nwarps = blockDim.x >> 5;
+  double2* Ab = A + (long long)b * sA;
+  int* ip = ipiv + (long long)b * n;
+  const bool live = t < n;
+  double2 row[NP_C];
+#pragma unroll
+  for (int j = 0; j < NP_C; ++j)
+    row[j] = (live && j < kb) ? Ab[(long long)(k0 + j) * n + t] : make_double2(0.0, 0.0);
+  int pos = live ? t : 0x7fffffff;
+  if (t == 0) s_extra = kb;
+  auto rotate = [&]() {
+    const double2 first = row[0];
+#pragma unroll
+    for (int j = 0; j < NP_C - 1; ++j) row[j] = row[j + 1];
+    row[NP_C - 1] = first;
+  };
+  // largest key of a warp and the lowest position that has it (keys: bits of |re| + |im| plus
+  // one, which order as the values; 0 = no candidate)
+  auto best_of = [&](unsigned long long key, int at, unsigned long long& best) -> int {
+    const unsigned hi = __reduce_max_sync(0xffffffffu, (unsigned)(key >> 32));
+    const unsigned lo = __reduce_max_sync(0xffffffffu, (unsigned)(key >> 32) == hi ? (unsigned)key : 0u);
+    best = ((unsigned long long)hi << 32) | lo;
+    return __reduce_min_sync(0xffffffffu, key == best ? at : 0x7fffffff);
+  };
+#pragma unroll 1
+  for (int c = 0; c < kb; ++c) {
+    const int r = k0 + c;
+    const double a = cabs1(row[0]);
+    unsigned long long best;
+    const int wpos = best_of(
+        (live && pos >= r && a == a) ? (unsigned long long)__double_as_longlong(a) + 1ULL : 0ULL, pos, best);
+    if (lane == 0) { w_key[warp] = best; w_pos[warp] = wpos; }
+    __syncthreads();
+    int p = best_of(lane < nwarps ? w_key[lane] : 0ULL, lane < nwarps ? w_pos[lane] : 0x7fffffff, best);
+    if (best == 0ULL) p = r;
+    const bool own = pos == p;
+    if (__any_sync(0xffffffffu, own)) {
+      if (own) {
+#pragma unroll
+        for (int j = 0; j < NP_C; ++j) raw[j] = row[j];
+        ip[r] = p;
+        if (row[0].x == 0.0 && row[0].y == 0.0 && info[b] == 0) info[b] = r + 1;
+      }
+      __syncwarp();
+      const double2 pv = raw[0];
+      if (lane < NP_C) {
+        const double2 d = (pv.x == 0.0 && pv.y == 0.0) ? pv : crcp(pv);
+        piv[lane] = lane == 0 ? d : cmul(raw[lane], d);
+      }
+    }
+    __syncthreads();
+    if (own) pos = r;
+    else if (pos == r) pos = p;
+    const double2 d = piv[0];
+    if (d.x == 0.0 && d.y == 0.0) {   // no pivot: the interchange only
+      rotate();
+      continue;
+    }
+    const double2 f = row[0];
+    if (own) {
+#pragma unroll
+      for (int j = 1; j < NP_C; ++j) row[j - 1] = piv[j];
+      row[NP_C - 1] = d;
+    } else {
+#pragma unroll
+      for (int j = 1; j < NP_C; ++j) {
+        const double2 rv = piv[j];
+        double2 v = row[j];
+        v.x = fma(-f.x, rv.x, v.x);
+        v.x = fma(f.y, rv.y, v.x);
+        v.y = fma(-f.x, rv.y, v.y);
+        v.y = fma(-f.y, rv.x, v.y);
+        row[j - 1] = v;
+      }
+      row[NP_C - 1] = cmul(make_double2(-f.x, -f.y), d);
+    }
+  }
+#pragma unroll 1
+  for (int c = kb; c < NP_C; ++c) rotate();
+  int* mv = moves + (long long)b * GJ_MOVES;
+  if (live) {
+#pragma unroll
+    for (int j = 0; j < NP_C; ++j)
+      if (j < kb) Ab[(long long)(k0 + j) * n + pos] = row[j];
+    const int q = (pos >= k0 && pos < k0 + kb) ? pos - k0 : (pos != t ? atomicAdd(&s_extra, 1) : -1);
+    if (q >= 0) {
+      mv[1 + 2 * q] = pos;
+      mv[2 + 2 * q] = t;
+    }
+  }
+  __syncthreads();
+  if (t == 0) mv[0] = s_extra;
+}
+
+// A(:, j) += P R(:, j) for the columns outside the panel, kb <= KB: tiles of 32 rows x 16
+// columns, two outputs a thread, each formed by gj_update_kernel's operations.  One matrix of
+// n = 144 is 45 tiles, where gj_update_kernel's 80 x 80 tiles are four; n = 576, K = 32, the few
+// matrices of a redone inverse: 107 -> 53 us.
+constexpr int NU_M = 32, NU_N = 16;
+template <int KB>
+__global__ void __launch_bounds__(256) gj_update_tiles_kernel(double2* A, long long sA, int n, int k0, int kb,
+                                                              const double2* R, long long sR) {
+  pdl_wait();
+  __shared__ double2 Ps[KB][NU_M], Rs[KB][NU_N + 1];
+  const int b = blockIdx.z, t = threadIdx.x;
+  const int m0 = blockIdx.x * NU_M, n0 = blockIdx.y * NU_N;
+  double2* Ab = A + (long long)b * sA;
+  const double2* Rb = R + (long long)b * sR;
+  for (int e = t; e < kb * NU_M; e += 256) {
+    const int k = e / NU_M, i = m0 + e % NU_M;
+    Ps[k][e % NU_M] = i < n ? Ab[(long long)(k0 + k) * n + i] : make_double2(0.0, 0.0);
+  }
+  for (int e = t; e < kb * NU_N; e += 256) {
+    const int j = n0 + e / kb;
+    Rs[e % kb][e / kb] = j < n ? Rb[(long long)j * kb + e % kb] : make_double2(0.0, 0.0);
+  }
+  __syncthreads();
+  const int i = t % NU_M, row = m0 + i;
+  for (int jj = t / NU_M; jj < NU_N; jj += 256 / NU_M) {
+    const int col = n0 + jj;
+    if (row >= n || col >= n || (col >= k0 && col < k0 + kb)) continue;
+    double2 s = make_double2(0.0, 0.0);
+    for (int k = 0; k < kb; ++k) cfma(s, Ps[k][i], Rs[k][jj]);
+    double2* c = Ab + (long long)col * n + row;
+    *c = cadd(s, *c);
+  }
 }
 
 // Row interchanges of one panel for the columns outside it, and the copy of rows K into R.
@@ -824,8 +972,12 @@ int gj_invert(T* A, long long sA, int n, int batch, InvWork& w, cudaStream_t st)
                                                              reinterpret_cast<const float2*>(rbuf), sR, nt, nt,
                                                              ntiles);
       } else {
-        dim3 gu(nt, nt, batch);
-        pdl_launch(gj_update_kernel<T>, gu, 256, upd_smem, st, A, sA, n, k0, kb, rbuf, sR);
+        // 80 x 80 tiles where they fill the device twice over, smaller ones for a few matrices
+        if ((long long)nt * nt * batch < 2LL * sm_count_cached())
+          pdl_launch(gj_update_tiles_kernel<32>, dim3((n + NU_M - 1) / NU_M, (n + NU_N - 1) / NU_N, batch), 256, 0, st, A,
+                     sA, n, k0, kb, rbuf, sR);
+        else
+          pdl_launch(gj_update_kernel<T>, dim3(nt, nt, batch), 256, upd_smem, st, A, sA, n, k0, kb, rbuf, sR);
       }
       NEGF_CUDA_TRY(cudaGetLastError());
       timed_end(st, sizeof(T) == 8 ? TK_F32 : TK_GEMM, eu);
@@ -843,7 +995,40 @@ int gj_invert(T* A, long long sA, int n, int batch, InvWork& w, cudaStream_t st)
 
 }  // namespace
 
-int zinv_f64(double2* A, long long sA, int n, int batch, InvWork& w, cudaStream_t st) {
+namespace {
+
+// n <= NP_MAX_N: panels of NP_C columns
+int gj_invert_narrow(double2* A, long long sA, int n, int batch, InvWork& w, cudaStream_t st) {
+  NEGF_CUDA_TRY(cudaMemsetAsync(w.info, 0, sizeof(int) * batch, st));
+  const long long sR = (long long)NP_C * n;
+  for (int k0 = 0; k0 < n; k0 += NP_C) {
+    const int kb = std::min(NP_C, n - k0);
+    cudaEvent_t ev;
+    timed_begin(st, TK_PANEL, 8.0 * n * (double)kb * kb * batch, &ev);
+    pdl_launch(gj_panel_narrow_kernel, batch, (n + 31) / 32 * 32, 0, st, A, sA, n, k0, kb, w.ipiv, w.info, w.moves);
+    NEGF_CUDA_TRY(cudaGetLastError());
+    timed_end(st, TK_PANEL, ev);
+    pdl_launch(gj_swap_kernel<double2>, dim3((n + SWAP_WARPS - 1) / SWAP_WARPS, batch), SWAP_WARPS * 32, 0, st, A, sA,
+               n, k0, kb, w.ipiv, w.moves, w.rbuf, sR);
+    NEGF_CUDA_TRY(cudaGetLastError());
+    timed_begin(st, TK_GEMM, 8.0 * n * (double)(n - kb) * kb * batch, &ev);
+    pdl_launch(gj_update_tiles_kernel<NP_C>, dim3((n + NU_M - 1) / NU_M, (n + NU_N - 1) / NU_N, batch), 256, 0, st, A, sA, n,
+               k0, kb, w.rbuf, sR);
+    NEGF_CUDA_TRY(cudaGetLastError());
+    timed_end(st, TK_GEMM, ev);
+    count_launch(3);
+  }
+  pdl_launch(gj_colswap_kernel<double2>, dim3((n + 127) / 128, batch), 128, 0, st, A, sA, n, w.ipiv);
+  NEGF_CUDA_TRY(cudaGetLastError());
+  count_launch();
+  return NEGF_OK;
+}
+
+}  // namespace
+
+int zinv_f64(double2* A, long long sA, int n, int batch, InvWork& w, cudaStream_t st, bool wide) {
+  if (!wide && n > 0 && n <= NP_MAX_N && batch > 0 && batch <= 65535 && n <= w.n_cap && batch <= w.batch_cap && NP_C <= w.nb)
+    return gj_invert_narrow(A, sA, n, batch, w, st);
   return gj_invert<double2>(A, sA, n, batch, w, st);
 }
 

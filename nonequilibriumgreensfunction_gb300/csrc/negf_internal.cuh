@@ -191,7 +191,9 @@ void inv_work_free(InvWork& w, cudaStream_t st = 0);
 int panel_width(int n, int elem_bytes = 16);
 // A: batch matrices of n x n, column-major, consecutive at stride sA.  On return A holds
 // the inverses; w.info[b] (device) holds the LAPACK-style INFO of each matrix.
-int zinv_f64(double2* A, long long sA, int n, int batch, InvWork& w, cudaStream_t st);
+// wide: 32-column panels whatever the size, which round differently.  The mixed form redoes its
+// worst-conditioned decimation blocks in FP64, and its results at small eta follow their last bits.
+int zinv_f64(double2* A, long long sA, int n, int batch, InvWork& w, cudaStream_t st, bool wide = false);
 // FP32 twin (the first guess of the mixed-form inverse).  form 0: panel / interchange /
 // update launches per 32-column panel; form 1: one fused launch with a CTA per matrix (needs
 // cinv_f32_fused_ok).  Both give bitwise the same result, form 0 perhaps with its columns still

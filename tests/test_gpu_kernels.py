@@ -2,7 +2,7 @@
 import numpy as np
 import pytest
 
-from nonequilibriumgreensfunction_gb300 import Solver, hamiltonian, scf
+from nonequilibriumgreensfunction_gb300 import Solver, capi, hamiltonian, scf
 from oracle import negf_oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -117,3 +117,18 @@ def test_small_cross_sections_in_every_cluster(need_gpu, channel, npy, npz):
     assert abs(r["T12"][0] - t12) <= 1e-9 * max(abs(t12), 1e-3)
     assert abs(r["DOSc1"][0] - cse["dosc"][0]) <= 1e-9 * abs(cse["dosc"][0])
     assert np.abs(rho[..., 0] - want).max() <= 1e-9 * np.abs(want).max()
+
+
+# The FP64 inverse has panels of eight columns up to n = 1024 (the last of 1, 7 or 8) and wider
+# ones beyond.  Tolerance: 100 n eps of the product of the norms; a zero column gives its INFO.
+@pytest.mark.parametrize("n", [1, 7, 8, 9, 33, 1024, 1025])
+def test_fp64_inverse_at_its_panel_sizes(need_gpu, n):
+    rng = np.random.default_rng(n)
+    a = rng.standard_normal((2, n, n)) + 1j * rng.standard_normal((2, n, n))
+    x, info = capi.zinv(a)
+    assert info == 0
+    for m, i in zip(a, x):
+        bound = 100 * n * np.finfo(float).eps * np.linalg.norm(m, 2) * np.linalg.norm(i, 2)
+        assert np.abs(m @ i - np.eye(n)).max() <= bound
+    a[1, :, n - 1] = 0.0
+    assert capi.zinv(a)[1] == n
