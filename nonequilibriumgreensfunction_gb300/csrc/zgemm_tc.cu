@@ -324,75 +324,87 @@ __device__ __forceinline__ int scale_exponent_strict(unsigned long long a) {
   return (E == 0x7FF || E < 200) ? EXP_DIRECT : E - 1022;
 }
 
-// row exponents of A (M x K complex, column-major): a CTA covers 32 rows, its 8 thread
-// rows stride over the columns (coalesced 512-byte row segments), reduced in shared memory
-template <bool STRICT>
-__global__ void row_exp_kernel(const double2* A, int lda, long long sA, int m, int k, int* ea) {
-  pdl_wait();
-  __shared__ unsigned long long part[8][32];
-  const int b = blockIdx.y;
-  const int tx = threadIdx.x, ty = threadIdx.y;
-  const int i = blockIdx.x * 32 + tx;
-  const double2* Ab = A + (long long)b * sA;
-  unsigned long long mx = 0;
-  if (i < m)
-    for (int kk = ty; kk < k; kk += 8) {
-      const double2 v = Ab[(long long)kk * lda + i];
-      if (STRICT) mx = max(mx, max(abs_bits_all(v.x), abs_bits_all(v.y)));
-      else mx = max(mx, max(abs_bits(v.x), abs_bits(v.y)));
-    }
-  part[ty][tx] = mx;
-  __syncthreads();
-  if (ty == 0 && i < m) {
-    for (int q = 1; q < 8; ++q) mx = max(mx, part[q][tx]);
-    ea[(long long)b * m + i] = STRICT ? scale_exponent_strict(mx) : scale_exponent(mx);
-  }
-}
-
 // A slices, K-major, two real rows per complex row i (kp = 2*half):
 //     out[((b*S + p)*2m + 2i)*kp + k]   = [Ar(i, :), -Ai(i, :)]
 //     out[((b*S + p)*2m + 2i+1)*kp + k] = [Ai(i, :),  Ar(i, :)],
-// zero in the padding k in [K, half).  A tile of 32 rows x 64 k is staged through shared
-// memory (coalesced column-major reads); each thread then slices one row x 8 consecutive
-// k and writes 16-byte vectors.
+// zero in the padding k in [K, half).  A CTA takes 8 rows, so that a column's piece is one 128-byte
+// line: it reads them once into shared memory, finds their exponents on the way, and slices from
+// there, 8 consecutive k of a row per thread, written as 16-byte vectors with 8 threads to a line.
+// Bound: memory, 16 bytes read and 8 S written an element (n = 400, 58 items: 8.2 to 8.7 TB/s, L2
+// included).  It replaces a kernel for the exponents and one for the slices, each of which read A:
+// 57 -> 45 us at three slices, 71 -> 60 at five, 87 -> 63 at seven; n = 320, 8 items, nine 35 -> 23.
+constexpr int SA_ROWS = 8;
+// where element (kk, row) is kept: eight threads that read two rows' groups of 8 kk apart meet in no bank
+__device__ __forceinline__ int sa_at(int kk, int row) { return kk * SA_ROWS + (row ^ ((kk >> 1) & 4)); }
 template <int S>
-__global__ void __launch_bounds__(256) slice_a_kernel(const double2* A, int lda, long long sA, int m, int k,
-                                                      const int* ea, __nv_bfloat16* out, int half) {
+__global__ void __launch_bounds__(256, S <= 5 ? 4 : S <= 8 ? 3 : 2)
+    slice_a_kernel(const double2* A, int lda, long long sA, int m, int k, int* ea, __nv_bfloat16* out, int half) {
   pdl_wait();
-  __shared__ double2 tile[64][33];
+  extern __shared__ __align__(16) double2 sa_rows[];   // [half][SA_ROWS]
+  __shared__ unsigned long long part[8][SA_ROWS];
+  constexpr bool STRICT = S == 9;
   const int kp = 2 * half;
-  const int b = blockIdx.z;
-  const int i0 = blockIdx.x * 32, k0 = blockIdx.y * 64;
-  const double2* Ab = A + (long long)b * sA;
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;   // 32 x 8
+  const int b = blockIdx.y;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int i0 = blockIdx.x * SA_ROWS;
+  {
+    const int row = threadIdx.x % SA_ROWS, g = threadIdx.x / SA_ROWS;
+    const double2* Ai = A + (long long)b * sA + i0 + row;
+    const bool live = i0 + row < m;
+    unsigned long long mx = 0;
+    constexpr int U = 4, STEP = 256 / SA_ROWS;   // U loads of a thread in flight
+    for (int kk = g; kk < half; kk += U * STEP) {
+      double2 v[U];
 #pragma unroll
-  for (int r = 0; r < 8; ++r) {
-    const int kk = k0 + ty + 8 * r, i = i0 + tx;
-    tile[ty + 8 * r][tx] = (i < m && kk < k) ? Ab[(long long)kk * lda + i] : make_double2(0.0, 0.0);
+      for (int u = 0; u < U; ++u)
+        v[u] = live && kk + u * STEP < k ? Ai[(long long)(kk + u * STEP) * lda] : make_double2(0.0, 0.0);
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        if (STRICT) mx = max(mx, max(abs_bits_all(v[u].x), abs_bits_all(v[u].y)));
+        else mx = max(mx, max(abs_bits(v[u].x), abs_bits(v[u].y)));
+        if (kk + u * STEP < half) sa_rows[sa_at(kk + u * STEP, row)] = v[u];
+      }
+    }
+    mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
+    mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 16));
+    if (lane < SA_ROWS) part[warp][lane] = mx;
   }
   __syncthreads();
-  const int row = threadIdx.x >> 3, kg = threadIdx.x & 7;
-  const int i = i0 + row, kb = k0 + 8 * kg;
-  if (i >= m || kb >= half) return;
-  const int e = ea[(long long)b * m + i];
-  __align__(16) __nv_bfloat16 sr[S][8], si[S][8], ni[S][8];
+  // a warp slices four rows, 64 k
+  const int row = 4 * (warp & 1) + (lane >> 3);
+  const int i = i0 + row;
+  if (i >= m) return;
+  unsigned long long mx = 0;
 #pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    const double2 v = tile[8 * kg + q][row];
-    __nv_bfloat16 a[S], c[S];
-    slice_value<S>(v.x, e, a);
-    slice_value<S>(v.y, e, c);
+  for (int w = 0; w < 8; ++w) mx = max(mx, part[w][row]);
+  const int e = STRICT ? scale_exponent_strict(mx) : scale_exponent(mx);
+  if (warp < 2 && (lane & 7) == 0) ea[(long long)b * m + i] = e;
+#pragma unroll 1
+  for (int kb = 8 * (lane & 7) + 64 * (warp >> 1); kb < half; kb += 256) {
+    // The real parts, then the imaginary ones: half the registers, so two to four CTAs an SM, some
+    // of which load while others slice (both parts at once: 70 us at five slices, 108 at seven).
+#pragma unroll 1
+    for (int im = 0; im < 2; ++im) {
+      __align__(16) __nv_bfloat16 sl[S][8];
 #pragma unroll
-    for (int p = 0; p < S; ++p) { sr[p][q] = a[p]; si[p][q] = c[p]; ni[p][q] = __hneg(c[p]); }
-  }
+      for (int q = 0; q < 8; ++q) {
+        const double2* v = &sa_rows[sa_at(kb + q, row)];
+        __nv_bfloat16 a[S];
+        slice_value<S>(im ? v->y : v->x, e, a);
 #pragma unroll
-  for (int p = 0; p < S; ++p) {
-    __nv_bfloat16* re_row = out + ((long long)(b * S + p) * 2 * m + 2 * i) * kp;
-    __nv_bfloat16* im_row = re_row + kp;
-    *reinterpret_cast<uint4*>(re_row + kb) = *reinterpret_cast<const uint4*>(sr[p]);
-    *reinterpret_cast<uint4*>(re_row + half + kb) = *reinterpret_cast<const uint4*>(ni[p]);
-    *reinterpret_cast<uint4*>(im_row + kb) = *reinterpret_cast<const uint4*>(si[p]);
-    *reinterpret_cast<uint4*>(im_row + half + kb) = *reinterpret_cast<const uint4*>(sr[p]);
+        for (int p = 0; p < S; ++p) sl[p][q] = a[p];
+      }
+#pragma unroll
+      for (int p = 0; p < S; ++p) {
+        uint4 v = *reinterpret_cast<const uint4*>(sl[p]);
+        __nv_bfloat16* re_row = out + ((long long)(b * S + p) * 2 * m + 2 * i) * kp;
+        __nv_bfloat16* im_row = re_row + kp;
+        *reinterpret_cast<uint4*>(im_row + (im ? 0 : half) + kb) = v;
+        constexpr unsigned neg = 0x80008000u;   // the sign bits of two BF16 values
+        if (im) v = make_uint4(v.x ^ neg, v.y ^ neg, v.z ^ neg, v.w ^ neg);
+        *reinterpret_cast<uint4*>(re_row + (im ? half : 0) + kb) = v;
+      }
+    }
   }
 }
 
@@ -426,7 +438,7 @@ __global__ void __launch_bounds__(256) slice_b_kernel(const double2* B, int ldb,
 #pragma unroll
     for (int q = 0; q < 8; ++q) {
       const int kk = c0 + lane + 32 * q;
-      ch[lane + 32 * q] = kk < k ? col[kk] : make_double2(0.0, 0.0);
+      ch[(lane + 32 * q) ^ (((lane + 32 * q) >> 3) & 7)] = kk < k ? col[kk] : make_double2(0.0, 0.0);
     }
     __syncwarp();
     const int kb = c0 + 8 * lane;
@@ -434,7 +446,7 @@ __global__ void __launch_bounds__(256) slice_b_kernel(const double2* B, int ldb,
       __align__(16) __nv_bfloat16 rr[S][8], ri[S][8];
 #pragma unroll
       for (int q = 0; q < 8; ++q) {
-        const double2 v = ch[8 * lane + q];
+        const double2 v = ch[8 * lane + (q ^ (lane & 7))];   // the exchanged places keep the lanes in different banks
         __nv_bfloat16 a[S], c[S];
         slice_value<S>(v.x, e, a);
         slice_value<S>(v.y, e, c);
@@ -1071,16 +1083,17 @@ int launch_persistent(const SlicedOperand& A, const SlicedOperand& B, const TcAr
 
 template <int S>
 int slice_a_t(const double2* A, int lda, long long sA, int m, int k, int batch, SlicedOperand& out, cudaStream_t st) {
+  if (2 * out.k > 1600) return NEGF_EINVAL;   // as the products; a CTA's rows fit its shared memory
+  const size_t smem = (size_t)SA_ROWS * out.k * sizeof(double2);
+  if (smem > 48 * 1024)
+    NEGF_CUDA_TRY(cudaFuncSetAttribute(slice_a_kernel<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   cudaEvent_t ev;
   timed_begin(st, TK_SLICE, 0.0, &ev);
-  dim3 g1((m + 31) / 32, batch);
-  pdl_launch(row_exp_kernel<S == 9>, g1, dim3(32, 8), 0, st, A, lda, sA, m, k, out.exps);
-  NEGF_CUDA_TRY(cudaGetLastError());
-  dim3 g2((m + 31) / 32, (out.k + 63) / 64, batch);
-  pdl_launch(slice_a_kernel<S>, g2, 256, 0, st, A, lda, sA, m, k, out.exps, out.data, out.k);
+  pdl_launch(slice_a_kernel<S>, dim3((m + SA_ROWS - 1) / SA_ROWS, batch), 256, smem, st, A, lda, sA, m, k, out.exps,
+             out.data, out.k);
   NEGF_CUDA_TRY(cudaGetLastError());
   timed_end(st, TK_SLICE, ev);
-  count_launch(2);
+  count_launch();
   return NEGF_OK;
 }
 

@@ -132,3 +132,19 @@ def test_fp64_inverse_at_its_panel_sizes(need_gpu, n):
         assert np.abs(m @ i - np.eye(n)).max() <= bound
     a[1, :, n - 1] = 0.0
     assert capi.zinv(a)[1] == n
+
+
+# The A side is sliced eight rows a block, 64 k a warp, its rows staged in shared memory (up to
+# k = 800).  Tolerance: 8 k eps of the product of moduli (NumPy's own rounding), and for the slice
+# pairs left out 8 S 2^(-7 S) k of a row's and a column's largest; row scales spread over 2^40.
+@pytest.mark.parametrize("slices", [3, 5, 7, 8])
+@pytest.mark.parametrize("m,k", [(1, 1), (7, 16), (8, 63), (9, 65), (33, 257), (17, 800)])
+def test_sliced_rows_at_their_block_sizes(need_gpu, m, k, slices):
+    rng = np.random.default_rng(m * k)
+    a = rng.standard_normal((2, m, k)) + 1j * rng.standard_normal((2, m, k))
+    a *= np.ldexp(1.0, rng.integers(-20, 20, (2, m, 1)))
+    b = rng.standard_normal((2, k, 11)) + 1j * rng.standard_normal((2, k, 11))
+    got = capi.zgemm(a, b, slices=slices)
+    bound = 8 * k * np.finfo(float).eps * (np.abs(a) @ np.abs(b)) + k * 8 * slices * 2.0**(-7 * slices) * (
+        np.abs(a).max(2, keepdims=True) * np.abs(b).max(1, keepdims=True))
+    assert (np.abs(got - a @ b) <= bound).all()
