@@ -325,7 +325,8 @@ int Engine::alloc() {
   {   // inv_work_alloc: R buffer, pivots, row origins, INFO, interchange lists
     const long long cap = std::max(B_, S_);
     if (!dry_) NEGF_TRY(inv_work_alloc(inv_, M_, (int)cap, pool_, own_st_));
-    bytes_ += 16LL * cap * panel_width(M_) * M_ + 8LL * cap * M_ + 4LL * cap + 4LL * cap * kGjMoves;
+    bytes_ += 16LL * cap * panel_width(M_) * M_ + 8LL * cap * M_ + 4LL * cap + 4LL * cap * kGjMoves + 4LL * kGjTickets +
+              gj_next_bytes(M_, cap);
   }
   if (tc_) {
     const long long before = bytes_;

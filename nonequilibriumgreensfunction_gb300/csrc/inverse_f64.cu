@@ -12,6 +12,8 @@
 //   2. gj_swap:    applies the panel's row interchanges to the other columns, copies
 //                  their rows K into R (nb x n) and zeroes them.
 //   3. gj_update:  A(:, not K) += P * R(:, not K), P = A(:, K) (the factorised panel).
+// The FP32 form (a thread a row, n <= 640) factorises each panel after the first beside the update
+// before it (gj_step_kernel).
 // After the last panel, gj_colswap undoes the row pivoting as column interchanges.
 // INFO follows ZGETRF: the 1-based index of the first exactly-zero pivot (0 if none).
 #include "negf_internal.cuh"
@@ -180,26 +182,32 @@ __global__ void __launch_bounds__(PANEL_THREADS) gj_panel_kernel(T* A, long long
 // 72 / 33 us, 576 96 / 44 us.
 constexpr int RP_MAX_N = 640;   // 640 threads of up to 102 registers
 constexpr int RP_C = 32;
-template <int MAXT>   // threads at most: 512 (128 registers each) or RP_MAX_N (96)
-__global__ void __launch_bounds__(MAXT, 1) gj_panel_reg_kernel(float2* A, long long sA, int n, int k0, int kb,
-                                                                   int* ipiv, int* info, int* moves, int* orig) {
-  pdl_wait();
-  __shared__ __align__(16) float2 raw[RP_C], piv[RP_C];   // pivot row, unscaled and scaled
-  __shared__ unsigned w_key[RP_MAX_N / 32];
-  __shared__ int w_pos[RP_MAX_N / 32];
-  __shared__ int s_extra;
-  const int b = blockIdx.x;
-  const int t = threadIdx.x, lane = t & 31, warp = t >> 5, nwarps = blockDim.x >> 5;
-  float2* Ab = A + (long long)b * sA;
-  int* ip = ipiv + (long long)b * n;
-  float2 row[RP_C];
+struct PanelShared {
+  float2 raw[RP_C], piv[RP_C];   // pivot row, unscaled and scaled
+  unsigned w_key[RP_MAX_N / 32];
+  int w_pos[RP_MAX_N / 32];
+  int extra;
+};
+__device__ __forceinline__ void named_barrier(int id, int threads) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+// Threads 0 .. nthreads-1 (whole warps, nthreads >= n) with the panel's rows; ip, info, mv and
+// orig are those of the matrix Ab.
+template <bool WHOLE>   // nthreads is the whole CTA
+__device__ __forceinline__ void panel_rows(float2 (&row)[RP_C], PanelShared& sh, float2* Ab, int n, int k0, int kb,
+                                           int* ip, int* info, int* mv, int* orig, int nthreads) {
+  float2 *raw = sh.raw, *piv = sh.piv;
+  unsigned* w_key = sh.w_key;
+  int* w_pos = sh.w_pos;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5, nwarps = nthreads >> 5;
+  auto sync = [&]() {
+    if constexpr (WHOLE) __syncthreads();
+    else named_barrier(3, nthreads);
+  };
   const bool live = t < n;
-#pragma unroll
-  for (int j = 0; j < RP_C; ++j)
-    row[j] = (live && j < kb) ? Ab[(long long)(k0 + j) * n + t] : make_float2(0.f, 0.f);
   int pos = live ? t : 0x7fffffff;
-  const int from = live && k0 > 0 ? orig[(long long)b * n + t] : t;   // the row of A that is here
-  if (t == 0) s_extra = kb;
+  const int from = live && k0 > 0 ? orig[t] : t;   // the row of A that is here
+  if (t == 0) sh.extra = kb;
   // key of a pivot candidate: larger |re|+|im| first (non-negative floats order as their bits),
   // 0 = no candidate (a row above the step, a NaN)
   auto key_of = [&](float2 v, int r) -> unsigned {
@@ -213,7 +221,7 @@ __global__ void __launch_bounds__(MAXT, 1) gj_panel_reg_kernel(float2* A, long l
     const int r = k0 + c;
     const int wpos = __reduce_min_sync(0xffffffffu, key == wmax ? pos : 0x7fffffff);
     if (lane == 0) { w_key[warp] = wmax; w_pos[warp] = wpos; }
-    __syncthreads();
+    sync();
     const unsigned ck = lane < nwarps ? w_key[lane] : 0u;
     const unsigned best = __reduce_max_sync(0xffffffffu, ck);
     int p = __reduce_min_sync(0xffffffffu, (lane < nwarps && ck == best) ? w_pos[lane] : 0x7fffffff);
@@ -226,14 +234,14 @@ __global__ void __launch_bounds__(MAXT, 1) gj_panel_reg_kernel(float2* A, long l
         for (int j = 0; j < RP_C; j += 2)
           *reinterpret_cast<float4*>(&raw[j]) = make_float4(row[j].x, row[j].y, row[j + 1].x, row[j + 1].y);
         ip[r] = p;
-        if (row[0].x == 0.f && row[0].y == 0.f && info[b] == 0) info[b] = r + 1;
+        if (row[0].x == 0.f && row[0].y == 0.f && *info == 0) *info = r + 1;
       }
       __syncwarp();
       const float2 pv = raw[0];
       const float2 d = (pv.x == 0.f && pv.y == 0.f) ? make_float2(0.f, 0.f) : crcp(pv);
       piv[lane] = lane == 0 ? d : cmul(raw[lane], d);
     }
-    __syncthreads();
+    sync();
     if (own) pos = r;
     else if (pos == r) pos = p;
     const float4 p01 = *reinterpret_cast<const float4*>(&piv[0]);
@@ -281,20 +289,35 @@ __global__ void __launch_bounds__(MAXT, 1) gj_panel_reg_kernel(float2* A, long l
   }
   // the panel's interchanges as (destination, origin) rows for gj_swap, the rows K first: at
   // most kb of the others moved
-  int* mv = moves + (long long)b * GJ_MOVES;
   if (live) {
 #pragma unroll
     for (int j = 0; j < RP_C; ++j)
       if (j < kb) Ab[(long long)(k0 + j) * n + pos] = row[j];
-    orig[(long long)b * n + pos] = from;
-    const int q = (pos >= k0 && pos < k0 + kb) ? pos - k0 : (pos != t ? atomicAdd(&s_extra, 1) : -1);
+    orig[pos] = from;
+    const int q = (pos >= k0 && pos < k0 + kb) ? pos - k0 : (pos != t ? atomicAdd(&sh.extra, 1) : -1);
     if (q >= 0) {
       mv[1 + 2 * q] = pos;
       mv[2 + 2 * q] = t;
     }
   }
-  __syncthreads();
-  if (t == 0) mv[0] = s_extra;
+  sync();
+  if (t == 0) mv[0] = sh.extra;
+}
+
+template <int MAXT>   // threads at most: 512 (128 registers each) or RP_MAX_N (96)
+__global__ void __launch_bounds__(MAXT, 1) gj_panel_reg_kernel(float2* A, long long sA, int n, int k0, int kb,
+                                                               int* ipiv, int* info, int* moves, int* orig, int* tickets) {
+  pdl_wait();
+  __shared__ __align__(16) PanelShared sh;
+  const int b = blockIdx.x, t = threadIdx.x;
+  if (b == 0 && t < kGjTickets) tickets[t] = 0;
+  float2* Ab = A + (long long)b * sA;
+  float2 row[RP_C];
+#pragma unroll
+  for (int j = 0; j < RP_C; ++j)
+    row[j] = (t < n && j < kb) ? Ab[(long long)(k0 + j) * n + t] : make_float2(0.f, 0.f);
+  panel_rows<true>(row, sh, Ab, n, k0, kb, ipiv + (long long)b * n, info + b, moves + (long long)b * GJ_MOVES,
+             orig + (long long)b * n, blockDim.x);
 }
 
 // The FP64 inverse (n <= 1024; not the mixed form's redone ones, see zinv_f64) with panels of
@@ -451,11 +474,63 @@ __global__ void __launch_bounds__(256) gj_update_tiles_kernel(double2* A, long l
 // before any store, so the gather is a simultaneous permutation), writes rows K to R
 // (kb x n, column-major) with zeros in A, and the other touched rows back in place.
 // Panel columns get R = 0.
+// ahead > 0 (FP32): the first CTAs of a matrix form the next panel's `ahead` columns as the update
+// by this panel leaves them, in `next` (n x RP_C), so that the next panel can be factorised beside
+// the update of all other columns (gj_step_kernel).  128 rows x 16 columns a CTA, a thread a row
+// and eight columns: it gathers the interchanged rows itself and writes elsewhere, so no CTA waits
+// for another.  Bound: latency, one chain of list -> rows -> 32 steps from P in registers.
 constexpr int SWAP_WARPS = 8;
+constexpr int AHEAD_ROWS = 128, AHEAD_COLS = 16;
+// the CTA's part of the next panel's columns: rows i0 .., columns k1 + c0 ..
+__device__ __forceinline__ void gj_columns_ahead(const float2* Ab, int n, int k0, int kb, int k1, int ahead, int i0, int c0,
+                                                 const int* trow, const int* torig, int nt, float2* next) {
+  __shared__ __align__(16) float2 rs[RP_C][AHEAD_COLS];   // R of the columns
+  __shared__ int origin[AHEAD_ROWS];                      // row that moves to i0 + r
+  const int t = threadIdx.x, r = t % AHEAD_ROWS, i = i0 + r;
+  const int u0 = t / AHEAD_ROWS * 8;
+  if (t < AHEAD_ROWS) origin[t] = i;
+  __syncthreads();
+  if (t < nt && trow[t] >= i0 && trow[t] < i0 + AHEAD_ROWS) origin[trow[t] - i0] = torig[t];
+  // rows K head the list: R(k, j) is row torig[k] of column j
+  for (int e = t; e < RP_C * AHEAD_COLS; e += 256) {
+    const int k = e / AHEAD_COLS, u = e % AHEAD_COLS;
+    rs[k][u] = k < kb && c0 + u < ahead ? Ab[(long long)(k1 + c0 + u) * n + torig[k]] : make_float2(0.f, 0.f);
+  }
+  __syncthreads();
+  if (i >= n) return;
+  const bool pivot_row = i >= k0 && i < k1;   // zero before the update
+  const int from = origin[r];
+  const float2* pk = Ab + (long long)k0 * n + i;
+  float2 acc[8], c[8];
+#pragma unroll
+  for (int u = 0; u < 8; ++u) {
+    acc[u] = make_float2(0.f, 0.f);
+    c[u] = !pivot_row && c0 + u0 + u < ahead ? Ab[(long long)(k1 + c0 + u0 + u) * n + from] : make_float2(0.f, 0.f);
+  }
+  constexpr int PF = 16;
+#pragma unroll 1
+  for (int k = 0; k < kb; k += PF) {   // kb = RP_C
+    float2 f[PF];
+#pragma unroll
+    for (int q = 0; q < PF; ++q) f[q] = pk[(long long)(k + q) * n];
+#pragma unroll
+    for (int q = 0; q < PF; ++q)
+#pragma unroll
+      for (int u = 0; u < 8; u += 2) {
+        const float4 v = *reinterpret_cast<const float4*>(&rs[k + q][u0 + u]);
+        cfma(acc[u], f[q], make_float2(v.x, v.y));
+        cfma(acc[u + 1], f[q], make_float2(v.z, v.w));
+      }
+  }
+#pragma unroll
+  for (int u = 0; u < 8; ++u)
+    if (c0 + u0 + u < ahead) next[(long long)(c0 + u0 + u) * n + i] = cadd(acc[u], c[u]);
+}
+
 template <typename T>
-__global__ void __launch_bounds__(SWAP_WARPS * 32) gj_swap_kernel(T* A, long long sA, int n, int k0, int kb,
-                                                                  const int* ipiv, const int* moves, T* R,
-                                                                  long long sR) {
+__global__ void __launch_bounds__(SWAP_WARPS * 32, sizeof(T) == 8 ? 3 : 1)
+    gj_swap_kernel(T* A, long long sA, int n, int k0, int kb, const int* ipiv, const int* moves, T* R, long long sR,
+                   int ahead, T* next) {
   pdl_wait();
   __shared__ int trow[64], torig[64];
   __shared__ int s_nt;
@@ -489,9 +564,20 @@ __global__ void __launch_bounds__(SWAP_WARPS * 32) gj_swap_kernel(T* A, long lon
   __syncthreads();
   const int nt = s_nt;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int j = blockIdx.x * SWAP_WARPS + warp;
-  if (j >= n) return;
-  if (j >= k0 && j < k0 + kb) {
+  const int k1 = k0 + kb;
+  int block = blockIdx.x;
+  if constexpr (sizeof(T) == 8) {
+    const int ng = (ahead + AHEAD_COLS - 1) / AHEAD_COLS, nahead = ng * ((n + AHEAD_ROWS - 1) / AHEAD_ROWS);
+    if (block < nahead) {
+      gj_columns_ahead(Ab, n, k0, kb, k1, ahead, block / ng * AHEAD_ROWS, block % ng * AHEAD_COLS, trow, torig, nt,
+                       next + (long long)b * RP_C * n);
+      return;
+    }
+    block -= nahead;
+  }
+  const int j = block * SWAP_WARPS + warp;
+  if (j >= n || (j >= k1 && j < k1 + ahead)) return;
+  if (j >= k0 && j < k1) {
     for (int c = lane; c < kb; c += 32) Rb[(long long)j * kb + c] = CplxTraits<T>::make(0, 0);
     return;
   }
@@ -502,12 +588,12 @@ __global__ void __launch_bounds__(SWAP_WARPS * 32) gj_swap_kernel(T* A, long lon
   __syncwarp();
   if (lane < nt) {
     const int r = trow[lane];
-    if (r >= k0 && r < k0 + kb) { Rb[(long long)j * kb + (r - k0)] = v0; colj[r] = CplxTraits<T>::make(0, 0); }
+    if (r >= k0 && r < k1) { Rb[(long long)j * kb + (r - k0)] = v0; colj[r] = CplxTraits<T>::make(0, 0); }
     else colj[r] = v0;
   }
   if (lane + 32 < nt) {
     const int r = trow[lane + 32];
-    if (r >= k0 && r < k0 + kb) { Rb[(long long)j * kb + (r - k0)] = v1; colj[r] = CplxTraits<T>::make(0, 0); }
+    if (r >= k0 && r < k1) { Rb[(long long)j * kb + (r - k0)] = v1; colj[r] = CplxTraits<T>::make(0, 0); }
     else colj[r] = v1;
   }
 }
@@ -701,6 +787,137 @@ __global__ void __launch_bounds__(256, 2) gj_update_f32_pipelined(float2* A, lon
   cp_async_wait<0>();
 }
 
+// One step of the FP32 inverse: the rank-kb update by panel k0 beside the factorisation of the
+// next panel, k1 = k0 + kb, whose columns gj_swap_kernel left updated in `next`.  CTA b < batch factorises
+// matrix b's; the other CTAs, and these when they are done, take output tiles of 80 x 48 of the
+// remaining columns from a counter, each half of a CTA its own tiles, as gj_update_f32_pipelined.
+// The two panels' columns are left out of the tiles' count, and 48 wide tiles leave less of it in a
+// last ragged one: at n = 400 7 x 48 of 336 columns, where 80 wide tiles of all are 5 x 80.
+// A panel is the work of one SM and bound by latency, so on its own it leaves the other SMs idle
+// and the update waits.  Bound now: the panel's chain of 32 steps for few matrices, the FP32 pipe
+// for many.  A whole inverse on GB300, panel, interchanges and update one after another against
+// this: n = 144, 8 matrices 178 / 153 us; n = 400, 8 650 / 526, 32 1028 / 768, 160 3680 / 3322;
+// n = 576, 8 1343 / 999, 32 2632 / 2022.
+// Every element is formed by the operations of the separate kernels, so the inverse is theirs bit
+// for bit.
+constexpr int ST_C = 3, ST_N = 16 * ST_C, ST_RS = ST_N + 1;   // columns a thread, of a tile, its stride
+constexpr int ST_SLABS = 32 * UPD_T + 32 * ST_RS;             // float2 of one buffer: P slab, then R slab
+template <int MAXT>
+__global__ void __launch_bounds__(MAXT, 1)
+    gj_step_kernel(float2* A, long long sA, int n, int k0, int kb, const float2* R, long long sR, int kb1, int* ipiv,
+                   int* info, int* moves, int* orig, int batch, int ntm, int ntn, long long ntiles, int* ticket, int pthreads, bool leave,
+                   const float2* next) {
+  pdl_wait();
+  extern __shared__ __align__(16) unsigned char step_raw[];
+  __shared__ __align__(16) PanelShared sh;
+  __shared__ int s_next[2];
+  const int t = threadIdx.x;
+  const int k1 = k0 + kb;
+  if (blockIdx.x < batch) {
+    const int b = blockIdx.x;
+    float2* Ab = A + (long long)b * sA;
+    if (t < pthreads) {
+      float2 row[RP_C];
+#pragma unroll
+      for (int j = 0; j < RP_C; ++j)
+        row[j] = (t < n && j < kb1) ? next[((long long)b * RP_C + j) * n + t] : make_float2(0.f, 0.f);
+      panel_rows<false>(row, sh, Ab, n, k1, kb1, ipiv + (long long)b * n, info + b, moves + (long long)b * GJ_MOVES,
+                 orig + (long long)b * n, pthreads);
+    }
+    if (leave) return;
+    __syncthreads();
+  }
+  if (t >= 512) return;
+  const int g = t >> 8, tg = t & 255;
+  const int tx = tg & 15, ty = tg >> 4;
+  float2* bufs = reinterpret_cast<float2*>(step_raw) + (long long)g * 2 * ST_SLABS;   // [2][ST_SLABS]
+  const long long per_item = (long long)ntm * ntn;
+  const int skip = kb + kb1, cols = n - skip;   // columns outside the two panels: c, from k0 on c + skip
+  auto column = [&](int c) { return c < k0 ? c : c + skip; };
+  auto issue = [&](long long q, float2* Ps) {
+    const int b = (int)(q / per_item);
+    const int r = (int)(q % per_item);
+    const int m0 = (r / ntn) * UPD_T, n0 = (r % ntn) * ST_N;
+    const float2* Ab = A + (long long)b * sA;
+    const float2* Rb = R + (long long)b * sR;
+    float2* Rs = Ps + 32 * UPD_T;
+    for (int e = tg; e < kb * UPD_T; e += 256) {
+      const int k = e / UPD_T, i = e % UPD_T;
+      const bool okp = m0 + i < n;
+      cp_async8(&Ps[k * UPD_T + i], okp ? (const void*)&Ab[(long long)(k0 + k) * n + m0 + i] : (const void*)Ab,
+                okp ? 8 : 0);
+    }
+    for (int e = tg; e < kb * ST_N; e += 256) {
+      const int j = e / kb, kk = e % kb;
+      const bool okr = n0 + j < cols;
+      cp_async8(&Rs[kk * ST_RS + j], okr ? (const void*)&Rb[(long long)column(n0 + j) * kb + kk] : (const void*)Rb,
+                okr ? 8 : 0);
+    }
+    cp_async_commit();
+  };
+  if (tg == 0) s_next[g] = atomicAdd(ticket, 1);
+  named_barrier(1 + g, 256);
+  long long q = s_next[g];
+  named_barrier(1 + g, 256);
+  if (q < ntiles) issue(q, bufs);
+  for (int it = 0; q < ntiles; ++it) {
+    const float2* Ps = bufs + (it & 1) * ST_SLABS;
+    const float2* Rs = Ps + 32 * UPD_T;
+    int taken = 0;
+    if (tg == 0) taken = atomicAdd(ticket, 1);
+    const int b = (int)(q / per_item);
+    const int r = (int)(q % per_item);
+    const int m0 = (r / ntn) * UPD_T, n0 = (r % ntn) * ST_N;
+    float2* Ab = A + (long long)b * sA;
+    auto updated = [&](int i, int j) -> float2* {   // nullptr: outside
+      const int row = m0 + tx + 16 * i, c = n0 + ty + 16 * j;
+      if (row >= n || c >= cols) return nullptr;
+      return Ab + (long long)column(c) * n + row;
+    };
+    float2 cin[UPD_R][ST_C];
+#pragma unroll
+    for (int j = 0; j < ST_C; ++j)
+#pragma unroll
+      for (int i = 0; i < UPD_R; ++i) {
+        const float2* cp = updated(i, j);
+        cin[i][j] = cp ? *cp : make_float2(0.0f, 0.0f);
+      }
+    cp_async_wait<0>();
+    if (tg == 0) s_next[g] = taken;
+    named_barrier(1 + g, 256);
+    // the next tile's slabs into the other buffer, which every thread finished reading before the
+    // barrier that ended the previous tile
+    const long long qn = s_next[g];
+    if (qn < ntiles) issue(qn, bufs + ((it + 1) & 1) * ST_SLABS);
+    float2 acc[UPD_R][ST_C];
+#pragma unroll
+    for (int i = 0; i < UPD_R; ++i)
+#pragma unroll
+      for (int j = 0; j < ST_C; ++j) acc[i][j] = make_float2(0.0f, 0.0f);
+#pragma unroll 1
+    for (int k = 0; k < kb; ++k) {
+      float2 av[UPD_R], bv[ST_C];
+#pragma unroll
+      for (int i = 0; i < UPD_R; ++i) av[i] = Ps[k * UPD_T + tx + 16 * i];
+#pragma unroll
+      for (int j = 0; j < ST_C; ++j) bv[j] = Rs[k * ST_RS + ty + 16 * j];
+#pragma unroll
+      for (int i = 0; i < UPD_R; ++i)
+#pragma unroll
+        for (int j = 0; j < ST_C; ++j) cfma(acc[i][j], av[i], bv[j]);
+    }
+#pragma unroll
+    for (int j = 0; j < ST_C; ++j)
+#pragma unroll
+      for (int i = 0; i < UPD_R; ++i) {
+        float2* cp = updated(i, j);
+        if (cp) *cp = cadd(acc[i][j], cin[i][j]);
+      }
+    named_barrier(1 + g, 256);   // this buffer is free for the tile after next, s_next for its number
+    q = qn;
+  }
+}
+
 // One thread per row: column interchanges in reverse pivot order.
 template <typename T>
 __global__ void gj_colswap_kernel(T* A, long long sA, int n, const int* ipiv) {
@@ -864,6 +1081,8 @@ int panel_width(int n, int elem_bytes) {
   return nb;
 }
 
+long long gj_next_bytes(int n, long long batch) { return n <= RP_MAX_N ? 8LL * RP_C * n * batch : 0; }
+
 int inv_work_alloc(InvWork& w, int n, int batch, cudaMemPool_t pool, cudaStream_t st) {
   if (w.n_cap >= n && w.batch_cap >= batch && w.rbuf) return NEGF_OK;
   inv_work_free(w, st);
@@ -877,6 +1096,8 @@ int inv_work_alloc(InvWork& w, int n, int batch, cudaMemPool_t pool, cudaStream_
   if (!get((void**)&w.ipiv, sizeof(int) * (size_t)batch * n)) return NEGF_ENOMEM;
   if (!get((void**)&w.info, sizeof(int) * (size_t)batch)) return NEGF_ENOMEM;
   if (!get((void**)&w.orig, sizeof(int) * (size_t)batch * n)) return NEGF_ENOMEM;
+  if (!get((void**)&w.tickets, sizeof(int) * kGjTickets)) return NEGF_ENOMEM;
+  if (n <= RP_MAX_N && !get((void**)&w.next, gj_next_bytes(n, batch))) return NEGF_ENOMEM;
   if (!get((void**)&w.moves, sizeof(int) * (size_t)batch * kGjMoves)) return NEGF_ENOMEM;
   w.n_cap = n;
   w.batch_cap = batch;
@@ -884,7 +1105,7 @@ int inv_work_alloc(InvWork& w, int n, int batch, cudaMemPool_t pool, cudaStream_
 }
 
 void inv_work_free(InvWork& w, cudaStream_t st) {
-  for (void* p : {(void*)w.rbuf, (void*)w.ipiv, (void*)w.info, (void*)w.orig, (void*)w.moves})
+  for (void* p : {(void*)w.rbuf, (void*)w.ipiv, (void*)w.info, (void*)w.orig, (void*)w.moves, (void*)w.tickets, (void*)w.next})
     if (p) {
       if (w.pooled) cudaFreeAsync(p, st);
       else cudaFree(p);
@@ -941,25 +1162,37 @@ int gj_invert(T* A, long long sA, int n, int batch, InvWork& w, cudaStream_t st)
   NEGF_CUDA_TRY(cudaMemsetAsync(w.info, 0, sizeof(int) * batch, st));
   T* rbuf = reinterpret_cast<T*>(w.rbuf);
   const long long sR = (long long)nb * n;
+  // Each panel after the first beside the update before it (gj_step_kernel).  With more matrices
+  // than SMs the panels of small ones share an SM better on their own: apart against together,
+  // n = 64, 160 matrices 92 / 101 us, 320 121 / 143; n = 144, 320 535 / 578; but n = 256, 320
+  // 2632 / 2217 us.
+  const bool steps = sizeof(T) == 8 && n <= RP_MAX_N && nb == RP_C && (batch <= sm_count_cached() || n >= 256);
   for (int k0 = 0; k0 < n; k0 += nb) {
     const int kb = (n - k0 < nb) ? (n - k0) : nb;
-    cudaEvent_t ev;
-    timed_begin(st, TK_PANEL, 8.0 * n * (double)kb * kb * batch, &ev);
-    const int* moves = nullptr;
-    if (sizeof(T) == 8 && n <= RP_MAX_N) {
-      const int threads = (n + 31) / 32 * 32;
-      auto panel = threads <= 512 ? gj_panel_reg_kernel<512> : gj_panel_reg_kernel<RP_MAX_N>;
-      pdl_launch(panel, batch, threads, 0, st, reinterpret_cast<float2*>(A), sA, n, k0, kb, w.ipiv, w.info, w.moves, w.orig);
-      moves = w.moves;
-    } else {
-      pdl_launch(gj_panel_kernel<T>, batch, PANEL_THREADS, smem, st, A, sA, n, k0, kb, w.ipiv, w.info);
+    const bool reg = sizeof(T) == 8 && n <= RP_MAX_N;
+    const int threads = (n + 31) / 32 * 32;   // of a panel in registers
+    const int* moves = reg ? w.moves : nullptr;
+    if (!steps || k0 == 0) {   // the others were factorised beside the last update
+      cudaEvent_t ev;
+      timed_begin(st, TK_PANEL, 8.0 * n * (double)kb * kb * batch, &ev);
+      if (reg) {
+        auto panel = threads <= 512 ? gj_panel_reg_kernel<512> : gj_panel_reg_kernel<RP_MAX_N>;
+        pdl_launch(panel, batch, threads, 0, st, reinterpret_cast<float2*>(A), sA, n, k0, kb, w.ipiv, w.info, w.moves,
+                   w.orig, w.tickets);
+      } else {
+        pdl_launch(gj_panel_kernel<T>, batch, PANEL_THREADS, smem, st, A, sA, n, k0, kb, w.ipiv, w.info);
+      }
+      NEGF_CUDA_TRY(cudaGetLastError());
+      timed_end(st, TK_PANEL, ev);
+      count_launch();
     }
+    const int ahead = steps ? std::min(nb, n - k0 - kb) : 0;   // the next panel's columns
+    const int nahead = (ahead + AHEAD_COLS - 1) / AHEAD_COLS * ((n + AHEAD_ROWS - 1) / AHEAD_ROWS);
+    dim3 g2((n + SWAP_WARPS - 1) / SWAP_WARPS + nahead, batch);
+    pdl_launch(gj_swap_kernel<T>, g2, SWAP_WARPS * 32, 0, st, A, sA, n, k0, kb, w.ipiv, moves, rbuf, sR, ahead,
+               reinterpret_cast<T*>(w.next));
     NEGF_CUDA_TRY(cudaGetLastError());
-    timed_end(st, TK_PANEL, ev);
-    dim3 g2((n + SWAP_WARPS - 1) / SWAP_WARPS, batch);
-    pdl_launch(gj_swap_kernel<T>, g2, SWAP_WARPS * 32, 0, st, A, sA, n, k0, kb, w.ipiv, moves, rbuf, sR);
-    NEGF_CUDA_TRY(cudaGetLastError());
-    count_launch(2);
+    count_launch();
     // A(:, j) += P R(:, j) for the columns outside the panel
     {
       cudaEvent_t eu;
@@ -967,10 +1200,23 @@ int gj_invert(T* A, long long sA, int n, int batch, InvWork& w, cudaStream_t st)
       const int nt = (n + UPD_T - 1) / UPD_T;
       if constexpr (sizeof(T) == 8) {
         const long long ntiles = (long long)nt * nt * batch;
-        const int grid = (int)std::min<long long>(ntiles, 2LL * sm_count_cached());
-        pdl_launch(gj_update_f32_pipelined, grid, 256, upp_smem, st, reinterpret_cast<float2*>(A), sA, n, k0, kb,
-                                                             reinterpret_cast<const float2*>(rbuf), sR, nt, nt,
-                                                             ntiles);
+        if (ahead > 0) {
+          const int sms = sm_count_cached();
+          auto stepk = threads <= 512 ? gj_step_kernel<512> : gj_step_kernel<RP_MAX_N>;
+          const size_t smem = 4 * sizeof(float2) * (size_t)ST_SLABS;
+          NEGF_CUDA_TRY(cudaFuncSetAttribute(stepk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+          const int ntn = (n - kb - ahead + ST_N - 1) / ST_N;
+          const long long tiles = (long long)nt * ntn * batch;
+          // a CTA an SM; with more matrices than SMs the CTAs for the tiles come after the panels'
+          const int grid = batch > sms ? batch + sms : (int)std::min<long long>(batch + (tiles + 1) / 2, sms);
+          pdl_launch(stepk, grid, threads <= 512 ? 512 : RP_MAX_N, smem, st, reinterpret_cast<float2*>(A), sA, n, k0, kb,
+                     reinterpret_cast<const float2*>(rbuf), sR, ahead, w.ipiv, w.info, w.moves, w.orig, batch, nt, ntn,
+                     tiles, w.tickets + k0 / nb, threads, batch > sms, w.next);
+        } else {
+          const int grid = (int)std::min<long long>(ntiles, 2LL * sm_count_cached());
+          pdl_launch(gj_update_f32_pipelined, grid, 256, upp_smem, st, reinterpret_cast<float2*>(A), sA, n, k0, kb,
+                     reinterpret_cast<const float2*>(rbuf), sR, nt, nt, ntiles);
+        }
       } else {
         // 80 x 80 tiles where they fill the device twice over, smaller ones for a few matrices
         if ((long long)nt * nt * batch < 2LL * sm_count_cached())
@@ -1009,7 +1255,7 @@ int gj_invert_narrow(double2* A, long long sA, int n, int batch, InvWork& w, cud
     NEGF_CUDA_TRY(cudaGetLastError());
     timed_end(st, TK_PANEL, ev);
     pdl_launch(gj_swap_kernel<double2>, dim3((n + SWAP_WARPS - 1) / SWAP_WARPS, batch), SWAP_WARPS * 32, 0, st, A, sA,
-               n, k0, kb, w.ipiv, w.moves, w.rbuf, sR);
+               n, k0, kb, w.ipiv, w.moves, w.rbuf, sR, 0, (double2*)nullptr);
     NEGF_CUDA_TRY(cudaGetLastError());
     timed_begin(st, TK_GEMM, 8.0 * n * (double)(n - kb) * kb * batch, &ev);
     pdl_launch(gj_update_tiles_kernel<NP_C>, dim3((n + NU_M - 1) / NU_M, (n + NU_N - 1) / NU_N, batch), 256, 0, st, A, sA, n,

@@ -175,12 +175,15 @@ int cgemm_f32(const GemmBatchT<float2>& g, cudaStream_t st);   // FP32 twin (inv
 // Batched in-place inverse (blocked Gauss-Jordan with partial row pivoting)
 // ----------------------------------------------------------------------------------
 constexpr int kGjMoves = 1 + 2 * 64;
+constexpr int kGjTickets = 32;   // more than the steps of an FP32 inverse with register panels
 struct InvWork {
   double2* rbuf = nullptr;   // batch * nb * n (FP64; reused as float2 storage by the FP32 form)
   int* ipiv = nullptr;       // batch * n
   int* info = nullptr;       // batch
   int* orig = nullptr;       // batch * n: row that each place held at first (FP32 form, register panels)
   bool columns_pending = false;   // the last FP32 inverse left its column interchanges to orig
+  int* tickets = nullptr;    // kGjTickets: the next output tile of each step (FP32 form)
+  float2* next = nullptr;    // batch * 32 * n: the next panel's columns (FP32 form, register panels)
   int* moves = nullptr;      // batch * kGjMoves: the interchanges of the panel at hand (FP32 form)
   int n_cap = 0, batch_cap = 0, nb = 0;
   bool pooled = false;       // allocated stream-ordered from a memory pool
@@ -188,6 +191,7 @@ struct InvWork {
 // pool = nullptr: plain cudaMalloc / cudaFree; otherwise stream-ordered on `st` from `pool`
 int inv_work_alloc(InvWork& w, int n, int batch, cudaMemPool_t pool = nullptr, cudaStream_t st = 0);
 void inv_work_free(InvWork& w, cudaStream_t st = 0);
+long long gj_next_bytes(int n, long long batch);   // of InvWork::next
 int panel_width(int n, int elem_bytes = 16);
 // A: batch matrices of n x n, column-major, consecutive at stride sA.  On return A holds
 // the inverses; w.info[b] (device) holds the LAPACK-style INFO of each matrix.

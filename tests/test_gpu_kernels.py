@@ -148,3 +148,23 @@ def test_sliced_rows_at_their_block_sizes(need_gpu, m, k, slices):
     bound = 8 * k * np.finfo(float).eps * (np.abs(a) @ np.abs(b)) + k * 8 * slices * 2.0**(-7 * slices) * (
         np.abs(a).max(2, keepdims=True) * np.abs(b).max(1, keepdims=True))
     assert (np.abs(got - a @ b) <= bound).all()
+
+
+# The FP32 inverse factorises a panel beside the update before it: a CTA a matrix up to one an SM,
+# the panels before the tiles with more (M >= 256), and on their own with more small ones; tiles of 48
+# columns outside the two panels.  No result depends on the batch: 160 energies at once (up to 320
+# lead blocks) and four at a time give the same bits.
+@pytest.mark.parametrize("npy,npz", [(3, 3), (5, 13), (5, 20)])
+def test_inverses_do_not_depend_on_the_batch(need_gpu, npy, npz):
+    htotd, hopx = hamiltonian.ti_wire(3, npy, npz, W=0.1, seed=3, flux=0.4, zeeman=0.01)
+    energies = np.linspace(-0.3, 0.3, 160)
+    out = []
+    for batch in (160, 4):
+        with Solver(3, npy, npz, eta=1e-2, sr_tol=1e-6, max_batch=batch, precision="mixed") as s:
+            s.set_hamiltonian(htotd, hopx)
+            pick = [energies] if batch == 160 else [energies[:4], energies[78:82], energies[-4:]]
+            res = [s.solve_batch(e, 0.7, 0.2, 1e-3) for e in pick]
+        out.append({k: np.concatenate([np.atleast_1d(r[k]) for r in res]) for k in ("T12", "Modec1", "sr_iters")})
+    some = np.r_[0:4, 78:82, 156:160]
+    for k, v in out[0].items():
+        assert np.array_equal(v[some], out[1][k]), k
