@@ -1,4 +1,4 @@
-// Host orchestration of the per-energy NEGF solve (FP64 form).
+// Host orchestration of the per-energy NEGF solve (FP64 and mixed forms).
 //
 // Mapping to the reference (all paths relative to the reference project):
 //   solve_sr   - Contact_Self_Energy / Sancho_Rubio, Source/Contact_Self_Energy.F90:68-101,110-223

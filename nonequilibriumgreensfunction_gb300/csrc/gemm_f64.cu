@@ -2,8 +2,9 @@
 //
 // GB300 (sm_103) executes about two FP64 fused multiply-adds per clock per SM: cuBLAS
 // ZGEMM measures 1.10 TFLOP/s on the whole part, and this kernel 1.00 TFLOP/s with its FP64
-// pipe busy on 97.6% of its active cycles (ncu).  The FP64 form is therefore bound by that
-// pipe, and this kernel only has to keep it busy: 64x64 complex output tiles, K steps of 8
+// pipe busy on 97.6% of its active cycles (ncu).  Where the FP64 form runs on it (M > 800, or
+// without room for the tensor-core form's workspace) it is bound by that pipe, and this kernel
+// only has to keep it busy: 64x64 complex output tiles, K steps of 8
 // staged through double-buffered shared memory, 4x4 complex accumulators per thread
 // (4 DFMA per complex multiply-add).  Replaces the ZGEMM calls of
 // Source/Recursive_Greens.F90, Source/Contact_Self_Energy.F90 and the zgemm-equivalent

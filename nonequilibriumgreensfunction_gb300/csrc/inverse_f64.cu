@@ -7,8 +7,8 @@
 // solves, which keeps the FP64 pipe of all SMs busy across a batch of matrices.
 //
 // Per panel K = [k0, k0+nb), nb = 8 in FP64 up to n = 1024 and 32 otherwise:
-//   1. gj_panel:   one CTA per matrix factorises the n x nb panel in shared memory
-//                  (pivot = first max of |re|+|im| over rows >= k, as LAPACK izamax).
+//   1. gj_panel:   one CTA per matrix (in FP64 a cluster of eight for a few matrices)
+//                  factorises the n x nb panel in shared memory or registers (pivot = first max of |re|+|im| over rows >= k, as LAPACK izamax).
 //   2. gj_swap:    applies the panel's row interchanges to the other columns, copies
 //                  their rows K into R (nb x n) and zeroes them.
 //   3. gj_update:  A(:, not K) += P * R(:, not K), P = A(:, K) (the factorised panel).
@@ -163,6 +163,127 @@ __global__ void __launch_bounds__(PANEL_THREADS) gj_panel_kernel(T* A, long long
   panel_factor<T>(Ps, n, k0, kb, ipiv + (long long)b * n, info + b, red_v, red_i, &s_piv, &s_d);
   T* dst = Ab + (long long)k0 * n;
   for (int e = t; e < n * kb; e += PANEL_THREADS) dst[e] = Ps[e];
+}
+
+// The FP64 panel of a few matrices: a cluster of eight CTAs a matrix, each with an eighth of the
+// rows in its shared memory.  A panel is 4 n nb^2 multiply-adds on FP64 pipes of about two a clock,
+// and one SM's was all that gj_panel_kernel used.  A column step is: every CTA's pivot candidates
+// to all (distributed shared memory), a cluster barrier, the pivot row scaled by its owner and sent
+// to all, the row it changes places with sent to that owner, a second barrier, and the elimination
+// of the own rows.  Pivots, ties and every element's operations are those of panel_factor, so the
+// panel is bitwise the same.  Bound: FP64 pipes, then the two barriers and the reciprocal of a step.
+// On GB300, one CTA against a cluster, a panel of a few matrices: n = 144, 32 columns 277 / 152 us;
+// n = 576, 16 columns 251 / 106 us.
+constexpr int CLP_CTAS = 8, CLP_THREADS = 256, CLP_WARPS = CLP_THREADS / 32;
+__device__ __forceinline__ void clp_barrier() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t clp_remote(const void* p, int rank) {
+  uint32_t a;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ void clp_store(const void* p, int rank, double2 v) {
+  asm volatile("st.shared::cluster.v2.f64 [%0], {%1, %2};" ::"r"(clp_remote(p, rank)), "d"(v.x), "d"(v.y) : "memory");
+}
+__global__ void __launch_bounds__(CLP_THREADS) gj_panel_cluster_kernel(double2* A, long long sA, int n, int k0, int kb,
+                                                                       int* ipiv, int* info) {
+  pdl_wait();
+  extern __shared__ __align__(16) unsigned char clp_raw[];
+  __shared__ __align__(16) double2 prow[33];   // new pivot row; [32]: the reciprocal, zero without a pivot
+  __shared__ __align__(16) double2 rrow[32];   // the row that goes to the pivot's place (in its owner)
+  __shared__ __align__(16) double2 cand[CLP_CTAS][CLP_WARPS];   // (measure, row) of every warp's best
+  const int b = blockIdx.x / CLP_CTAS, rank = blockIdx.x % CLP_CTAS;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int share = (n + CLP_CTAS - 1) / CLP_CTAS;   // rows a CTA
+  const int r0 = rank * share, nr = max(0, min(share, n - r0));
+  double2* Ps = reinterpret_cast<double2*>(clp_raw);   // [kb][share]
+  double2* fcol = Ps + (long long)kb * share;          // the column of the step, before it
+  double2* Ab = A + (long long)b * sA + (long long)k0 * n;
+  for (int e = t; e < nr * kb; e += CLP_THREADS) Ps[e / nr * share + e % nr] = Ab[(long long)(e / nr) * n + r0 + e % nr];
+  clp_barrier();   // all CTAs of the cluster are there
+  for (int c = 0; c < kb; ++c) {
+    const int r = k0 + c;
+    // the measure as an integer, which orders as it does: comparisons stay off the FP64 pipe;
+    // 0: no candidate (a row above the step, a NaN)
+    unsigned long long bv = 0;
+    int bi = n;
+    for (int il = t; il < nr; il += CLP_THREADS) {
+      const double2 v = Ps[c * share + il];
+      fcol[il] = v;
+      const unsigned long long m = (unsigned long long)__double_as_longlong(cabs1(v));
+      if (r0 + il >= r && m <= 0x7FF0000000000000ULL) argmax_combine(bv, bi, m + 1, r0 + il);
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+      const unsigned long long ov = __shfl_xor_sync(0xffffffffu, bv, off);
+      const int oi = __shfl_xor_sync(0xffffffffu, bi, off);
+      argmax_combine(bv, bi, ov, oi);
+    }
+    if (lane < CLP_CTAS)
+      clp_store(&cand[rank][warp], lane, make_double2(__longlong_as_double((long long)bv), __longlong_as_double(bi)));
+    clp_barrier();
+    // every warp of every CTA finds the same pivot among the 64 candidates
+    static_assert(CLP_CTAS * CLP_WARPS == 64, "two candidates a lane");
+    const double2 c0 = cand[0][lane], c1 = cand[CLP_CTAS / 2][lane];
+    bv = (unsigned long long)__double_as_longlong(c0.x);
+    bi = (int)__double_as_longlong(c0.y);
+    argmax_combine(bv, bi, (unsigned long long)__double_as_longlong(c1.x), (int)__double_as_longlong(c1.y));
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+      const unsigned long long ov = __shfl_xor_sync(0xffffffffu, bv, off);
+      const int oi = __shfl_xor_sync(0xffffffffu, bi, off);
+      argmax_combine(bv, bi, ov, oi);
+    }
+    const int p = bi >= n ? r : bi;
+    if (warp == 0 && p / share == rank) {
+      const double2 pv = fcol[p - r0];
+      const bool zero = pv.x == 0 && pv.y == 0;
+      double2 d = make_double2(0, 0);
+      if (!zero) d = crcp(pv);
+      if (lane == 0) {
+        ipiv[(long long)b * n + r] = p;
+        if (zero) atomicCAS(&info[b], 0, r + 1);   // other columns' owners are other CTAs
+      }
+      const bool singular = d.x == 0 && d.y == 0;
+      double2 v = make_double2(0, 0);
+      if (lane < kb) {
+        v = Ps[lane * share + p - r0];
+        if (!singular) v = lane == c ? d : cmul(v, d);
+      }
+      for (int q = 0; q < CLP_CTAS; ++q) {
+        clp_store(&prow[lane], q, v);
+        if (lane == 0) clp_store(&prow[32], q, d);
+      }
+    }
+    if (warp == 1 && r / share == rank && lane < kb) clp_store(&rrow[lane], p / share, Ps[lane * share + r - r0]);
+    clp_barrier();
+    const double2 d = prow[32];
+    const bool singular = d.x == 0 && d.y == 0;
+    for (int e = t; e < nr * kb; e += CLP_THREADS) {
+      const int j = e / nr, il = e % nr, i = r0 + il;
+      double2* at = &Ps[j * share + il];
+      if (i == r) { *at = prow[j]; continue; }
+      const bool moved = i == p;   // holds row r from here on
+      double2 v = moved ? rrow[j] : *at;
+      if (!singular) {
+        const double2 f = moved ? rrow[c] : fcol[il];
+        if (j == c) {
+          v = cmul(make_double2(-f.x, -f.y), d);
+        } else {
+          const double2 rv = prow[j];
+          v.x = fma(-f.x, rv.x, v.x);
+          v.x = fma(f.y, rv.y, v.x);
+          v.y = fma(-f.x, rv.y, v.y);
+          v.y = fma(-f.y, rv.x, v.y);
+        }
+      }
+      *at = v;
+    }
+    __syncthreads();
+  }
+  for (int e = t; e < nr * kb; e += CLP_THREADS) Ab[(long long)(e / nr) * n + r0 + e % nr] = Ps[e / nr * share + e % nr];
 }
 
 // The FP32 panel with its rows in registers: thread t holds row t of the panel (32 float2), so
@@ -1167,6 +1288,10 @@ int gj_invert(T* A, long long sA, int n, int batch, InvWork& w, cudaStream_t st)
   // n = 64, 160 matrices 92 / 101 us, 320 121 / 143; n = 144, 320 535 / 578; but n = 256, 320
   // 2632 / 2217 us.
   const bool steps = sizeof(T) == 8 && n <= RP_MAX_N && nb == RP_C && (batch <= sm_count_cached() || n >= 256);
+  // FP64 panels of a few matrices on clusters.  Whole inverses, one CTA against clusters: n = 144, 1
+  // matrix 1.81 / 1.12 ms, 24 2.34 / 1.77; n = 576, 1 11.4 / 6.2 ms, 24 53.1 / 49.2.  More clusters
+  // than that share SMs, and their barriers wait for one another.
+  const bool clustered = sizeof(T) == 16 && 4 * batch * CLP_CTAS <= 5 * sm_count_cached();
   for (int k0 = 0; k0 < n; k0 += nb) {
     const int kb = (n - k0 < nb) ? (n - k0) : nb;
     const bool reg = sizeof(T) == 8 && n <= RP_MAX_N;
@@ -1179,6 +1304,11 @@ int gj_invert(T* A, long long sA, int n, int batch, InvWork& w, cudaStream_t st)
         auto panel = threads <= 512 ? gj_panel_reg_kernel<512> : gj_panel_reg_kernel<RP_MAX_N>;
         pdl_launch(panel, batch, threads, 0, st, reinterpret_cast<float2*>(A), sA, n, k0, kb, w.ipiv, w.info, w.moves,
                    w.orig, w.tickets);
+      } else if (sizeof(T) == 16 && clustered) {
+        const size_t csmem = sizeof(double2) * (size_t)((n + CLP_CTAS - 1) / CLP_CTAS) * (kb + 1);
+        NEGF_CUDA_TRY(cudaFuncSetAttribute(gj_panel_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csmem));
+        pdl_launch_cluster(dim3(CLP_CTAS), gj_panel_cluster_kernel, batch * CLP_CTAS, CLP_THREADS, csmem, st,
+                           reinterpret_cast<double2*>(A), sA, n, k0, kb, w.ipiv, w.info);
       } else {
         pdl_launch(gj_panel_kernel<T>, batch, PANEL_THREADS, smem, st, A, sA, n, k0, kb, w.ipiv, w.info);
       }

@@ -119,8 +119,8 @@ def test_small_cross_sections_in_every_cluster(need_gpu, channel, npy, npz):
     assert np.abs(rho[..., 0] - want).max() <= 1e-9 * np.abs(want).max()
 
 
-# The FP64 inverse has panels of eight columns up to n = 1024 (the last of 1, 7 or 8) and wider
-# ones beyond.  Tolerance: 100 n eps of the product of the norms; a zero column gives its INFO.
+# The FP64 inverse has panels of eight columns up to n = 1024 (the last of 1, 7 or 8); beyond, and in
+# the mixed form's redone inverses, a few matrices have their panels on clusters of eight CTAs.  Tolerance: 100 n eps of the product of the norms; a zero column gives its INFO.
 @pytest.mark.parametrize("n", [1, 7, 8, 9, 33, 1024, 1025])
 def test_fp64_inverse_at_its_panel_sizes(need_gpu, n):
     rng = np.random.default_rng(n)
