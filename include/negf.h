@@ -56,7 +56,9 @@ extern "C" {
 #define NEGF_ESCRATCH    (-12)   /* negf_zgemm_noalloc: sizes exceed its static scratch  */
 
 /* ---- arithmetic form ------------------------------------------------------------- */
-#define NEGF_PREC_FP64     0     /* plain FP64 complex throughout                        */
+#define NEGF_PREC_FP64     0     /* FP64 complex results throughout.  32 <= M <= 800: products on the
+                                    tensor cores as nine exact BF16 slices, inverses refined to
+                                    FP64; other sizes on the FP64 pipe                   */
 #define NEGF_PREC_MIXED    1     /* tcgen05 BF16 sliced products, FP64 refinement        */
 
 typedef struct negf_params {
@@ -145,14 +147,14 @@ typedef struct negf_stats {
     double  gemm_flops;      /* their real flops, 8*m*n*k per complex GEMM                 */
     int64_t panel_launches;  /* Gauss-Jordan panel factorisations                          */
     double  panel_ms;
-    int64_t tc_launches;     /* tcgen05 sliced-BF16 GEMM launches (mixed form)             */
+    int64_t tc_launches;     /* tcgen05 sliced-BF16 GEMM launches                          */
     double  tc_ms;
     double  tc_flops;        /* BF16 tensor flops issued: S(S+1)/2 slice pairs x 8*m*n*k   */
     double  tc_complex_flops;/* the complex products they compute, 8*m*n*k                 */
-    int64_t fallbacks;       /* mixed form: inverses redone in FP64 (residual too large)   */
-    double  ns_residual_max; /* mixed form: largest accepted first Newton-Schulz residual  */
-    double  f32_gemm_ms;     /* FP32 Gauss-Jordan rank-nb updates (mixed form)             */
-    double  slice_ms;        /* operand slicing kernels (mixed form)                       */
+    int64_t fallbacks;       /* refined inverses redone in FP64 (residual too large)       */
+    double  ns_residual_max; /* largest accepted first Newton-Schulz residual              */
+    double  f32_gemm_ms;     /* FP32 Gauss-Jordan updates, and the panels beside them      */
+    double  slice_ms;        /* operand slicing kernels                                    */
     double  phase_sr_ms;     /* whole Sancho-Rubio phases                                  */
     double  phase_rgf_ms;    /* whole RGF sweeps (including their inverses)                */
     double  phase_inv_ms;    /* all inverses (Sancho-Rubio and RGF)                        */

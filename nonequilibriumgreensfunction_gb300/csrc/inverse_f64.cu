@@ -8,7 +8,8 @@
 //
 // Per panel K = [k0, k0+nb), nb = 8 in FP64 up to n = 1024 and 32 otherwise:
 //   1. gj_panel:   one CTA per matrix (in FP64 a cluster of eight for a few matrices)
-//                  factorises the n x nb panel in shared memory or registers (pivot = first max of |re|+|im| over rows >= k, as LAPACK izamax).
+//                  factorises the n x nb panel in shared memory or registers
+//                  (pivot = first max of |re|+|im| over rows >= k, as LAPACK izamax).
 //   2. gj_swap:    applies the panel's row interchanges to the other columns, copies
 //                  their rows K into R (nb x n) and zeroes them.
 //   3. gj_update:  A(:, not K) += P * R(:, not K), P = A(:, K) (the factorised panel).
