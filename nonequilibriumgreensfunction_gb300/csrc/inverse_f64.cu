@@ -1252,7 +1252,8 @@ int sm_count_cached() {
 int gj_invert_fused_f32(float2* A, long long sA, int n, int batch, InvWork& w, cudaStream_t st) {
   const size_t smem = gj_fused_smem(n);
   w.columns_pending = false;
-  NEGF_CUDA_TRY(cudaFuncSetAttribute(gj_fused_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  NEGF_CUDA_TRY(cudaFuncSetAttribute(gj_fused_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)gj_fused_smem(FUSED_MAX_N)));
   NEGF_CUDA_TRY(cudaMemsetAsync(w.info, 0, sizeof(int) * batch, st));
   cudaEvent_t ev;
   timed_begin(st, TK_F32, 8.0 * (double)n * n * n * batch, &ev);
@@ -1306,8 +1307,8 @@ int gj_invert(T* A, long long sA, int n, int batch, InvWork& w, cudaStream_t st)
         pdl_launch(panel, batch, threads, 0, st, reinterpret_cast<float2*>(A), sA, n, k0, kb, w.ipiv, w.info, w.moves,
                    w.orig, w.tickets);
       } else if (sizeof(T) == 16 && clustered) {
+        // an eighth of a panel and of a column: at most 32 KB of what panel_width allows, no opt-in
         const size_t csmem = sizeof(double2) * (size_t)((n + CLP_CTAS - 1) / CLP_CTAS) * (kb + 1);
-        NEGF_CUDA_TRY(cudaFuncSetAttribute(gj_panel_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)csmem));
         pdl_launch_cluster(dim3(CLP_CTAS), gj_panel_cluster_kernel, batch * CLP_CTAS, CLP_THREADS, csmem, st,
                            reinterpret_cast<double2*>(A), sA, n, k0, kb, w.ipiv, w.info);
       } else {

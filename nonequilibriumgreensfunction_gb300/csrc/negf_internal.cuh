@@ -127,6 +127,10 @@ void timed_begin(cudaStream_t st, int kind, double flops, cudaEvent_t* a);
 void timed_end(cudaStream_t st, int kind, cudaEvent_t a);
 void instrument_resolve();   // accumulate the elapsed times of finished event pairs
 
+// A kernel's dynamic shared memory beyond 48 KB is allowed by a limit of the function, one for the
+// whole process, and handles launch from several threads: each launch sets it to the most that its
+// kernel can be asked for and not to its own size, which another thread's launch may exceed.
+
 // ----------------------------------------------------------------------------------
 // Dependent launches.  A solve is thousands of kernels of a few microseconds, each waiting for
 // the one before.  pdl_launch lets the device prepare a kernel's launch while its predecessor

@@ -276,6 +276,7 @@ __global__ void poisson_rhs_kernel(int nx, int ny, int nz, int grids, const doub
 // CTA per grid still has an SM to itself: 40 grids of 60 x 12 x 12 take 2.7 against 5.1 ms, 80
 // grids 5.5 against 5.4 ms, 64 grids of 16 x 8 x 8 1.17 against 1.09 ms.
 constexpr int PCL_MAX_GRIDS = 40;
+constexpr int PCL_SMEM_MAX = 200 * 1024;
 
 // *done: launched; otherwise the grids do not fit clusters
 int launch_clustered(int nx, int ny, int nz, int grids, const double* b, double* u, double tol, int max_iter, int* iters,
@@ -283,8 +284,8 @@ int launch_clustered(int nx, int ny, int nz, int grids, const double* b, double*
   const long long n = (long long)nx * ny * nz;
   const long long per = (n + PCG_THREADS - 1) / PCG_THREADS * PCL_T;
   const long long smem = per * (4 * (long long)sizeof(double) + 1);
-  if (grids > PCL_MAX_GRIDS || smem > 200 * 1024) return NEGF_OK;
-  NEGF_CUDA_TRY(cudaFuncSetAttribute(poisson_cg_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (grids > PCL_MAX_GRIDS || smem > PCL_SMEM_MAX) return NEGF_OK;
+  NEGF_CUDA_TRY(cudaFuncSetAttribute(poisson_cg_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PCL_SMEM_MAX));
   NEGF_CUDA_TRY(cudaFuncSetAttribute(poisson_cg_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)(grids * PCL_CTAS));

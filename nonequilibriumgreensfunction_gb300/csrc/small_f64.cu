@@ -480,9 +480,13 @@ __global__ void __launch_bounds__(SMALL_THREADS) small_rgf_kernel(SmallRgf a) {
   sync_all<CS>();
 }
 
+// nblocks: M x M blocks of a CTA
 template <typename K, typename A>
-int launch(K kernel, int cs, int count, size_t smem, const A& a, cudaStream_t st) {
-  NEGF_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+int launch(K kernel, int cs, int count, int nblocks, const A& a, cudaStream_t st) {
+  const size_t block = sizeof(double2) * nblocks;
+  const size_t smem = block * a.n * a.n;
+  NEGF_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)(block * SMALL_MAX_M * SMALL_MAX_M)));
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)(count * cs));
   cfg.blockDim = dim3(SMALL_THREADS);
@@ -512,9 +516,9 @@ int cluster_size(int n, int count) {
 }
 
 template <typename A>
-int launch_sized(int cs, int count, size_t smem, const A& a, cudaStream_t st, void (*k1)(A), void (*k2)(A),
+int launch_sized(int cs, int count, int nblocks, const A& a, cudaStream_t st, void (*k1)(A), void (*k2)(A),
                  void (*k4)(A), void (*k8)(A)) {
-  return launch(cs == 8 ? k8 : cs == 4 ? k4 : cs == 2 ? k2 : k1, cs, count, smem, a, st);
+  return launch(cs == 8 ? k8 : cs == 4 ? k4 : cs == 2 ? k2 : k1, cs, count, nblocks, a, st);
 }
 
 }  // namespace
@@ -522,12 +526,12 @@ int launch_sized(int cs, int count, size_t smem, const A& a, cudaStream_t st, vo
 int small_sr_steps() { return SR_STEPS; }
 
 int small_sr(const SmallSr& a, cudaStream_t st) {
-  return launch_sized(cluster_size(a.n, a.count), a.count, sizeof(double2) * SR_BLOCKS * (size_t)a.n * a.n, a, st,
+  return launch_sized(cluster_size(a.n, a.count), a.count, SR_BLOCKS, a, st,
                       small_sr_kernel<1>, small_sr_kernel<2>, small_sr_kernel<4>, small_sr_kernel<8>);
 }
 
 int small_rgf(const SmallRgf& a, int count, cudaStream_t st) {
-  return launch_sized(cluster_size(a.n, count), count, sizeof(double2) * RGF_BLOCKS * (size_t)a.n * a.n, a, st,
+  return launch_sized(cluster_size(a.n, count), count, RGF_BLOCKS, a, st,
                       small_rgf_kernel<1>, small_rgf_kernel<2>, small_rgf_kernel<4>, small_rgf_kernel<8>);
 }
 

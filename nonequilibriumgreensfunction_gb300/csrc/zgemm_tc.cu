@@ -1086,7 +1086,8 @@ int slice_a_t(const double2* A, int lda, long long sA, int m, int k, int batch, 
   if (2 * out.k > 1600) return NEGF_EINVAL;   // as the products; a CTA's rows fit its shared memory
   const size_t smem = (size_t)SA_ROWS * out.k * sizeof(double2);
   if (smem > 48 * 1024)
-    NEGF_CUDA_TRY(cudaFuncSetAttribute(slice_a_kernel<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    NEGF_CUDA_TRY(cudaFuncSetAttribute(slice_a_kernel<S>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)(SA_ROWS * 800 * sizeof(double2))));
   cudaEvent_t ev;
   timed_begin(st, TK_SLICE, 0.0, &ev);
   pdl_launch(slice_a_kernel<S>, dim3((m + SA_ROWS - 1) / SA_ROWS, batch), 256, smem, st, A, lda, sA, m, k, out.exps,
