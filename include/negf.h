@@ -130,7 +130,9 @@ NEGF_API int  negf_device_bytes(const negf_handle* h, int64_t* bytes);
  * host without a device (the admission unit of the serving layer: the Npx*M^2*16-byte
  * block store per batch entry plus the Hamiltonian slots and work buffers).  No reference
  * counterpart: the reference allocates its arrays per rank at start-up
- * (Source/Read_In_Allocate.F90:104-238).  NEGF_EINVAL for parameters negf_create refuses. */
+ * (Source/Read_In_Allocate.F90:104-238).  On a device short of memory the FP64 form takes a
+ * smaller tensor-core workspace instead of failing, and negf_device_bytes of that handle is
+ * less than this.  NEGF_EINVAL for parameters negf_create refuses.                      */
 NEGF_API int  negf_estimate_device_bytes(const negf_params* p, int64_t* bytes);
 
 /* Run the handle's work on a caller-owned CUDA stream (cudaStream_t passed as void*);
@@ -335,7 +337,10 @@ NEGF_API int negf_solve_batch_ex(negf_handle* h, const negf_request* req, int32_
  * their energy points are packed, with those of every other admitted request of the same
  * geometry, into the next device batch (continuous batching).  Each geometry is served by
  * its own worker thread and CUDA stream, so work of different geometries overlaps on the
- * device.  A request's results do not depend on what it was batched with.               */
+ * device.  A request's results do not depend on what it was batched with, nor on how much
+ * workspace the budget left its engine; only an FP64 engine whose budget (or device) does not
+ * hold one matrix's tensor-core workspace, 324 M^2 bytes, works on the FP64 pipe and rounds
+ * differently.                                                                          */
 typedef struct negf_server negf_server;
 
 typedef struct negf_serve_params {

@@ -225,7 +225,7 @@ int Engine::configure(const negf_params& p) {
   // BF16 slice pairs some twenty times that (a sweep of M = 400: 1155 -> 116 ms); at M = 2 the
   // launches of the sliced path cost more than they save (46 against 28 ms an energy).
   const bool one_kernel = M_ <= SMALL_MAX_M && !currents_ && !keep_columns_ && p.contact_type != NEGF_CONTACT_SC;
-  if (!mixed_ && !lean_ && !one_kernel && M_ >= 32 && 2 * padded_k(M_) <= 1600) {
+  if (!mixed_ && tc_limit_ > 0 && !one_kernel && M_ >= 32 && 2 * padded_k(M_) <= 1600) {
     // Each step's residual is as fine as the step's result has to be: FP32 Gauss-Jordan leaves
     // ~1e-3, and the steps ~1e-7, ~1e-12 and the rounding of a double.
     tc_ = true;
@@ -237,16 +237,17 @@ int Engine::configure(const negf_params& p) {
     ns_steps_ = 3;
     ns_max_steps_ = 6;
     ns_tol_ = 1e-9;   // squared by the last update: below a double's rounding
-    // about 300 M^2 bytes a matrix: at most some 3 GB of workspace, and at least 32 matrices
+    // up to 324 M^2 bytes a matrix: some 3 GB of workspace, or 32 matrices where these are more
+    // (6.6 GB at M = 800); tc_limit_ lowers it
     const long long fit = 10000000 / std::max<long long>(MM_, 1);
-    tc_cap_ = (int)std::min<long long>(tc_cap_, std::max<long long>(fit, 32));
+    tc_cap_ = (int)std::min<long long>(std::min(tc_cap_, tc_limit_), std::max<long long>(fit, 32));
   }
   return NEGF_OK;
 }
 
-long long Engine::estimate_bytes(const negf_params& p, bool lean) {
+long long Engine::estimate_bytes(const negf_params& p, int tc_limit) {
   Engine e;
-  e.lean_ = lean;
+  e.tc_limit_ = tc_limit;
   if (e.configure(p) != NEGF_OK) return -1;
   e.dry_ = true;
   if (e.alloc() != NEGF_OK) return -1;
@@ -329,15 +330,20 @@ int Engine::alloc() {
               gj_next_bytes(M_, cap);
   }
   if (tc_) {
+    // Without room for it, first the blocks that the pool keeps go back to the device; then the
+    // FP64 form takes a smaller one, which changes no result, and runs on the FP64 pipe only when
+    // the device does not even hold one matrix's.
     const long long before = bytes_;
     int rc = alloc_tc();
-    if (rc == NEGF_ENOMEM && !mixed_) {   // the FP64 form runs without it
+    for (bool trimmed = false; rc == NEGF_ENOMEM && !mixed_ && tc_; trimmed = true) {
       free_tc();
       NEGF_CUDA_TRY(cudaStreamSynchronize(own_st_));
       cudaGetLastError();   // (the failed allocation)
       bytes_ = before;
-      tc_ = false;
-      rc = NEGF_OK;
+      if (!trimmed) NEGF_TRY(pool_trim(p_.device));
+      else if (tc_cap_ > 1) tc_cap_ /= 2;
+      else tc_ = false;
+      rc = tc_ ? alloc_tc() : NEGF_OK;
     }
     NEGF_TRY(rc);
   }
@@ -559,7 +565,7 @@ int Engine::gemm_tc_nn(int batch, const double2* A, long long sA, const double2*
 }
 
 // C = A G with G's B-operand slicing made once per sweep (Gamma_L, Gamma_R); without the
-// tensor cores, or for a batch in pieces, a plain product with G itself
+// tensor cores a plain product; a batch in pieces slices G again, for the same bits
 int Engine::gemm_gamma(int batch, const double2* A, long long sA, const double2* G, const SlicedOperand& sg,
                        double2* C, long long sC) {
   const double2 one = make_double2(1, 0), zero = make_double2(0, 0);

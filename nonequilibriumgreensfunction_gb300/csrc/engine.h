@@ -34,10 +34,12 @@ class Engine {
   int init(const negf_params& p);
   // device bytes an engine with these parameters allocates at init (< 0: invalid
   // parameters); the serving layer admits engines by it
-  static long long estimate_bytes(const negf_params& p, bool lean = false);
-  // before init: an FP64 engine without the tensor-core workspace (DFMA products and FP64
-  // inverses), for a budget that does not hold the other
-  void set_lean() { lean_ = true; }
+  static long long estimate_bytes(const negf_params& p, int tc_limit = kTcNoLimit);
+  // before init: an FP64 engine whose tensor-core workspace holds at most `matrices` matrices, for a
+  // budget that does not hold the whole; larger batches go through it in pieces, with the same
+  // results.  0: no workspace, DFMA products and FP64 inverses, which round differently.
+  static constexpr int kTcNoLimit = 1 << 30;
+  void limit_tc(int matrices) { tc_limit_ = matrices; }
   int set_hamiltonian(int slot, const double* Htotd, const double* HopX);
   // Htotd of `slot` generated on the device from a wire model (Build_Hamiltonian)
   int build_hamiltonian(int slot, const negf_wire_model& m);
@@ -156,7 +158,7 @@ class Engine {
   // holds) and three steps, for M <= 800 when its workspace fits the device.
   bool mixed_ = false;
   bool tc_ = false;
-  bool lean_ = false;        // FP64 form: no workspace for it
+  int tc_limit_ = kTcNoLimit;   // FP64 form: most matrices of its workspace
   int tc_cap_ = 0;           // matrices of one sliced product or inverse; larger batches go in pieces
   int s_rgf_ = 5;      // RGF block products
   int s_sr_ = 8;       // Sancho-Rubio products: 2^-56, the decimation is ill-conditioned near band edges

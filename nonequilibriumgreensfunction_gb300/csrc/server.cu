@@ -114,9 +114,10 @@ struct negf_server {
 
   // an engine's device bytes: Engine::alloc counted without allocating, plus 64 MB for the
   // allocator's rounding and the library's per-context state
+  static constexpr long long kEngineSlack = 64LL << 20;
   long long estimate(const GeomKey& k) const {
     const long long b = negf::Engine::estimate_bytes(engine_params(k));
-    return b < 0 ? b : b + (64LL << 20);
+    return b < 0 ? b : b + kEngineSlack;
   }
 
   // Destroy idle workers (no admitted requests, not running a batch) until `need` bytes
@@ -167,10 +168,15 @@ struct negf_server {
         w = wi->second.get();
       } else {
         long long need = estimate(r->key);
-        bool lean = false;
-        if (need > budget) {   // an FP64 engine also runs without its tensor-core workspace
-          const long long least = negf::Engine::estimate_bytes(engine_params(r->key), true);
-          if (least >= 0 && least <= budget) { need = least; lean = true; }
+        int tc_limit = negf::Engine::kTcNoLimit;
+        if (need > budget) {
+          // an FP64 engine's results do not depend on how many matrices its tensor-core workspace
+          // holds, and it runs on the FP64 pipe without it
+          const negf_params ep = engine_params(r->key);
+          for (tc_limit = 2 * ep.max_batch; tc_limit > 0 && need > budget; ) {
+            tc_limit /= 2;
+            need = negf::Engine::estimate_bytes(ep, tc_limit) + (tc_limit > 0 ? kEngineSlack : 0);
+          }
         }
         if (need < 0 || need > budget) {
           // a geometry no engine accepts (e.g. M > 800 in the mixed form), or one whose
@@ -195,14 +201,14 @@ struct negf_server {
           auto nw = std::make_unique<Worker>();
           nw->key = r->key;
           nw->eng = std::make_unique<negf::Engine>();
-          if (lean) nw->eng->set_lean();
+          nw->eng->limit_tc(tc_limit);
           const double t0 = now();
           int irc = nw->eng->init(engine_params(r->key));
           if (irc == NEGF_ENOMEM) {
             // the library's pool keeps released engines' blocks for reuse; when they do not
             // fit this engine's buffers, give them back to the device and try once more
             nw->eng = std::make_unique<negf::Engine>();
-            if (lean) nw->eng->set_lean();
+            nw->eng->limit_tc(tc_limit);
             negf::pool_trim(p.device);
             irc = nw->eng->init(engine_params(r->key));
           }

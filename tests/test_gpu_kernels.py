@@ -168,3 +168,19 @@ def test_inverses_do_not_depend_on_the_batch(need_gpu, npy, npz):
     some = np.r_[0:4, 78:82, 156:160]
     for k, v in out[0].items():
         assert np.array_equal(v[some], out[1][k]), k
+
+
+# The FP64 form's tensor-core workspace holds at most max(32, 10^7 / M^2) matrices: larger batches go
+# through it in pieces (M = 400: 62 matrices; M = 576: 32), which no result shows.
+@pytest.mark.parametrize("npy,npz,n", [(10, 10, 64), (12, 12, 33)])
+def test_fp64_batches_beyond_the_workspace_give_the_same_bits(need_gpu, npy, npz, n):
+    model = hamiltonian.wire_model(W=0.1, seed=3, flux=0.4, zeeman=0.01)
+    energies = np.linspace(-0.3, 0.3, n)
+    pick = np.r_[0, n // 2, n - 1]
+    out = []
+    for e in (energies, energies[pick]):
+        with Solver(2, npy, npz, eta=1e-2, sr_tol=1e-6, max_batch=len(e)) as s:
+            s.build_hamiltonian(model)
+            out.append(s.solve_batch(e, 0.7, 0.2, 1e-3))
+    for k, v in out[1].items():
+        assert np.array_equal(out[0][k][pick], v), k
