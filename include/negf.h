@@ -153,7 +153,8 @@ typedef struct negf_stats {
     double  tc_ms;
     double  tc_flops;        /* BF16 tensor flops issued: S(S+1)/2 slice pairs x 8*m*n*k   */
     double  tc_complex_flops;/* the complex products they compute, 8*m*n*k                 */
-    int64_t fallbacks;       /* refined inverses redone in FP64 (residual too large)       */
+    int64_t fallbacks;       /* refined inverses redone in FP64 (residual too large); FP64
+                                form: also leads and energies solved again on the FP64 pipe */
     double  ns_residual_max; /* largest accepted first Newton-Schulz residual              */
     double  f32_gemm_ms;     /* FP32 Gauss-Jordan updates, and the panels beside them      */
     double  slice_ms;        /* operand slicing kernels                                    */

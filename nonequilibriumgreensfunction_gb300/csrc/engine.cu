@@ -168,6 +168,7 @@ void Engine::free_tc() {
   dfree(sb_.exps, s); dfree(sw_.data, s); dfree(sw_.exps, s); dfree(sgl_.data, s); dfree(sgl_.exps, s);
   dfree(sgr_.data, s); dfree(sgr_.exps, s);
   dfree(dRnorm_, s); dfree(dNsIdx_, s); dfree(dNsX_, s); dfree(dNsW_, s); dfree(dTcErr_, s);
+  dfree(dGraded_, s);
 }
 
 int pool_trim(int device) {
@@ -318,7 +319,7 @@ int Engine::alloc() {
   double2** srb[] = {&dSrSigL_, &dSrSigR_, &dSrGamL_, &dSrGamR_};
   for (double2** b : srb) NEGF_TRY(dalloc(b, (size_t)(S_ * MM_), bytes_, dry_, pool_, own_st_));
   NEGF_TRY(dalloc(&dSrCmax_, (size_t)2 * S_, bytes_, dry_, pool_, own_st_));
-  NEGF_TRY(dalloc(&dSrDos_, (size_t)2 * S_, bytes_, dry_, pool_, own_st_));
+  NEGF_TRY(dalloc(&dSrDos_, (size_t)4 * S_, bytes_, dry_, pool_, own_st_));   // and as many of leads solved again
   NEGF_TRY(dalloc(&dSrActive_, (size_t)8 * S_, bytes_, dry_, pool_, own_st_));
   NEGF_TRY(dalloc(&dSrE_, (size_t)S_, bytes_, dry_, pool_, own_st_));
   NEGF_TRY(dalloc(&dSrHend_, (size_t)S_, bytes_, dry_, pool_, own_st_));
@@ -356,7 +357,7 @@ int Engine::alloc() {
     const size_t cap = (size_t)std::max(B_, S_);
     double* p = nullptr;
     NEGF_TRY(pinned_take(sizeof(double) * (2 * (size_t)S_ + 5 * (size_t)B_ + 2 * cap) +
-                             sizeof(int) * (cap + 4 * (size_t)S_ + (size_t)B_ + 2), &p, &hSmallBytes_));
+                             sizeof(int) * (cap + 6 * (size_t)S_ + (size_t)B_ + 2), &p, &hSmallBytes_));
     hSmall_ = p;
     hDos_ = p;
     hTr_ = hDos_ + 2 * (size_t)S_;
@@ -368,6 +369,7 @@ int Engine::alloc() {
     hRst_ = hSr_ + 4 * (size_t)S_;
     hErr_ = hRst_ + B_;
     *hErr_ = 0;
+    hGraded_ = hErr_ + 2;
   }
   // the allocations are ordered on the engine's stream; after this they are usable from
   // any stream (the caller's, through negf_set_stream) and by the synchronous copies below
@@ -437,6 +439,7 @@ int Engine::alloc_tc() {
   NEGF_TRY(dalloc(&dNsX_, (size_t)cap * MM_, bytes_, dry_, pool_, own_st_));
   NEGF_TRY(dalloc(&dNsW_, (size_t)cap * MM_, bytes_, dry_, pool_, own_st_));
   NEGF_TRY(dalloc(&dTcErr_, (size_t)1, bytes_, dry_, pool_, own_st_));
+  if (!mixed_) NEGF_TRY(dalloc(&dGraded_, (size_t)2 * S_, bytes_, dry_, pool_, own_st_));
   if (!dry_) NEGF_CUDA_TRY(cudaMemsetAsync(dTcErr_, 0, sizeof(int), own_st_));
   return NEGF_OK;
 }
@@ -787,10 +790,55 @@ int Engine::set_refinement(int max_steps, double tol, double accept) {
 int Engine::solve_sr(const std::vector<SrJob>& jobs, std::vector<int>& status, std::vector<int>& iters) {
   cudaEvent_t ph;
   timed_begin(st_, TK_PH_SR, 0.0, &ph);
-  const int rc = p_.contact_type == NEGF_CONTACT_LEADS ? solve_sr_impl(jobs, status, iters)
-                                                       : solve_contact_model(jobs, status, iters);
+  int rc = p_.contact_type == NEGF_CONTACT_LEADS ? solve_sr_impl(jobs, status, iters)
+                                                 : solve_contact_model(jobs, status, iters);
+  if (rc == NEGF_OK && tc_ && !mixed_ && p_.contact_type == NEGF_CONTACT_LEADS)
+    rc = redo_graded_leads(jobs, status, iters);
   timed_end(st_, TK_PH_SR, ph);
   return rc;
+}
+
+// The nine-slice products and the refined inverses are as exact as FP64 relative to the largest
+// entries of a row and a column.  FP64 itself is relative to each term, so that a site that hardly
+// couples to the others (behind a wall of high potential, or many decay lengths inside a gap) keeps
+// its digits however small its amplitudes are, where slices lose them: a wire with walls of 1e8 eV
+// had densities that were wrong in the first digit where they were 1e-40 of the others'.  So
+// a lead or an energy whose sites' amplitudes are further apart than 2^14 is solved again on the FP64
+// pipe, as every wire was that has no workspace for the slices.  At 2^14 the slices' rounding, 2^-63
+// of the largest amplitude with the growth of a product's sum, is about that of the FP64 path's chain
+// of products (some 1e-13).  The choice is the energy's own: it does not depend on its batch.
+constexpr double kGradedAmplitudes = 16384.0;
+
+int Engine::redo_graded_leads(const std::vector<SrJob>& jobs, std::vector<int>& status, std::vector<int>& iters) {
+  const int S = (int)jobs.size();
+  if (S == 0) return NEGF_OK;
+  auto graded = [&](int s) { return (jobs[s].want_l && hGraded_[s]) || (jobs[s].want_r && hGraded_[S + s]); };
+  double2** const blocks[] = {&dSrSigL_, &dSrSigR_, &dSrGamL_, &dSrGamR_};
+  for (int a = 0, e = 0; a < S; a = e + 1) {   // runs [a, e) of them, in the order of the leads
+    for (e = a; e < S && graded(e);) ++e;
+    if (e == a) continue;
+    const int k = e - a;
+    std::vector<int> st, its;
+    double* const dos = dSrDos_;
+    for (double2** p : blocks) *p += a * MM_;
+    dSrDos_ = dos + 2 * S_;
+    tc_ = false;
+    const int rc = solve_sr_impl(std::vector<SrJob>(jobs.begin() + a, jobs.begin() + e), st, its);
+    tc_ = true;
+    for (double2** p : blocks) *p -= a * MM_;
+    dSrDos_ = dos;
+    NEGF_TRY(rc);
+    for (int lead = 0; lead < 2; ++lead)
+      NEGF_CUDA_TRY(cudaMemcpyAsync(dos + lead * S + a, dos + 2 * S_ + lead * k, sizeof(double) * k,
+                                    cudaMemcpyDeviceToDevice, st_));
+    for (int s = 0; s < k; ++s) {
+      status[a + s] = st[s];
+      iters[a + s] = its[s];
+      iters[S + a + s] = its[k + s];
+    }
+    fallbacks_ += k;
+  }
+  return NEGF_OK;
 }
 
 int Engine::solve_sr_impl(const std::vector<SrJob>& jobs, std::vector<int>& status, std::vector<int>& iters) {
@@ -959,6 +1007,10 @@ int Engine::solve_sr_impl(const std::vector<SrJob>& jobs, std::vector<int>& stat
   }
   const int* st = hSr_;
   NEGF_CUDA_TRY(cudaMemcpyAsync(hSr_, dSrStatus_, sizeof(int) * S, cudaMemcpyDeviceToHost, st_));
+  if (tc_ && !mixed_) {   // for redo_graded_leads
+    NEGF_TRY(graded_rows(M_, p_.norb, S, dSrSigL_, dSrSigR_, MM_, kGradedAmplitudes, dGraded_, st_));
+    NEGF_CUDA_TRY(cudaMemcpyAsync(hGraded_, dGraded_, sizeof(int) * 2 * S, cudaMemcpyDeviceToHost, st_));
+  }
   NEGF_TRY(read_tc_error());
   NEGF_CUDA_TRY(cudaStreamSynchronize(st_));
   if (*hErr_) return NEGF_ETIMEDOUT;
@@ -1066,9 +1118,55 @@ int Engine::solve_contact_model(const std::vector<SrJob>& jobs, std::vector<int>
 int Engine::solve_rgf(const std::vector<Item>& items, bool keep_columns) {
   cudaEvent_t ph;
   timed_begin(st_, TK_PH_RGF, 0.0, &ph);
-  const int rc = solve_rgf_impl(items, keep_columns);
+  int rc = solve_rgf_impl(items, keep_columns);
+  if (rc == NEGF_OK && tc_ && !mixed_) rc = redo_graded_items(items, keep_columns);
   timed_end(st_, TK_PH_RGF, ph);
   return rc;
+}
+
+int Engine::redo_graded_items(const std::vector<Item>& items, bool keep_columns) {
+  const int B = (int)items.size();
+  if (B == 0) return NEGF_OK;
+  const long long sP = (long long)p_.npx * M_ * p_.norb, sD = (long long)M_ * p_.norb;
+  NEGF_TRY(graded_sites(M_, p_.norb, p_.npx, B, dP1_, dP2_, sP, kGradedAmplitudes * kGradedAmplitudes, dGraded_, st_));
+  NEGF_CUDA_TRY(cudaMemcpyAsync(hGraded_, dGraded_, sizeof(int) * B, cudaMemcpyDeviceToHost, st_));
+  NEGF_CUDA_TRY(cudaStreamSynchronize(st_));
+  // what a sweep leaves for each item (without currents or SC contacts some are null)
+  double2** const blocks[] = {&dP1_, &dP2_, &dPx1_, &dPy1_, &dPz1_, &dPx2_, &dPy2_, &dPz2_};
+  bool any = false;
+  for (int a = 0, e = 0; a < B; a = e + 1) {   // runs [a, e) of them
+    for (e = a; e < B && hGraded_[e];) ++e;
+    if (e == a) continue;
+    any = true;
+    for (double2** p : blocks) *p = *p ? *p + a * sP : nullptr;
+    double2* const g11 = dG11_;
+    dG11_ = g11 ? g11 + a * sD : nullptr;
+    dTr_ += 4 * a;
+    dStatus_ += a;
+    tc_ = false;
+    const int rc = solve_rgf_impl(std::vector<Item>(items.begin() + a, items.begin() + e), keep_columns && a == 0);
+    tc_ = true;
+    for (double2** p : blocks) *p = *p ? *p - a * sP : nullptr;
+    dG11_ = g11;
+    dTr_ -= 4 * a;
+    dStatus_ -= a;
+    NEGF_TRY(rc);
+    fallbacks_ += e - a;
+  }
+  if (!any) return NEGF_OK;
+  // the items and their self-energies are the whole batch's again
+  NEGF_CUDA_TRY(cudaMemcpyAsync(dItems_, items.data(), sizeof(Item) * B, cudaMemcpyHostToDevice, st_));
+  return gather_contacts(B);
+}
+
+int Engine::gather_contacts(int batch) {
+  const int istride = (int)(sizeof(Item) / sizeof(int));
+  const int* idx_l = reinterpret_cast<const int*>(reinterpret_cast<const char*>(dItems_) + offsetof(Item, sr_l));
+  const int* idx_r = reinterpret_cast<const int*>(reinterpret_cast<const char*>(dItems_) + offsetof(Item, sr_r));
+  NEGF_TRY(gather_blocks(M_, batch, dSrSigL_, idx_l, istride, dSigL_, MM_, st_));
+  NEGF_TRY(gather_blocks(M_, batch, dSrSigR_, idx_r, istride, dSigR_, MM_, st_));
+  NEGF_TRY(gather_blocks(M_, batch, dSrGamL_, idx_l, istride, dGamL_, MM_, st_));
+  return gather_blocks(M_, batch, dSrGamR_, idx_r, istride, dGamR_, MM_, st_);
 }
 
 int Engine::solve_rgf_impl(const std::vector<Item>& items, bool keep_columns) {
@@ -1091,13 +1189,7 @@ int Engine::solve_rgf_impl(const std::vector<Item>& items, bool keep_columns) {
     a.G = dG_; a.P1 = dP1_; a.P2 = dP2_; a.traces = dTr_; a.status = dStatus_;
     return small_rgf(a, B, st_);
   }
-  const int istride = (int)(sizeof(Item) / sizeof(int));
-  const int* idx_l = reinterpret_cast<const int*>(reinterpret_cast<const char*>(dItems_) + offsetof(Item, sr_l));
-  const int* idx_r = reinterpret_cast<const int*>(reinterpret_cast<const char*>(dItems_) + offsetof(Item, sr_r));
-  NEGF_TRY(gather_blocks(M_, B, dSrSigL_, idx_l, istride, dSigL_, sM, st_));
-  NEGF_TRY(gather_blocks(M_, B, dSrSigR_, idx_r, istride, dSigR_, sM, st_));
-  NEGF_TRY(gather_blocks(M_, B, dSrGamL_, idx_l, istride, dGamL_, sM, st_));
-  NEGF_TRY(gather_blocks(M_, B, dSrGamR_, idx_r, istride, dGamR_, sM, st_));
+  NEGF_TRY(gather_contacts(B));
   if (tc_ && B <= tc_cap_) {   // Gamma is the right factor of every G(:,c) Gamma_c product of the sweep
     NEGF_TRY(slice_b(dGamL_, M_, sM, M_, M_, B, s_rgf_, sgl_, st_));
     NEGF_TRY(slice_b(dGamR_, M_, sM, M_, M_, B, s_rgf_, sgr_, st_));

@@ -149,6 +149,7 @@ class Engine {
   double *hDos_ = nullptr, *hTr_ = nullptr, *hTrJ_ = nullptr;     // [2 S_], [4 B_], [B_]
   unsigned long long *hR0_ = nullptr, *hRk_ = nullptr;            // [cap] residual norms of an inverse
   int *hInfo_ = nullptr, *hSr_ = nullptr, *hRst_ = nullptr, *hErr_ = nullptr;   // [cap], [4 S_], [B_], [1]
+  int* hGraded_ = nullptr;                                                      // [2 S_]
 
   InvWork inv_;
 
@@ -186,6 +187,8 @@ class Engine {
   long long ns_unconverged_ = 0;   // matrices still above ns_tol_ after ns_max_steps_ (redone in FP64)
   double last_rk_max_ = 0.0;       // largest residual norm before the last update of an accepted matrix
   int* dTcErr_ = nullptr;
+  // FP64 form: results whose sites are too far apart for the slices are solved again on the FP64 pipe
+  int* dGraded_ = nullptr;         // [2 S_]
   long long fallbacks_ = 0;
   double last_rnorm_max_ = 0.0;
   // Newton-Schulz policy of the mixed form (negf_set_refinement); <= 0 restores a default
@@ -202,6 +205,9 @@ class Engine {
   bool small_() const { return !mixed_ && !tc_ && M_ <= SMALL_MAX_M; }
   int solve_sr_small(const std::vector<SrJob>& jobs, std::vector<int>& status, std::vector<int>& iters);
   int solve_rgf_impl(const std::vector<Item>& items, bool keep_columns);
+  int redo_graded_leads(const std::vector<SrJob>& jobs, std::vector<int>& status, std::vector<int>& iters);
+  int redo_graded_items(const std::vector<Item>& items, bool keep_columns);
+  int gather_contacts(int batch);   // the items' self-energies and Gammas from the decimation's
   int densities_impl(const std::vector<Item>& items, std::vector<double>& edens, std::vector<double>& hdens);
   HopBD hop() const {
     HopBD h;

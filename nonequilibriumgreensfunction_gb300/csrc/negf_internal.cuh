@@ -362,6 +362,13 @@ struct SmallRgf {
 };
 int small_rgf(const SmallRgf& a, int count, cudaStream_t st);
 
+// flag[b] = 1 where the sites of a slice (their densities), or of a matrix (the largest entries of their
+// rows; those of A0, then those of A1), are further apart than `range`
+int graded_sites(int n, int norb, int npx, int batch, const double2* P1, const double2* P2, long long sP, double range,
+                 int* flag, cudaStream_t st);
+int graded_rows(int n, int norb, int batch, const double2* A0, const double2* A1, long long sA, double range, int* flag,
+                cudaStream_t st);
+
 // density / spin from the site blocks of both leads.  P1, P2: [item][x][n][norb].
 // site_out: [item][nf][npx*npy*npz], fields 0..4 = (RhoN, RhoP, SigX, SigY, SigZ) already
 // weighted by dE/(2 pi) (fields 5..7 = Jx, Jy, Jz when nf = 8, bond_currents);

@@ -595,6 +595,70 @@ __global__ void __launch_bounds__(RED_THREADS) gamma_dos_kernel(int n, const dou
   if (threadIdx.x == 0) dos[b] = -red[0] / 3.14159265358979323846;
 }
 
+// ---- how far apart the sites of a slice are -------------------------------------------
+// flag[b] = 1 where the densities |tr P| of a slice's sites, of either lead, are further apart than
+// `range`.  One CTA per slice and item; memory-latency bound, a few microseconds a sweep.
+constexpr int GRADED_THREADS = 128;
+__device__ __forceinline__ void spread_note(double lo, double hi, double range, int* flag) {
+  __shared__ double low[32], high[32];
+  for (int o = 16; o > 0; o >>= 1) {
+    lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+    hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+  }
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) { low[threadIdx.x >> 5] = lo; high[threadIdx.x >> 5] = hi; }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < (int)blockDim.x / 32; ++w) { lo = fmin(lo, low[w]); hi = fmax(hi, high[w]); }
+    if (hi > range * lo) *flag = 1;
+  }
+}
+__global__ void __launch_bounds__(GRADED_THREADS) graded_sites_kernel(int n, int no, const double2* P1, const double2* P2,
+                                                                      long long sP, double range, int* flag) {
+  pdl_wait();
+  const int b = blockIdx.y;
+  for (int lead = 0; lead < 2; ++lead) {
+    const double2* P = (lead == 0 ? P1 : P2) + (long long)b * sP + (long long)blockIdx.x * n * no;
+    double lo = __longlong_as_double(0x7FF0000000000000LL), hi = 0.0;
+    for (int s = threadIdx.x; s < n / no; s += GRADED_THREADS) {
+      double t = 0.0;
+      for (int a = 0; a < no; ++a) t += P[((long long)s * no + a) * no + a].x;
+      lo = fmin(lo, fabs(t));
+      hi = fmax(hi, fabs(t));
+    }
+    spread_note(lo, hi, range, flag + b);
+  }
+}
+
+// The same of the largest entries of each site's rows of two sets of n x n matrices; a site without any
+// (its hop is zero) does not count.
+constexpr int GRADED_ROWS_THREADS = 1024;
+__global__ void __launch_bounds__(GRADED_ROWS_THREADS) graded_rows_kernel(int n, int no, int batch, const double2* A0,
+                                                                          const double2* A1, long long sA, double range,
+                                                                          int* flag) {
+  pdl_wait();
+  extern __shared__ unsigned long long site_max[];   // [n / no] bits of |re| + |im|
+  const int b = blockIdx.x;
+  const double2* Ab = b < batch ? A0 + b * sA : A1 + (b - batch) * sA;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5, ns = n / no;
+  for (int s = t; s < ns; s += GRADED_ROWS_THREADS) site_max[s] = 0;
+  __syncthreads();
+  for (int i = lane; i < n; i += 32) {
+    double m = 0.0;
+#pragma unroll 8
+    for (int j = warp; j < n; j += GRADED_ROWS_THREADS / 32) m = fmax(m, cabs1(Ab[(long long)j * n + i]));
+    atomicMax(&site_max[i / no], (unsigned long long)__double_as_longlong(m));
+  }
+  __syncthreads();
+  double lo = __longlong_as_double(0x7FF0000000000000LL), hi = 0.0;
+  for (int s = t; s < ns; s += GRADED_ROWS_THREADS) {
+    const double m = __longlong_as_double((long long)site_max[s]);
+    if (m > 0.0) lo = fmin(lo, m);
+    hi = fmax(hi, m);
+  }
+  spread_note(lo, hi, range, flag + b);
+}
+
 // ---- densities and spin from the site blocks (Calculate_Gnp.F90:117-124,
 //      Calculate_Observables.F90:10-43) -------------------------------------------------
 // One thread per (item, x, site).  Gn_site = f1 P1 + f2 P2, Gp_site = (1-f1) P1 + (1-f2) P2.
@@ -1084,6 +1148,25 @@ int sr_sigma(const HopBD& h, int n, int nprob, int lead, const double2* g, long 
     count_launch();
   }
   pdl_launch(gamma_dos_kernel, nprob, RED_THREADS, 0, st, n, sig, sSig, gam, sGam, dos);
+  NEGF_CUDA_TRY(cudaGetLastError());
+  count_launch();
+  return NEGF_OK;
+}
+
+int graded_sites(int n, int norb, int npx, int batch, const double2* P1, const double2* P2, long long sP, double range,
+                 int* flag, cudaStream_t st) {
+  NEGF_CUDA_TRY(cudaMemsetAsync(flag, 0, sizeof(int) * batch, st));
+  pdl_launch(graded_sites_kernel, dim3(npx, batch), GRADED_THREADS, 0, st, n, norb, P1, P2, sP, range, flag);
+  NEGF_CUDA_TRY(cudaGetLastError());
+  count_launch();
+  return NEGF_OK;
+}
+
+int graded_rows(int n, int norb, int batch, const double2* A0, const double2* A1, long long sA, double range, int* flag,
+                cudaStream_t st) {
+  NEGF_CUDA_TRY(cudaMemsetAsync(flag, 0, sizeof(int) * 2 * batch, st));
+  pdl_launch(graded_rows_kernel, 2 * batch, GRADED_ROWS_THREADS, sizeof(unsigned long long) * (size_t)(n / norb), st, n, norb,
+             batch, A0, A1, sA, range, flag);
   NEGF_CUDA_TRY(cudaGetLastError());
   count_launch();
   return NEGF_OK;
