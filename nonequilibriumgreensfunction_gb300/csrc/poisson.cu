@@ -274,8 +274,12 @@ __global__ void poisson_rhs_kernel(int nx, int ny, int nz, int grids, const doub
 
 // Up to this many grids take a cluster each.  Beyond, the clusters queue for the SMs while one
 // CTA per grid still has an SM to itself: 40 grids of 60 x 12 x 12 take 2.7 against 5.1 ms, 80
-// grids 5.5 against 5.4 ms, 64 grids of 16 x 8 x 8 1.17 against 1.09 ms.
-constexpr int PCL_MAX_GRIDS = 40;
+// grids 5.5 against 5.4 ms, 64 grids of 16 x 8 x 8 1.17 against 1.09 ms.  Small grids are barriers
+// rather than arithmetic and gain less from a cluster, so fewer of them pay for the queue, one CTA
+// against a cluster: 81 sites, 20 grids 0.41 / 0.39 ms, 24 0.41 / 0.43, 40 0.41 / 0.46; 256 sites, 20
+// 0.49 / 0.47, 24 0.50 / 0.51, 40 0.50 / 0.59; 500 sites, 32 0.66 / 0.62, 40 0.66 / 0.68; 1024 sites,
+// 40 1.05 / 0.86.
+constexpr int pcl_max_grids(long long n) { return n < 400 ? 20 : n < 640 ? 32 : 40; }
 constexpr int PCL_SMEM_MAX = 200 * 1024;
 
 // *done: launched; otherwise the grids do not fit clusters
@@ -284,7 +288,7 @@ int launch_clustered(int nx, int ny, int nz, int grids, const double* b, double*
   const long long n = (long long)nx * ny * nz;
   const long long per = (n + PCG_THREADS - 1) / PCG_THREADS * PCL_T;
   const long long smem = per * (4 * (long long)sizeof(double) + 1);
-  if (grids > PCL_MAX_GRIDS || smem > PCL_SMEM_MAX) return NEGF_OK;
+  if (grids > pcl_max_grids(n) || smem > PCL_SMEM_MAX) return NEGF_OK;
   NEGF_CUDA_TRY(cudaFuncSetAttribute(poisson_cg_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PCL_SMEM_MAX));
   NEGF_CUDA_TRY(cudaFuncSetAttribute(poisson_cg_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   cudaLaunchConfig_t cfg{};

@@ -184,3 +184,16 @@ def test_fp64_batches_beyond_the_workspace_give_the_same_bits(need_gpu, npy, npz
             out.append(s.solve_batch(e, 0.7, 0.2, 1e-3))
     for k, v in out[1].items():
         assert np.array_equal(out[0][k][pick], v), k
+
+
+# Grids of fewer than 400 sites take clusters up to 20 at a time, of fewer than 640 up to 32: the same
+# bits and steps on both sides of the lines.
+@pytest.mark.parametrize("shape,most", [((5, 1, 1), 20), ((21, 19, 1), 20), ((20, 20, 1), 32), ((71, 9, 1), 32),
+                                        ((16, 8, 5), 40)])
+def test_poisson_small_grids_on_both_sides_of_the_lines(need_gpu, shape, most):
+    rho = 1e-3 * np.random.default_rng(3).standard_normal(shape + (most + 1,))
+    one_cta, steps = scf.poisson_solve(rho, (0.02, -0.02, 0.1), 1.8)
+    cluster, few = scf.poisson_solve(rho[..., :most], (0.02, -0.02, 0.1), 1.8)
+    last, more = scf.poisson_solve(rho[..., most:], (0.02, -0.02, 0.1), 1.8)
+    assert np.array_equal(one_cta[..., :most], cluster) and np.array_equal(one_cta[..., most:], last)
+    assert max(few, more) == steps
