@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "../../include/negf.h"
+#include "scalar.cuh"
 
 namespace negf {
 

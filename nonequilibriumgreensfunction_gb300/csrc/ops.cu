@@ -504,19 +504,14 @@ __global__ void sr_accumulate_kernel(int n, const int* active, const double2* ch
   double m = 0.0;
   for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < nn; e += (long long)gridDim.x * blockDim.x) {
     const double2 v = c[e];
-    double a = hypot(v.x, v.y);
-    if (isnan(a)) a = __longlong_as_double(0x7FF8000000000000LL);
-    m = (isnan(a) || isnan(m)) ? a : fmax(m, a);
+    const double a = hypot(v.x, v.y);
+    m = max_or_nan(m, a);
     if (act) t[e] = cadd(t[e], v);
   }
   red[threadIdx.x] = m;
   __syncthreads();
   for (int w = EW_THREADS / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) {
-      const double o = red[threadIdx.x + w];
-      red[threadIdx.x] = (isnan(o) || isnan(red[threadIdx.x])) ? __longlong_as_double(0x7FF8000000000000LL)
-                                                                : fmax(red[threadIdx.x], o);
-    }
+    if (threadIdx.x < w) red[threadIdx.x] = max_or_nan(red[threadIdx.x], red[threadIdx.x + w]);
     __syncthreads();
   }
   if (threadIdx.x == 0) atomicMax(cmax + b, (unsigned long long)__double_as_longlong(red[0]));

@@ -298,9 +298,7 @@ __global__ void __launch_bounds__(SMALL_THREADS) small_sr_kernel(SmallSr a) {
       double m = 0.0;
       for (int e = t; e < nn; e += SMALL_THREADS) {
         const double2 v = w1[e];
-        double c = hypot(v.x, v.y);
-        if (isnan(c)) c = __longlong_as_double(0x7FF8000000000000LL);
-        m = (isnan(c) || isnan(m)) ? c : fmax(m, c);
+        m = max_or_nan(m, hypot(v.x, v.y));
         if (act[l]) sum[l][e] = cadd(sum[l][e], v);
       }
       atomicMax(&cmax, (unsigned long long)__double_as_longlong(m));   // (a NaN's bits exceed all others)
