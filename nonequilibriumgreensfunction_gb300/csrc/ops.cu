@@ -23,25 +23,6 @@ __device__ __forceinline__ double2 hbe(const HopBD& h, int s, int a, int c) {
   return h.hb[((long long)s * h.norb + a) * h.norb + c];
 }
 
-// FP64 <-> FP32 by integer operations where the value is in FP32's normal range (or zero): the
-// conversion instructions occupy the FP64 pipe for several multiply-adds each.  Rounded to
-// nearest even, as the conversions round.
-__device__ __forceinline__ float narrow(double x) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
-  const unsigned e = (unsigned)(b >> 52) & 0x7FFu, sign = (unsigned)(b >> 32) & 0x80000000u;
-  if (e - 897u > 1150u - 897u) return (b << 1) == 0 ? __uint_as_float(sign) : (float)x;
-  const unsigned long long t = (b & 0x7FFFFFFFFFFFFFFFULL) - ((unsigned long long)896 << 52);
-  return __uint_as_float(sign | (unsigned)((t + 0x0FFFFFFFULL + ((t >> 29) & 1ULL)) >> 29));
-}
-__device__ __forceinline__ double widen(float x) {
-  const unsigned b = __float_as_uint(x), m = b & 0x7FFFFFFFu;
-  if (m - 0x00800000u >= 0x7F000000u) return m == 0 ? __longlong_as_double((long long)((unsigned long long)b << 32)) : (double)x;
-  const unsigned long long t = ((unsigned long long)m << 29) + ((unsigned long long)896 << 52);
-  return __longlong_as_double((long long)(t | ((unsigned long long)(b & 0x80000000u) << 32)));
-}
-__device__ __forceinline__ float2 narrow(double2 v) { return make_float2(narrow(v.x), narrow(v.y)); }
-__device__ __forceinline__ double2 widen(float2 v) { return make_double2(widen(v.x), widen(v.y)); }
-
 // ---- W assembly (Energy_Sweep.F90:31-38 + Recursive_Greens.F90:18-20 / :70-72) ----------
 // element e of item b's W, and its FP32 copy where the inverse starts from one
 __device__ __forceinline__ void store_w(const FormW& a, double2* W, int b, long long e, double2 v) {

@@ -81,28 +81,6 @@ struct InvScratch {
   int info;
 };
 
-// 1 / a by a power-of-two scaling of a, an FP32 estimate of 1 / |a|^2, a Newton step, and the
-// quotients with one correction from their remainders (a rounding or two, as crcp): seven FP64
-// operations in sequence, where the two dependent divisions of crcp are some thirty, each of
-// which takes an SM's FP64 pipe a warp's turn
-__device__ __forceinline__ double2 small_rcp(double2 a) {
-  const unsigned long long m = max((unsigned long long)__double_as_longlong(fabs(a.x)),
-                                   (unsigned long long)__double_as_longlong(fabs(a.y)));
-  const int e = (int)(m >> 52);
-  if (e < 64 || e > 1982) return crcp(a);   // beyond the scaling: zeros, subnormals, infinities, NaN
-  const double scale = __longlong_as_double((long long)(2046 - e) << 52);   // 2^(1023 - e): |a| scale in [1, 2.9)
-  const double x = a.x * scale, y = a.y * scale;
-  const float fx = (float)x, fy = (float)y;
-  double r = (double)__frcp_rn(fmaf(fx, fx, fy * fy));
-  const double den = fma(x, x, y * y);
-  const double xs = x * scale, ys = -(y * scale);
-  r = fma(r, fma(-den, r, 1.0), r);
-  double qx = xs * r, qy = ys * r;
-  qx = fma(fma(-qx, den, xs), r, qx);
-  qy = fma(fma(-qy, den, ys), r, qy);
-  return make_double2(qx, qy);
-}
-
 // bits of |re| + |im|, plus one (they order as the values); 0, no candidate, for a NaN
 __device__ __forceinline__ unsigned long long pivot_key(double2 a) {
   const double v = cabs1(a);
