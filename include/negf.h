@@ -56,9 +56,13 @@ extern "C" {
 #define NEGF_ESCRATCH    (-12)   /* negf_zgemm_noalloc: sizes exceed its static scratch  */
 
 /* ---- arithmetic form ------------------------------------------------------------- */
-#define NEGF_PREC_FP64     0     /* FP64 complex results throughout.  32 <= M <= 800: products on the
-                                    tensor cores as nine exact BF16 slices, inverses refined to
-                                    FP64; other sizes on the FP64 pipe                   */
+#define NEGF_PREC_FP64     0     /* FP64 complex results throughout.  39 <= M <= 800 (from M = 32 with
+                                    calc_currents, keep_g_columns or superconducting contacts):
+                                    products on the tensor cores as nine BF16 slices, 63 bits of a
+                                    row's or column's largest entry, and inverses refined to FP64;
+                                    a lead or an energy whose sites' amplitudes are further apart
+                                    than 2^14 is solved again on the FP64 pipe, which every other
+                                    size uses                                             */
 #define NEGF_PREC_MIXED    1     /* tcgen05 BF16 sliced products, FP64 refinement        */
 
 typedef struct negf_params {

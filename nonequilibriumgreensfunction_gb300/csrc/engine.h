@@ -155,8 +155,9 @@ class Engine {
 
   // Products on the tensor cores on S integer BF16 slices and inverses as FP32 Gauss-Jordan +
   // Newton-Schulz steps with the residual at s_res_ slices: the mixed form always; the FP64
-  // form with nine slices (63 bits below each row's or column's maximum, more than a double
-  // holds) and three steps, for M <= 800 when its workspace fits the device.
+  // form with nine slices (63 bits below each row's or column's maximum; results whose sites are
+  // further apart than that serves are solved again on the FP64 pipe) and three steps, for
+  // M <= 800 when its workspace, if only one matrix's, fits the device.
   bool mixed_ = false;
   bool tc_ = false;
   int tc_limit_ = kTcNoLimit;   // FP64 form: most matrices of its workspace

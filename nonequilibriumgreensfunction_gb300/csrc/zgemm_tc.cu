@@ -40,8 +40,8 @@
 // Every mbarrier wait is bounded; on expiry the kernel records an error code and returns
 // after draining its own TMA copies and freeing its TMEM.
 //
-// Replaces, in the mixed form, the ZGEMM calls of Source/Recursive_Greens.F90 and the
-// G Gamma products of Source/Calculate_Gnp.F90.
+// Replaces, in the mixed form and in the FP64 form's sliced range (engine.cu, Engine::configure), the
+// ZGEMM calls of Source/Recursive_Greens.F90 and the G Gamma products of Source/Calculate_Gnp.F90.
 #include <algorithm>
 #include <cstdlib>
 #include <mutex>
@@ -235,7 +235,7 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
 // slicing
 // ---------------------------------------------------------------------------------
 // Slices of x at scale exponent e (|x| < 2^e): the fixed-point integer
-// F = round(x 2^(6 + 7(S-1) - e)), |F| <= 2^(6 + 7(S-1)) <= 2^55, built from the bits of x
+// F = round(x 2^(6 + 7(S-1) - e)), |F| <= 2^(6 + 7(S-1)) (2^55 for eight slices, 2^62 for nine), built from the bits of x
 // with integer operations only (GB300's FP64 pipe is 1/64 of its FP32 rate), then written
 // as balanced base-128 digits: F = sum_p s_p 128^(S-1-p), lower digits in [-64, 63], the
 // top digit in [-64, 64].  Every digit is exact in BF16; the truncation is <= 2^-7S of 2^e.
