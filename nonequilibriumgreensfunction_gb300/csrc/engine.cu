@@ -408,7 +408,12 @@ int Engine::alloc() {
     at(1, 0, 1) = mi;  at(1, 1, 0) = pi_;
     at(2, 0, 0) = one; at(2, 1, 1) = m1;
   }
-  NEGF_CUDA_TRY(cudaMemcpy(dSpin_, spin.data(), sizeof(double2) * spin.size(), cudaMemcpyHostToDevice));
+  return upload(dSpin_, spin.data(), spin.size());
+}
+
+int Engine::upload(double2* dst, const double2* src, size_t count) {
+  NEGF_CUDA_TRY(cudaMemcpyAsync(dst, src, sizeof(double2) * count, cudaMemcpyHostToDevice, own_st_));
+  NEGF_CUDA_TRY(cudaStreamSynchronize(own_st_));
   return NEGF_OK;
 }
 
@@ -451,7 +456,7 @@ int Engine::set_hopx(const double2* hx) {
     // a different HopX invalidates every slot uploaded with the old one
     if (!blocks_equal(cur.data(), hx, MM_)) std::fill(slot_set_.begin(), slot_set_.end(), 0);
   }
-  NEGF_CUDA_TRY(cudaMemcpy(dHop_, hx, sizeof(double2) * MM_, cudaMemcpyHostToDevice));
+  NEGF_TRY(upload(dHop_, hx, (size_t)MM_));
   // block-diagonal detection (site blocks of norb x norb)
   const int no = p_.norb;
   bool bd = true;
@@ -467,7 +472,7 @@ int Engine::set_hopx(const double2* hx) {
     for (int s = 0; s < nsite_; ++s)
       for (int a = 0; a < no; ++a)
         for (int c = 0; c < no; ++c) hb[((size_t)s * no + a) * no + c] = hx[(long long)(s * no + c) * M_ + s * no + a];
-    NEGF_CUDA_TRY(cudaMemcpy(dHopBD_, hb.data(), sizeof(double2) * hb.size(), cudaMemcpyHostToDevice));
+    NEGF_TRY(upload(dHopBD_, hb.data(), hb.size()));
     hop_uniform_ = no == 4;
     for (size_t e = 16; e < hb.size() && hop_uniform_; ++e)
       if (hb[e].x != hb[e % 16].x || hb[e].y != hb[e % 16].y) hop_uniform_ = false;
@@ -508,7 +513,7 @@ int Engine::set_hamiltonian(int slot, const double* Htotd, const double* HopX) {
   const double2* h = reinterpret_cast<const double2*>(Htotd);
   const long long N = p_.npx;
   if (HopX) NEGF_TRY(set_hopx(reinterpret_cast<const double2*>(HopX)));
-  NEGF_CUDA_TRY(cudaMemcpy(dH_ + (long long)slot * N * MM_, h, sizeof(double2) * N * MM_, cudaMemcpyHostToDevice));
+  NEGF_TRY(upload(dH_ + (long long)slot * N * MM_, h, (size_t)(N * MM_)));
   end_h1_[slot].assign(h, h + MM_);
   end_hn_[slot].assign(h + (N - 1) * MM_, h + N * MM_);
   slot_set_[slot] = 1;

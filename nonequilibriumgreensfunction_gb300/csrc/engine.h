@@ -252,6 +252,10 @@ class Engine {
   int merge_info(int batch);
   // upload HopX (M x M) and its site-block form; a changed HopX invalidates every slot
   int set_hopx(const double2* hx);
+  // Host to device, there on return for work on any stream.  (cudaMemcpy from pageable memory may return
+  // with its last piece only staged: ordered on the default stream, which the handle's stream does not
+  // wait for, so that a solve right after it could still read what was there before.)
+  int upload(double2* dst, const double2* src, size_t count);
 };
 
 int merge_info_kernel_launch(int batch, const int* info, int* status, cudaStream_t st);
